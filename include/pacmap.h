@@ -256,6 +256,9 @@ pacmap_status pacmap_fit_transform_learned_device(const float* d_x, uint64_t n, 
  * d x d matrix (f64, row-major) into axes (d x k, row-major), by descending eigenvalue, each column's
  * largest-magnitude entry positive. Cyclic Jacobi for d <= 160, else subspace iteration + Rayleigh-Ritz. */
 pacmap_status pacmap_pca_axes(const double* cov, uint64_t d, uint64_t k, double* out_axes);
+/* The subspace iteration of pacmap_pca_axes as fits run it, on the device (160 < d <= 1024, k <= 128): the
+ * same operations in the same order, so the same bits. cov and out_axes are host memory. */
+pacmap_status pacmap_pca_axes_device(const double* cov, uint64_t d, uint64_t k, int32_t device, double* out_axes);
 
 /* --- the learned model on disk and the transform of new points (no reference analogue: the reference
  * embeds only the points it was fitted on, README.md:165) ---

@@ -119,6 +119,8 @@ void pca_project_device(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint64
 // The k leading eigenvectors of a symmetric d x d matrix (host, f64): axes (d x k, row-major), by
 // descending eigenvalue, each column's largest-magnitude entry positive.
 void pca_top_axes(const double* cov, uint64_t d, uint64_t k, double* axes);
+// The same axes, bit for bit, from the device's subspace iteration (160 < d <= 1024, k <= 128).
+void pca_top_axes_device(Ctx& c, const double* cov, uint64_t d, uint64_t k, double* axes);
 // d_out (n x k) = scale * x[:, :k] for x (n x w).
 void leading_columns(Ctx& c, const float* d_x, uint64_t n, uint64_t w, uint64_t k, float scale, float* d_out);
 void init_random_device(Ctx& c, uint64_t n, uint64_t dim, uint64_t seed, float* d_y);

@@ -7,15 +7,19 @@
 //   1. column means (f64, fixed-order two-level sums);
 //   2. the d x d covariance of the centred rows in f64: at most 64 row chunks (of at least 16,384 rows)
 //      write 32 x 32 partial tiles, reduced over the chunks in order (deterministic, no atomics);
-//   3. the top-k axes on the host (f64): cyclic Jacobi of the whole matrix for d <= 160, above that
+//   3. the top-k axes (f64): cyclic Jacobi of the whole matrix on the host for d <= 160, above that
 //      subspace iteration on k + 24 vectors with a Rayleigh-Ritz step (the power iteration the
-//      reference's randomized SVD uses); axes by descending variance, each axis's largest-magnitude
-//      loading made positive (the reference's SVD sign is LAPACK's and unpinned);
+//      reference's randomized SVD uses), on the GPU when the data is there (top_axes_device) and on the
+//      host for pacmap_pca_axes, with the same operations in the same order: the axes are the same bits;
+//      axes by descending variance, each axis's largest-magnitude loading made positive (the reference's
+//      SVD sign is LAPACK's and unpinned);
 //   4. the projection (x - mean) V_k by a tiled f32 kernel with f64 accumulation.
 #include <algorithm>
 #include <cmath>
 #include <numeric>
 #include <vector>
+
+#include <cooperative_groups.h>
 
 #include "engine.cuh"
 
@@ -192,28 +196,63 @@ void orthonormalise(std::vector<double>& q, int d, int m) {
   }
 }
 
+constexpr int JACOBI_MAX_D = 160;    // whole-matrix Jacobi up to here, subspace iteration above
+constexpr int SUBSPACE_EXTRA = 24;   // vectors iterated beyond the k wanted
+constexpr int SUBSPACE_ITERS = 20;
+
+// The subspace iteration's fixed start, element e (row-major) of the d x m block: the e-th value of a
+// splitmix64 stream (Steele, Lea, Flood 2014) in [-1, 1).
+__host__ __device__ __forceinline__ uint64_t start_bits(uint64_t e) {
+  uint64_t z = 0x9E3779B97F4A7C15ull * (e + 2);
+  z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+  z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+  z ^= z >> 31;
+  return z >> 11;
+}
+
+// Eigenvectors of the m x m Rayleigh-Ritz projection (its rounding symmetrised first) into z, values into w.
+void ritz_eigen(std::vector<double>& proj, int m, std::vector<double>& w, std::vector<double>& z) {
+  for (int i = 0; i < m; ++i)
+    for (int j = i + 1; j < m; ++j) {
+      const double s = 0.5 * (proj[static_cast<size_t>(i) * m + j] + proj[static_cast<size_t>(j) * m + i]);
+      proj[static_cast<size_t>(i) * m + j] = proj[static_cast<size_t>(j) * m + i] = s;
+    }
+  jacobi_eigen(proj, m, w, z);
+}
+
+// The k columns of the d x m block vecs with the largest eigenvalues w, in descending order, each with its
+// largest-magnitude entry positive (d x k, row-major).
+std::vector<double> leading_axes(const std::vector<double>& vecs, const std::vector<double>& w, int d, int m, int k) {
+  std::vector<int> order(m);
+  std::iota(order.begin(), order.end(), 0);
+  std::stable_sort(order.begin(), order.end(), [&](int p, int q) { return w[p] > w[q]; });
+  std::vector<double> V(static_cast<size_t>(d) * k);
+  for (int j = 0; j < k; ++j) {
+    const int col = order[j];
+    int arg = 0;
+    for (int r = 1; r < d; ++r)
+      if (std::fabs(vecs[static_cast<size_t>(r) * m + col]) > std::fabs(vecs[static_cast<size_t>(arg) * m + col])) arg = r;
+    const double sign = vecs[static_cast<size_t>(arg) * m + col] < 0 ? -1.0 : 1.0;
+    for (int r = 0; r < d; ++r) V[static_cast<size_t>(r) * k + j] = sign * vecs[static_cast<size_t>(r) * m + col];
+  }
+  return V;
+}
+
 // The k leading eigenvectors of the symmetric d x d matrix a (columns of the returned d x k matrix,
-// by descending eigenvalue, largest-magnitude entry positive).
+// by descending eigenvalue, largest-magnitude entry positive), on the host.
 std::vector<double> top_axes(std::vector<double>& a, int d, int k) {
   std::vector<double> vecs, w;  // d x m eigenvector block and its eigenvalues
   int m;
-  if (d <= 160) {
+  if (d <= JACOBI_MAX_D) {
     jacobi_eigen(a, d, w, vecs);
     m = d;
   } else {
-    m = std::min(d, k + 24);
+    m = std::min(d, k + SUBSPACE_EXTRA);
     std::vector<double> q(static_cast<size_t>(d) * m), t(static_cast<size_t>(d) * m);
-    uint64_t state = 0x9E3779B97F4A7C15ull;  // fixed start: a splitmix64 stream in [-1, 1)
-    for (auto& e : q) {
-      state += 0x9E3779B97F4A7C15ull;
-      uint64_t z = state;
-      z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
-      z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
-      z ^= z >> 31;
-      e = static_cast<double>(z >> 11) * (2.0 / 9007199254740992.0) - 1.0;
-    }
+    for (size_t e = 0; e < q.size(); ++e)
+      q[e] = static_cast<double>(start_bits(e)) * (2.0 / 9007199254740992.0) - 1.0;
     orthonormalise(q, d, m);
-    for (int it = 0; it < 20; ++it) {
+    for (int it = 0; it < SUBSPACE_ITERS; ++it) {
       std::fill(t.begin(), t.end(), 0.0);
       for (int r = 0; r < d; ++r)
         for (int l = 0; l < d; ++l) {
@@ -238,12 +277,7 @@ std::vector<double> top_axes(std::vector<double>& a, int d, int k) {
         for (int r = 0; r < d; ++r) s += q[static_cast<size_t>(r) * m + i] * aq[static_cast<size_t>(r) * m + j];
         proj[static_cast<size_t>(i) * m + j] = s;
       }
-    for (int i = 0; i < m; ++i)  // symmetrise the rounding
-      for (int j = i + 1; j < m; ++j) {
-        const double s = 0.5 * (proj[static_cast<size_t>(i) * m + j] + proj[static_cast<size_t>(j) * m + i]);
-        proj[static_cast<size_t>(i) * m + j] = proj[static_cast<size_t>(j) * m + i] = s;
-      }
-    jacobi_eigen(proj, m, w, z);
+    ritz_eigen(proj, m, w, z);
     vecs.assign(static_cast<size_t>(d) * m, 0.0);
     for (int r = 0; r < d; ++r)
       for (int j = 0; j < m; ++j) {
@@ -252,19 +286,163 @@ std::vector<double> top_axes(std::vector<double>& a, int d, int k) {
         vecs[static_cast<size_t>(r) * m + j] = s;
       }
   }
-  std::vector<int> order(m);
-  std::iota(order.begin(), order.end(), 0);
-  std::stable_sort(order.begin(), order.end(), [&](int p, int q) { return w[p] > w[q]; });
-  std::vector<double> V(static_cast<size_t>(d) * k);
-  for (int j = 0; j < k; ++j) {
-    const int col = order[j];
-    int arg = 0;
-    for (int r = 1; r < d; ++r)
-      if (std::fabs(vecs[static_cast<size_t>(r) * m + col]) > std::fabs(vecs[static_cast<size_t>(arg) * m + col])) arg = r;
-    const double sign = vecs[static_cast<size_t>(arg) * m + col] < 0 ? -1.0 : 1.0;
-    for (int r = 0; r < d; ++r) V[static_cast<size_t>(r) * k + j] = sign * vecs[static_cast<size_t>(r) * m + col];
+  return leading_axes(vecs, w, d, m, k);
+}
+
+// ------------------------------------------------------------------------------------------------
+// The subspace iteration on the GPU. Every sum runs over its index in ascending order with separately rounded
+// multiplications and additions, as the host's loops do, so each element is the host's bit for bit: the
+// parallelism is over elements only, and what bounds it is the serial chain of d additions per element.
+// 784 columns, 100 axes: 620-720 ms on a host core, 46 ms here (21 orthonormalisations 32 ms, 22 products 5 ms,
+// the rest the host's Ritz problem and copies); a 60,000 x 784 fit from the default start 759 -> 172 ms.
+// ------------------------------------------------------------------------------------------------
+__global__ void subspace_start_kernel(double* __restrict__ q, uint64_t count) {
+  const uint64_t e = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (e < count)
+    q[e] = __dsub_rn(__dmul_rn(static_cast<double>(start_bits(e)), 2.0 / 9007199254740992.0), 1.0);
+}
+
+// out (rows x m) = A (rows x inner) B (inner x m), all row-major: block = AP_ROWS rows x every column (m <= 160,
+// one thread per column), the block's rows of A in shared memory, B's rows read once per block from L2. Four rows a
+// block: 196 blocks for 784 rows (eight rows would leave a third of the SMs without one).
+constexpr int AP_ROWS = 4, AP_COLS = 160;
+__global__ void __launch_bounds__(AP_COLS) block_apply_kernel(const double* __restrict__ A, int rows, int inner,
+                                                              const double* __restrict__ B, int m,
+                                                              double* __restrict__ out) {
+  extern __shared__ double as[];  // [AP_ROWS][inner]
+  const int r0 = blockIdx.x * AP_ROWS, nr = min(AP_ROWS, rows - r0);
+  for (int e = threadIdx.x; e < AP_ROWS * inner; e += AP_COLS)
+    as[e] = e < nr * inner ? A[static_cast<size_t>(r0) * inner + e] : 0.0;
+  __syncthreads();
+  const int j = threadIdx.x;
+  if (j >= m) return;
+  double acc[AP_ROWS] = {};
+#pragma unroll 8
+  for (int l = 0; l < inner; ++l) {
+    const double b = B[static_cast<size_t>(l) * m + j];
+#pragma unroll
+    for (int r = 0; r < AP_ROWS; ++r) acc[r] = __dadd_rn(acc[r], __dmul_rn(as[r * inner + l], b));
   }
-  return V;
+#pragma unroll
+  for (int r = 0; r < AP_ROWS; ++r)
+    if (r < nr) out[static_cast<size_t>(r0 + r) * m + j] = acc[r];
+}
+
+// proj (m x m) = q^T aq over the d rows in order; one thread per element.
+__global__ void ritz_project_kernel(const double* __restrict__ q, const double* __restrict__ aq, int d, int m,
+                                    double* __restrict__ proj) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y;
+  if (j >= m) return;
+  double s = 0.0;
+#pragma unroll 8
+  for (int r = 0; r < d; ++r)
+    s = __dadd_rn(s, __dmul_rn(q[static_cast<size_t>(r) * m + i], aq[static_cast<size_t>(r) * m + j]));
+  proj[static_cast<size_t>(i) * m + j] = s;
+}
+
+// Modified Gram-Schmidt of the columns of a d x m matrix (row-major in and out; in == out allowed) by one cluster of
+// eight blocks, column c in the shared memory of block c % 8. Column by column: its owner normalises it, every block
+// copies it over distributed shared memory, and takes its part out of the later columns it owns. For each column
+// the projections onto the earlier ones are removed in ascending order, as in the host's column-by-column loop.
+// Bound by two serial chains of d additions per column (the norm, then the dot products: those of a block's columns
+// run side by side in the lanes of one warp): 12 us per column of 784 rows, about 14 cycles an addition; forming
+// the next products ahead of the additions did not change it. The columns lie an odd number of doubles apart, so
+// that the lanes' reads fall in different banks. At most 152 columns of 1024 rows: 19 columns per block, 164 KB.
+constexpr int MGS_BLOCKS = 8, MGS_THREADS = 512;
+__host__ __device__ __forceinline__ int mgs_ld(int d) { return d | 1; }
+size_t mgs_smem(int d, int m) {
+  return (static_cast<size_t>((m + MGS_BLOCKS - 1) / MGS_BLOCKS) * mgs_ld(d) + d) * sizeof(double);
+}
+
+__device__ __forceinline__ double chain_dot(const double* a, const double* b, int d) {
+  double s = 0.0;
+#pragma unroll 8
+  for (int r = 0; r < d; ++r) s = __dadd_rn(s, __dmul_rn(a[r], b[r]));
+  return s;
+}
+
+__global__ void __cluster_dims__(MGS_BLOCKS, 1, 1) __launch_bounds__(MGS_THREADS)
+    mgs_kernel(const double* __restrict__ in, int d, int m, double* __restrict__ out) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  extern __shared__ double cols[];  // own columns [ncol][ld], then the current column [d]
+  __shared__ double dots[32], norm;
+  const int rank = static_cast<int>(cluster.block_rank()), tid = threadIdx.x, ld = mgs_ld(d);
+  const int ncol = (m - rank + MGS_BLOCKS - 1) / MGS_BLOCKS;  // columns rank, rank + 8, ... < m
+  double* cur = cols + static_cast<size_t>((m + MGS_BLOCKS - 1) / MGS_BLOCKS) * ld;
+  for (int e = tid; e < ncol * d; e += MGS_THREADS) {
+    const int r = e / ncol, q = e % ncol;
+    cols[q * ld + r] = in[static_cast<size_t>(r) * m + rank + q * MGS_BLOCKS];
+  }
+  __syncthreads();
+  for (int i = 0; i < m; ++i) {
+    const int owner = i % MGS_BLOCKS, slot = i / MGS_BLOCKS;
+    if (rank == owner) {
+      double* v = cols + slot * ld;
+      if (tid == 0) norm = __dsqrt_rn(chain_dot(v, v, d));
+      __syncthreads();
+      const double nrm = norm;
+      for (int r = tid; r < d; r += MGS_THREADS) v[r] = nrm > 0 ? __ddiv_rn(v[r], nrm) : 0.0;
+    }
+    cluster.sync();  // column i is final (nothing writes it again) and may be read by every block
+    const int first = rank > owner ? slot : slot + 1;  // own columns after i
+    if (first >= ncol) continue;
+    const double* src = cluster.map_shared_rank(cols, owner) + slot * ld;
+    for (int r = tid; r < d; r += MGS_THREADS) cur[r] = src[r];
+    __syncthreads();
+    if (tid < ncol - first) dots[tid] = chain_dot(cur, cols + (first + tid) * ld, d);
+    __syncthreads();
+    for (int r = tid; r < d; r += MGS_THREADS) {
+      const double c = cur[r];
+      for (int q = first; q < ncol; ++q) cols[q * ld + r] = __dsub_rn(cols[q * ld + r], __dmul_rn(dots[q - first], c));
+    }
+    __syncthreads();
+  }
+  for (int e = tid; e < ncol * d; e += MGS_THREADS) {
+    const int r = e / ncol, q = e % ncol;
+    out[static_cast<size_t>(r) * m + rank + q * MGS_BLOCKS] = cols[q * ld + r];
+  }
+  cluster.sync();  // no block leaves while another may still read its columns
+}
+
+// top_axes for d > JACOBI_MAX_D with the covariance on the device. The m x m Ritz problem (m <= 152, nearly
+// diagonal by then) stays on the host.
+std::vector<double> top_axes_device(Ctx& c, const double* d_cov, int d, int k) {
+  const int m = std::min(d, k + SUBSPACE_EXTRA);
+  PM_REQUIRE(m <= AP_COLS && (m + MGS_BLOCKS - 1) / MGS_BLOCKS <= 32, PACMAP_ERR_UNSUPPORTED,
+             "PCA supports at most 128 components");
+  const uint64_t dm = static_cast<uint64_t>(d) * m;
+  DevBuf<double> q(c, dm), t(c, dm), proj(c, static_cast<uint64_t>(m) * m), z(c, static_cast<uint64_t>(m) * m);
+  const size_t ms = mgs_smem(d, m);
+  PM_CUDA(cudaFuncSetAttribute(mgs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(ms)));
+  auto mgs = [&](const double* in, double* out) {
+    mgs_kernel<<<MGS_BLOCKS, MGS_THREADS, ms, c.stream>>>(in, d, m, out);
+    PM_LAUNCHED();
+  };
+  auto apply = [&](const double* A, int inner, const double* B, double* out) {
+    block_apply_kernel<<<(d + AP_ROWS - 1) / AP_ROWS, AP_COLS, static_cast<size_t>(AP_ROWS) * inner * sizeof(double),
+                         c.stream>>>(A, d, inner, B, m, out);
+    PM_LAUNCHED();
+  };
+  subspace_start_kernel<<<ceil_div(dm, 256), 256, 0, c.stream>>>(q.get(), dm);
+  PM_LAUNCHED();
+  mgs(q.get(), q.get());
+  for (int it = 0; it < SUBSPACE_ITERS; ++it) {
+    apply(d_cov, d, q.get(), t.get());
+    mgs(t.get(), q.get());
+  }
+  apply(d_cov, d, q.get(), t.get());
+  ritz_project_kernel<<<dim3(ceil_div(m, 64), m), 64, 0, c.stream>>>(q.get(), t.get(), d, m, proj.get());
+  PM_LAUNCHED();
+  std::vector<double> hp(proj.count), w, hz, vecs(dm);
+  PM_CUDA(cudaMemcpyAsync(hp.data(), proj.get(), proj.bytes(), cudaMemcpyDeviceToHost, c.stream));
+  PM_CUDA(cudaStreamSynchronize(c.stream));
+  ritz_eigen(hp, m, w, hz);
+  PM_CUDA(cudaMemcpyAsync(z.get(), hz.data(), z.bytes(), cudaMemcpyHostToDevice, c.stream));
+  apply(q.get(), m, z.get(), t.get());
+  PM_CUDA(cudaMemcpyAsync(vecs.data(), t.get(), dm * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
+  PM_CUDA(cudaStreamSynchronize(c.stream));
+  return leading_axes(vecs, w, d, m, k);
 }
 
 // out (n x k) = scale * x[:, :k] for x (n x w).
@@ -284,6 +462,16 @@ void pca_top_axes(const double* cov, uint64_t d, uint64_t k, double* axes) {
   PM_REQUIRE(k >= 1 && k <= d && d <= 1024, PACMAP_ERR_UNSUPPORTED, "axes need 1 <= k <= d <= 1024");
   std::vector<double> a(cov, cov + d * d);
   const std::vector<double> V = top_axes(a, static_cast<int>(d), static_cast<int>(k));
+  std::copy(V.begin(), V.end(), axes);
+}
+
+void pca_top_axes_device(Ctx& c, const double* cov, uint64_t d, uint64_t k, double* axes) {
+  PM_REQUIRE(k >= 1 && k <= static_cast<uint64_t>(PJ_K) && k <= d && d <= 1024 &&
+                 d > static_cast<uint64_t>(JACOBI_MAX_D),
+             PACMAP_ERR_UNSUPPORTED, "axes on the device need 1 <= k <= 128 and 160 < d <= 1024");
+  DevBuf<double> dc;
+  upload(c, dc, cov, d * d);
+  const std::vector<double> V = top_axes_device(c, dc.get(), static_cast<int>(d), static_cast<int>(k));
   std::copy(V.begin(), V.end(), axes);
 }
 
@@ -315,11 +503,16 @@ void pca_project_device(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint64
   PM_LAUNCHED();
   cov_reduce_kernel<<<ceil_div(d * d, 256), 256, 0, c.stream>>>(part.get(), chunks, d * d, cov.get());
   PM_LAUNCHED();
-  std::vector<double> a(d * d);
-  PM_CUDA(cudaMemcpyAsync(a.data(), cov.get(), d * d * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
-  PM_CUDA(cudaStreamSynchronize(c.stream));
   // 3. axes
-  const std::vector<double> V64 = top_axes(a, static_cast<int>(d), static_cast<int>(k));
+  std::vector<double> V64;
+  if (d > static_cast<uint64_t>(JACOBI_MAX_D)) {
+    V64 = top_axes_device(c, cov.get(), static_cast<int>(d), static_cast<int>(k));
+  } else {
+    std::vector<double> a(d * d);
+    PM_CUDA(cudaMemcpyAsync(a.data(), cov.get(), d * d * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
+    PM_CUDA(cudaStreamSynchronize(c.stream));
+    V64 = top_axes(a, static_cast<int>(d), static_cast<int>(k));
+  }
   std::vector<float> V(d * k);
   for (uint64_t e = 0; e < d * k; ++e) V[e] = static_cast<float>(V64[e]);
   if (axes_out) *axes_out = V;
