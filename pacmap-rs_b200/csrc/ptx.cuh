@@ -58,6 +58,13 @@ __device__ __noinline__ inline bool mbar_wait(uint64_t* bar, uint32_t parity, vo
   }
 }
 
+// 16 bytes global -> shared (both 16-byte aligned), asynchronous; joined by cp.async groups.
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)),
+               "l"(reinterpret_cast<uint64_t>(src))
+               : "memory");
+}
+
 // Untiled bulk copy global -> shared (both 16-byte aligned, size a multiple of 16), completing on bar.
 __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
