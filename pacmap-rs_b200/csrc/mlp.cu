@@ -4,7 +4,7 @@
 // (src/lib.rs:753-766 rescales it to std 1e-4, so only its geometry matters).
 //
 // Every GEMM of the forward and backward pass is one hand-written tcgen05 kernel, C = A . B^T with
-// both operands K-major BF16 (TMA, 128-byte swizzle, 4-stage pipeline, FP32 accumulator in TMEM) and a
+// both operands K-major BF16 (TMA, 128-byte swizzle, FP32 accumulator in TMEM) and a
 // fused epilogue: bias + ReLU -> BF16, ReLU backprop through the stored activation -> BF16, or FP32.
 // Operands needed in the other orientation (X^T, H^T, dZ^T, W^T) come from a BF16 transpose kernel.
 // FP32 master weights, AdamW (decoupled weight decay), BF16 copies refreshed after each step.
@@ -26,7 +26,10 @@ namespace {
 
 constexpr int MLP_H = 512;
 constexpr int GEMM_THREADS = 192;  // warp 0 TMA, warp 1 MMA + TMEM owner, warps 2..5 epilogue
-constexpr int GEMM_STAGES = 2;  // 66 KB at BN = 128: three blocks per SM overlap each other's epilogues
+// Operand pipeline depth. Two stages (66 KB at BN = 128) leave room for three blocks per SM, which overlap each
+// other's waits and epilogues; a grid of at most one block per SM has nobody to overlap with and hides the copies
+// behind six stages instead.
+constexpr int GEMM_STAGES_MANY = 2, GEMM_STAGES_FEW = 6;
 constexpr int A_STAGE = 128 * 128;  // 128 rows x 64 bf16
 
 enum Epi : int { EPI_F32 = 0, EPI_BIAS_RELU = 1, EPI_DRELU = 2 };
@@ -40,8 +43,8 @@ struct GemmOut {
 };
 
 struct alignas(8) GemmShared {
-  uint64_t full[GEMM_STAGES];
-  uint64_t empty[GEMM_STAGES];
+  uint64_t full[GEMM_STAGES_FEW];
+  uint64_t empty[GEMM_STAGES_FEW];
   uint64_t done;
   uint32_t tmem_base;
   int abort_flag;
@@ -52,7 +55,7 @@ __host__ __device__ constexpr int tmem_cols() {
   return BN <= 32 ? 32 : (BN <= 64 ? 64 : (BN <= 128 ? 128 : 256));
 }
 
-template <int BN, int EPI>
+template <int BN, int EPI, int GEMM_STAGES>
 __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tn_kernel(const __grid_constant__ CUtensorMap amap,
                                                                   const __grid_constant__ CUtensorMap bmap, int K,
                                                                   GemmOut o, uint32_t* __restrict__ err) {
@@ -356,17 +359,23 @@ __global__ void f32_to_bf16_kernel(const float* __restrict__ src, uint64_t count
 // ---------------------------------------------------------------------------------------------
 inline int pad_to(int v, int m) { return (v + m - 1) / m * m; }
 
+template <int BN, int EPI, int STAGES>
+void gemm_launch(Ctx& c, const CUtensorMap& am, const CUtensorMap& bm, dim3 grid, int K, const GemmOut& o) {
+  const size_t smem = 1024 + STAGES * (A_STAGE + BN * 128) + sizeof(GemmShared);
+  PM_CUDA(cudaFuncSetAttribute(gemm_tn_kernel<BN, EPI, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               static_cast<int>(smem)));
+  gemm_tn_kernel<BN, EPI, STAGES><<<grid, GEMM_THREADS, smem, c.stream>>>(am, bm, K, o, c.d_err);
+  PM_LAUNCHED();
+}
+
 template <int BN, int EPI>
 void gemm(Ctx& c, const __nv_bfloat16* A, int M_rows_alloc, const __nv_bfloat16* Bm, int N_rows_alloc, int K,
           const GemmOut& o) {
   const CUtensorMap am = make_tmap_2d_16b(A, M_rows_alloc, K, 128, true);
   const CUtensorMap bm = make_tmap_2d_16b(Bm, N_rows_alloc, K, BN, true);
-  const size_t smem = 1024 + GEMM_STAGES * (A_STAGE + BN * 128) + sizeof(GemmShared);
-  PM_CUDA(cudaFuncSetAttribute(gemm_tn_kernel<BN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               static_cast<int>(smem)));
   const dim3 grid(static_cast<unsigned>(M_rows_alloc / 128), static_cast<unsigned>((N_rows_alloc + BN - 1) / BN));
-  gemm_tn_kernel<BN, EPI><<<grid, GEMM_THREADS, smem, c.stream>>>(am, bm, K, o, c.d_err);
-  PM_LAUNCHED();
+  if (grid.x * grid.y <= static_cast<unsigned>(c.sm_count)) gemm_launch<BN, EPI, GEMM_STAGES_FEW>(c, am, bm, grid, K, o);
+  else gemm_launch<BN, EPI, GEMM_STAGES_MANY>(c, am, bm, grid, K, o);
 }
 
 void transpose(Ctx& c, const __nv_bfloat16* src, int R, int C, __nv_bfloat16* dst) {
