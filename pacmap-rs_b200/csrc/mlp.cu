@@ -330,21 +330,43 @@ __global__ void gather_rows_kernel(const float* __restrict__ src, const uint32_t
   dst[t] = src[static_cast<uint64_t>(rows[r]) * dim + (t % dim)];
 }
 
-// AdamW (decoupled weight decay) on an f32 master tensor; also writes its bf16 copy.
-__global__ void adamw_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
-                             float* __restrict__ v, uint64_t count, float lr, float wd, float b1c, float b2c,
-                             __nv_bfloat16* __restrict__ pb) {
-  const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-  for (uint64_t t = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; t < count; t += stride) {
-    const float gg = g[t];
-    float mm = 0.9f * m[t] + 0.1f * gg;
-    float vv = 0.999f * v[t] + 0.001f * gg * gg;
-    m[t] = mm;
-    v[t] = vv;
-    float w = p[t] * (1.0f - lr * wd);
-    w -= lr * (mm / b1c) / (sqrtf(vv / b2c) + 1e-8f);
-    p[t] = w;
-    if (pb) pb[t] = __float2bfloat16_rn(w);
+// One AdamW step (decoupled weight decay on the weights, not on the biases) of all six tensors in one launch, each
+// thread writing its parameter's bf16 copies in the operand layouts too: W1b, W2b and W2^T, W3 and its padded
+// transpose (the padding columns stay the zeros that MlpNet::refresh wrote). A step's 330,000 parameters are a few
+// microseconds of traffic, so what counts is the launches: this one replaces 12.
+struct AdamArgs {
+  float *p[6], *m[6], *v[6];
+  const float* g[6];
+  uint32_t end[6];  // running ends of the tensors in the flat index
+  __nv_bfloat16 *W1b, *W2b, *W2Tb, *W3b, *W3Tb;
+  int dp16, dp64;
+};
+
+__global__ void __launch_bounds__(256) adamw_kernel(AdamArgs a, float lr, float wd, float b1c, float b2c) {
+  const uint32_t i = blockIdx.x * 256 + threadIdx.x;
+  if (i >= a.end[5]) return;
+  int q = 0;
+  while (i >= a.end[q]) ++q;
+  const uint32_t t = i - (q ? a.end[q - 1] : 0u);
+  const float decay = (q % 2 == 0) ? wd : 0.0f;
+  const float gg = a.g[q][t];
+  float mm = 0.9f * a.m[q][t] + 0.1f * gg;
+  float vv = 0.999f * a.v[q][t] + 0.001f * gg * gg;
+  a.m[q][t] = mm;
+  a.v[q][t] = vv;
+  float w = a.p[q][t] * (1.0f - lr * decay);
+  w -= lr * (mm / b1c) / (sqrtf(vv / b2c) + 1e-8f);
+  a.p[q][t] = w;
+  const __nv_bfloat16 wb = __float2bfloat16_rn(w);
+  if (q == 0) {
+    a.W1b[t] = wb;
+  } else if (q == 2) {
+    a.W2b[t] = wb;
+    a.W2Tb[(t % MLP_H) * MLP_H + t / MLP_H] = wb;
+  } else if (q == 4) {  // W3T [512][dp16]
+    const uint32_t r = t / a.dp16, c = t % a.dp16;
+    a.W3b[c * MLP_H + r] = wb;
+    a.W3Tb[r * a.dp64 + c] = wb;
   }
 }
 
@@ -501,13 +523,15 @@ void mlp_forward(Ctx& c, MlpNet& net, const __nv_bfloat16* X, int rows, __nv_bfl
   gemm<16, EPI_F32>(c, H2, rows, net.W3b.get(), net.dp16, MLP_H, f);
 }
 
+constexpr int LOSS_PARTS = 64;  // blocks of mse_grad_kernel
+
 // Scratch for one batch of B rows.
 struct MlpBatch {
   int B = 0;
   DevBuf<__nv_bfloat16> X, XT, H1, H1T, H2, H2T, dZ3, dZ3T, dZ2, dZ2T, dZ1, dZ1T;
   DevBuf<float> out, tgt, gW1, gb1, gW2, gb2, gW3T, gb3;
-  DevBuf<double> partial;
-  void alloc(Ctx& c, const MlpNet& net, int B_) {
+  DevBuf<double> partial;  // LOSS_PARTS partial losses per step, of `steps` steps
+  void alloc(Ctx& c, const MlpNet& net, int B_, uint64_t steps = 1) {
     B = B_;
     X.alloc(c, static_cast<size_t>(B) * net.dp);
     XT.alloc(c, static_cast<size_t>(B) * net.dp);
@@ -529,17 +553,17 @@ struct MlpBatch {
     gb2.alloc(c, MLP_H);
     gW3T.alloc(c, net.W3T.count);
     gb3.alloc(c, net.dp16);
-    partial.alloc(c, 64);
+    partial.alloc(c, LOSS_PARTS * steps);
   }
 };
 
 // Forward + backward of one batch (X and tgt already filled); gradients into bt.g*, returns nothing
-// (the loss partials are in bt.partial).
-void mlp_forward_backward(Ctx& c, MlpNet& net, MlpBatch& bt) {
+// (the loss partials go to bt.partial, slot `step`).
+void mlp_forward_backward(Ctx& c, MlpNet& net, MlpBatch& bt, uint64_t step = 0) {
   const int B = bt.B;
   mlp_forward(c, net, bt.X.get(), B, bt.H1.get(), bt.H2.get(), bt.out.get(), B);
-  mse_grad_kernel<<<64, 256, 0, c.stream>>>(bt.out.get(), net.dp16, bt.tgt.get(), B, net.dim, net.dp64, bt.dZ3.get(),
-                                           bt.partial.get());
+  mse_grad_kernel<<<LOSS_PARTS, 256, 0, c.stream>>>(bt.out.get(), net.dp16, bt.tgt.get(), B, net.dim, net.dp64,
+                                                   bt.dZ3.get(), bt.partial.get() + step * LOSS_PARTS);
   PM_LAUNCHED();
   // dW3^T [512][dp16] = H2^T . dZ3  (A = H2^T [512][B], B = dZ3^T [dp16][B], K = B)
   transpose(c, bt.H2.get(), B, MLP_H, bt.H2T.get());
@@ -604,15 +628,26 @@ void adamw_step(Ctx& c, MlpNet& net, MlpBatch& bt, std::vector<DevBuf<float>>& m
   const float b1c = 1.0f - std::pow(0.9f, static_cast<float>(t));
   const float b2c = 1.0f - std::pow(0.999f, static_cast<float>(t));
   float* P[6] = {net.W1.get(), net.b1.get(), net.W2.get(), net.b2.get(), net.W3T.get(), net.b3.get()};
-  float* G[6] = {bt.gW1.get(), bt.gb1.get(), bt.gW2.get(), bt.gb2.get(), bt.gW3T.get(), bt.gb3.get()};
-  const uint64_t N[6] = {net.W1.count, net.b1.count, net.W2.count, net.b2.count, net.W3T.count, net.b3.count};
+  const float* G[6] = {bt.gW1.get(), bt.gb1.get(), bt.gW2.get(), bt.gb2.get(), bt.gW3T.get(), bt.gb3.get()};
+  const size_t N[6] = {net.W1.count, net.b1.count, net.W2.count, net.b2.count, net.W3T.count, net.b3.count};
+  AdamArgs a{};
+  uint32_t end = 0;  // d <= 4096: below 2^22 parameters
   for (int q = 0; q < 6; ++q) {
-    const float decay = (q % 2 == 0) ? wd : 0.0f;  // weights decay, biases do not
-    adamw_kernel<<<static_cast<unsigned>(std::min<uint64_t>(ceil_div(N[q], 256), 1024)), 256, 0, c.stream>>>(
-        P[q], G[q], mom[2 * q].get(), mom[2 * q + 1].get(), N[q], lr, decay, b1c, b2c, nullptr);
-    PM_LAUNCHED();
+    a.p[q] = P[q];
+    a.g[q] = G[q];
+    a.m[q] = mom[2 * q].get();
+    a.v[q] = mom[2 * q + 1].get();
+    a.end[q] = end += static_cast<uint32_t>(N[q]);
   }
-  net.refresh(c);
+  a.W1b = net.W1b.get();
+  a.W2b = net.W2b.get();
+  a.W2Tb = net.W2Tb.get();
+  a.W3b = net.W3b.get();
+  a.W3Tb = net.W3Tb.get();
+  a.dp16 = net.dp16;
+  a.dp64 = net.dp64;
+  adamw_kernel<<<ceil_div(end, 256), 256, 0, c.stream>>>(a, lr, wd, b1c, b2c);
+  PM_LAUNCHED();
 }
 
 }  // namespace
@@ -683,8 +718,8 @@ void mlp_grad_device(Ctx& c, const float* params, uint64_t d, uint64_t dim, cons
   PM_CUDA(cudaMemcpyAsync(g.W3T.get(), bt.gW3T.get(), bt.gW3T.bytes(), cudaMemcpyDeviceToDevice, c.stream));
   PM_CUDA(cudaMemcpyAsync(g.b3.get(), bt.gb3.get(), bt.gb3.bytes(), cudaMemcpyDeviceToDevice, c.stream));
   g.download(c, grads_flat);
-  std::vector<double> part(64);
-  PM_CUDA(cudaMemcpyAsync(part.data(), bt.partial.get(), 64 * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
+  std::vector<double> part(LOSS_PARTS);
+  PM_CUDA(cudaMemcpyAsync(part.data(), bt.partial.get(), bt.partial.bytes(), cudaMemcpyDeviceToHost, c.stream));
   PM_CUDA(cudaStreamSynchronize(c.stream));
   double s = 0.0;
   for (double v : part) s += v;
@@ -701,7 +736,8 @@ void mlp_train_device(Ctx& c, float* params, uint64_t d, uint64_t dim, const flo
   net.alloc(c, static_cast<int>(d), static_cast<int>(dim));
   net.upload(c, params);
   MlpBatch bt;
-  bt.alloc(c, net, static_cast<int>(batch));
+  const uint64_t steps = n / batch;
+  bt.alloc(c, net, static_cast<int>(batch), steps);
   std::vector<DevBuf<float>> mom(12);
   const uint64_t cnt[6] = {net.W1.count, net.b1.count, net.W2.count, net.b2.count, net.W3T.count, net.b3.count};
   for (int q = 0; q < 6; ++q) {
@@ -713,7 +749,7 @@ void mlp_train_device(Ctx& c, float* params, uint64_t d, uint64_t dim, const flo
   std::vector<uint32_t> perm(n);
   DevBuf<uint32_t> dperm(c, n);
   std::mt19937_64 rng(seed);
-  const uint64_t steps = n / batch;
+  std::vector<double> part(LOSS_PARTS * steps);
   int t = 0;
   for (uint64_t ep = 0; ep < epochs; ++ep) {
     for (uint64_t i = 0; i < n; ++i) perm[i] = static_cast<uint32_t>(i);
@@ -727,13 +763,15 @@ void mlp_train_device(Ctx& c, float* params, uint64_t d, uint64_t dim, const flo
       gather_rows_kernel<<<ceil_div(batch * dim, 256), 256, 0, c.stream>>>(d_t, rows, batch, static_cast<int>(dim),
                                                                           bt.tgt.get());
       PM_LAUNCHED();
-      mlp_forward_backward(c, net, bt);
+      mlp_forward_backward(c, net, bt, st);
       adamw_step(c, net, bt, mom, lr, wd, ++t);
-      std::vector<double> part(64);
-      PM_CUDA(cudaMemcpyAsync(part.data(), bt.partial.get(), 64 * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
-      PM_CUDA(cudaStreamSynchronize(c.stream));
+    }
+    // the epoch's losses in one read: a step does not wait for the host
+    PM_CUDA(cudaMemcpyAsync(part.data(), bt.partial.get(), bt.partial.bytes(), cudaMemcpyDeviceToHost, c.stream));
+    PM_CUDA(cudaStreamSynchronize(c.stream));
+    for (uint64_t st = 0; st < steps; ++st) {
       double s = 0.0;
-      for (double v : part) s += v;
+      for (int e = 0; e < LOSS_PARTS; ++e) s += part[st * LOSS_PARTS + e];
       ep_loss += s / static_cast<double>(batch * dim);
     }
     if (epoch_loss) epoch_loss[ep] = static_cast<float>(ep_loss / std::max<uint64_t>(steps, 1));
