@@ -99,6 +99,8 @@ void sample_fp_device(Ctx& c, const uint32_t* d_pnn, uint64_t n, uint64_t k, uin
 struct Csr {
   DevBuf<uint32_t> row_ptr;  // 3n + 1 offsets: segments (row, type) with type NN = 0, MN = 1, FP = 2
   DevBuf<uint32_t> col;      // partner of each entry, ascending within a segment
+  DevBuf<uint32_t> long_rows;  // the rows with the most entries, which the gradient gives a warp each
+  uint32_t n_long = 0;
   uint64_t entries = 0;
 };
 // grouped_known: the lists are known to hold each point's pairs together (generated lists), so the

@@ -394,6 +394,22 @@ struct Sched {
   float w_nn, w_mn, w_fp, lr_t;
 };
 
+constexpr int GRAD_G = 8;  // lanes per row
+
+// What one iteration reads and writes: y_cur -> y_next, m and v in place (grad_only: none of them written).
+struct GradArgs {
+  const float* y_cur;
+  float *y_next, *m, *v;
+  const uint32_t *rp, *col;
+  uint64_t n;
+  const uint32_t* long_rows;
+  uint32_t n_long;
+  const Sched* sched;
+  float a1, a2;
+  float *row_loss, *grad_out;  // may be null
+  int grad_only;
+};
+
 // y of partner j (DIM consecutive floats; one 8-byte load for 2-D).
 template <int DIM>
 __device__ __forceinline__ void load_y(const float* __restrict__ y, uint32_t j, float (&out)[DIM]) {
@@ -407,8 +423,31 @@ __device__ __forceinline__ void load_y(const float* __restrict__ y, uint32_t j, 
   }
 }
 
+// The force of partner yj on yi (per-pair arithmetic of gradient.rs:120-147) and the pair's loss.
+template <int DIM, bool REPULSIVE>
+__device__ __forceinline__ void pair_term(const float (&yi)[DIM], const float (&yj)[DIM], float c1, float c2, float w,
+                                          float (&term)[DIM], float& loss, bool want_loss) {
+  float df[DIM];
+  float dsq = 1.0f;
+#pragma unroll
+  for (int c = 0; c < DIM; ++c) {
+    df[c] = __fsub_rn(yi[c], yj[c]);
+    dsq = __fadd_rn(dsq, __fmul_rn(df[c], df[c]));
+  }
+  const float tt = __fadd_rn(c1, dsq);
+  const float w1 = __fmul_rn(w, __fdiv_rn(c2, __fmul_rn(tt, tt)));
+#pragma unroll
+  for (int c = 0; c < DIM; ++c) {
+    const float gterm = __fmul_rn(w1, df[c]);
+    term[c] = REPULSIVE ? -gterm : gterm;
+  }
+  if (want_loss)
+    loss = REPULSIVE ? __fmul_rn(w, __fdiv_rn(1.0f, __fadd_rn(1.0f, dsq))) : __fmul_rn(w, __fdiv_rn(dsq, tt));
+}
+
 // One segment (one pair type) of a row: lane gl of a G-lane group takes entries s + gl, s + gl + G, ...
-// in that order, with the partner index and y of the next entry loaded ahead (two-deep pipeline).
+// in that order, with the partner index and y of the next entry loaded ahead (two-deep pipeline; four entries in
+// flight need 74 registers instead of 48 and made the 1M x 128 iterations 2 % slower).
 // The type's constants (c1, c2, weight, sign) are fixed for the whole segment.
 template <int DIM, bool REPULSIVE>
 __device__ __forceinline__ void accumulate_segment(const float* __restrict__ y, const uint32_t* __restrict__ col,
@@ -426,90 +465,158 @@ __device__ __forceinline__ void accumulate_segment(const float* __restrict__ y, 
     float yb[DIM];
     if (j + g < e) load_y<DIM>(y, jb, yb);
     const uint32_t jc = j + 2 * g < e ? col[j + 2 * g] : 0u;
-    float df[DIM];
-    float dsq = 1.0f;
+    float term[DIM], loss = 0.0f;
+    pair_term<DIM, REPULSIVE>(yi, ya, c1, c2, w, term, loss, want_loss);
 #pragma unroll
-    for (int c = 0; c < DIM; ++c) {
-      df[c] = __fsub_rn(yi[c], ya[c]);
-      dsq = __fadd_rn(dsq, __fmul_rn(df[c], df[c]));
-    }
-    const float tt = __fadd_rn(c1, dsq);
-    const float w1 = __fmul_rn(w, __fdiv_rn(c2, __fmul_rn(tt, tt)));
-#pragma unroll
-    for (int c = 0; c < DIM; ++c) {
-      const float gterm = __fmul_rn(w1, df[c]);
-      acc[c] = __fadd_rn(acc[c], REPULSIVE ? -gterm : gterm);
-    }
-    if (want_loss)
-      lacc += REPULSIVE ? __fmul_rn(w, __fdiv_rn(1.0f, __fadd_rn(1.0f, dsq))) : __fmul_rn(w, __fdiv_rn(dsq, tt));
+    for (int c = 0; c < DIM; ++c) acc[c] = __fadd_rn(acc[c], term[c]);
+    if (want_loss) lacc += loss;
 #pragma unroll
     for (int c = 0; c < DIM; ++c) ya[c] = yb[c];
     jb = jc;
   }
 }
 
-// A row's forces: the NN, MN (skipped when w_mn = 0) and FP segments in turn (per-pair arithmetic of
-// gradient.rs:120-147: c = 10, 10000 and 1 in the denominators, FP repulsive).
-template <int DIM>
+// The same segment by a whole warp, for rows of more than GRAD_LONG entries: each lane forms the terms of its own
+// entries (LONG_U x 32 in flight), and lane l then adds, from the four lanes l % 8 + 8 r in turn, the entries
+// that lane l % 8 of an eight-lane group would have added, in the same order: the sums are the same bits. (Entry t of
+// the segment belongs to lane t % 8 in both.)
+constexpr uint32_t GRAD_LONG = 1024;
+constexpr int LONG_U = 4;
+template <int DIM, bool REPULSIVE>
+__device__ __forceinline__ void accumulate_segment_warp(const float* __restrict__ y, const uint32_t* __restrict__ col,
+                                                        uint32_t s, uint32_t e, int lane, const float (&yi)[DIM],
+                                                        float c1, float c2, float w, float (&acc)[DIM], float& lacc,
+                                                        bool want_loss) {
+  const uint32_t ln = static_cast<uint32_t>(lane), gl = ln & 7u;
+  uint32_t nj[LONG_U];
+#pragma unroll
+  for (int u = 0; u < LONG_U; ++u) nj[u] = s + u * 32 + ln < e ? col[s + u * 32 + ln] : 0u;
+  for (uint32_t b = s; b < e; b += LONG_U * 32) {
+    float ya[LONG_U][DIM];
+#pragma unroll
+    for (int u = 0; u < LONG_U; ++u) load_y<DIM>(y, nj[u], ya[u]);  // past the end: point 0, not added below
+#pragma unroll
+    for (int u = 0; u < LONG_U; ++u) {
+      const uint32_t t = b + (LONG_U + u) * 32 + ln;
+      nj[u] = t < e ? col[t] : 0u;
+    }
+#pragma unroll
+    for (int u = 0; u < LONG_U; ++u) {
+      float term[DIM], loss = 0.0f;
+      pair_term<DIM, REPULSIVE>(yi, ya[u], c1, c2, w, term, loss, want_loss);
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const bool in = b + u * 32 + gl + 8 * r < e;
+#pragma unroll
+        for (int c = 0; c < DIM; ++c) {
+          const float tv = __shfl_sync(0xFFFFFFFFu, term[c], gl + 8 * r);
+          if (in) acc[c] = __fadd_rn(acc[c], tv);
+        }
+        if (want_loss) {
+          const float lv = __shfl_sync(0xFFFFFFFFu, loss, gl + 8 * r);
+          if (in) lacc += lv;
+        }
+      }
+    }
+  }
+}
+
+// A row's forces: the NN, MN (skipped when w_mn = 0) and FP segments in turn (c = 10, 10000 and 1 in the
+// denominators, FP repulsive). WARP: the whole warp on one row, else the G lanes of a group.
+template <int DIM, bool WARP>
 __device__ __forceinline__ void accumulate_row(const float* __restrict__ y, const uint32_t* __restrict__ col,
                                                uint32_t s0, uint32_t s1, uint32_t s2, uint32_t s3, bool use_mn,
                                                int gl, int G, const float (&yi)[DIM], const Sched& sc,
                                                float (&acc)[DIM], float& lacc, bool want_loss) {
-  accumulate_segment<DIM, false>(y, col, s0, s1, gl, G, yi, 10.0f, 20.0f, sc.w_nn, acc, lacc, want_loss);
-  if (use_mn)
-    accumulate_segment<DIM, false>(y, col, s1, s2, gl, G, yi, 10000.0f, 20000.0f, sc.w_mn, acc, lacc, want_loss);
-  accumulate_segment<DIM, true>(y, col, s2, s3, gl, G, yi, 1.0f, 2.0f, sc.w_fp, acc, lacc, want_loss);
+  if constexpr (WARP) {
+    accumulate_segment_warp<DIM, false>(y, col, s0, s1, gl, yi, 10.0f, 20.0f, sc.w_nn, acc, lacc, want_loss);
+    if (use_mn)
+      accumulate_segment_warp<DIM, false>(y, col, s1, s2, gl, yi, 10000.0f, 20000.0f, sc.w_mn, acc, lacc, want_loss);
+    accumulate_segment_warp<DIM, true>(y, col, s2, s3, gl, yi, 1.0f, 2.0f, sc.w_fp, acc, lacc, want_loss);
+  } else {
+    accumulate_segment<DIM, false>(y, col, s0, s1, gl, G, yi, 10.0f, 20.0f, sc.w_nn, acc, lacc, want_loss);
+    if (use_mn)
+      accumulate_segment<DIM, false>(y, col, s1, s2, gl, G, yi, 10000.0f, 20000.0f, sc.w_mn, acc, lacc, want_loss);
+    accumulate_segment<DIM, true>(y, col, s2, s3, gl, G, yi, 1.0f, 2.0f, sc.w_fp, acc, lacc, want_loss);
+  }
 }
 
-template <int G, int DIM>
-__global__ void __launch_bounds__(256) grad_adam_kernel(const float* __restrict__ y_cur, float* __restrict__ y_next,
-                                                        float* __restrict__ m, float* __restrict__ v,
-                                                        const uint32_t* __restrict__ rp,
-                                                        const uint32_t* __restrict__ col, uint64_t n,
-                                                        const Sched* __restrict__ sched, int itr, float a1, float a2,
-                                                        float* __restrict__ row_loss, float* __restrict__ grad_out,
-                                                        int grad_only) {
-  const Sched sc = sched[itr];
-  const int gl = threadIdx.x & (G - 1);
-  const uint64_t groups = static_cast<uint64_t>(gridDim.x) * (blockDim.x / G);
-  const bool want_loss = row_loss != nullptr;
-  const unsigned gmask = (G == 32) ? 0xFFFFFFFFu : (((1u << G) - 1u) << ((threadIdx.x & 31) & ~(G - 1)));
-  for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * (blockDim.x / G) + threadIdx.x / G; i < n; i += groups) {
-    float yi[DIM], acc[DIM];
+// Adam (adam.rs:45-57) of one coordinate: updates m and v, returns the new y.
+__device__ __forceinline__ float adam_coord(float g, float yi, float* __restrict__ m, float* __restrict__ v, float a1,
+                                            float a2, float lr_t) {
+  float mm = *m, vv = *v;
+  mm = __fadd_rn(mm, __fmul_rn(a1, __fsub_rn(g, mm)));
+  vv = __fadd_rn(vv, __fmul_rn(a2, __fsub_rn(__fmul_rn(g, g), vv)));
+  const float step = __fdiv_rn(__fmul_rn(lr_t, mm), __fadd_rn(__fsqrt_rn(vv), 1e-7f));
+  *m = mm;
+  *v = vv;
+  return __fsub_rn(yi, step);
+}
+
+// One row's iteration by the lanes gl of an eight-lane group (gmask: its lanes), or by a whole warp.
+template <int DIM, bool WARP>
+__device__ __forceinline__ void grad_adam_row(const GradArgs& p, const Sched& sc, uint64_t i, uint32_t s0, uint32_t s1,
+                                              uint32_t s2, uint32_t s3, int gl, unsigned gmask) {
+  constexpr int G = GRAD_G;
+  const bool want_loss = p.row_loss != nullptr;
+  float yi[DIM], acc[DIM];
+#pragma unroll
+  for (int c = 0; c < DIM; ++c) {
+    yi[c] = p.y_cur[i * DIM + c];
+    acc[c] = 0.0f;
+  }
+  float lacc = 0.0f;
+  accumulate_row<DIM, WARP>(p.y_cur, p.col, s0, s1, s2, s3, sc.w_mn != 0.0f, gl, G, yi, sc, acc, lacc, want_loss);
+#pragma unroll
+  for (int o = G / 2; o > 0; o >>= 1) {
+#pragma unroll
+    for (int c = 0; c < DIM; ++c) acc[c] = __fadd_rn(acc[c], __shfl_xor_sync(gmask, acc[c], o, G));
+    if (want_loss) lacc += __shfl_xor_sync(gmask, lacc, o, G);
+  }
+  if (gl == 0) {
 #pragma unroll
     for (int c = 0; c < DIM; ++c) {
-      yi[c] = y_cur[i * DIM + c];
-      acc[c] = 0.0f;
+      if (!p.grad_only)
+        p.y_next[i * DIM + c] = adam_coord(acc[c], yi[c], p.m + i * DIM + c, p.v + i * DIM + c, p.a1, p.a2, sc.lr_t);
+      if (p.grad_out) p.grad_out[i * DIM + c] = acc[c];
     }
-    float lacc = 0.0f;
-    const uint32_t s0 = rp[3 * i], s1 = rp[3 * i + 1], s2 = rp[3 * i + 2], s3 = rp[3 * i + 3];
-    accumulate_row<DIM>(y_cur, col, s0, s1, s2, s3, sc.w_mn != 0.0f, gl, G, yi, sc, acc, lacc, want_loss);
-#pragma unroll
-    for (int o = G / 2; o > 0; o >>= 1) {
-#pragma unroll
-      for (int c = 0; c < DIM; ++c) acc[c] = __fadd_rn(acc[c], __shfl_xor_sync(gmask, acc[c], o, G));
-      if (want_loss) lacc += __shfl_xor_sync(gmask, lacc, o, G);
-    }
-    if (gl == 0 && grad_only) {
-#pragma unroll
-      for (int c = 0; c < DIM; ++c) grad_out[i * DIM + c] = acc[c];
-      if (want_loss) row_loss[i] = lacc;
-    } else if (gl == 0) {
-#pragma unroll
-      for (int c = 0; c < DIM; ++c) {
-        const float g = acc[c];
-        float mm = m[i * DIM + c], vv = v[i * DIM + c];
-        mm = __fadd_rn(mm, __fmul_rn(a1, __fsub_rn(g, mm)));
-        vv = __fadd_rn(vv, __fmul_rn(a2, __fsub_rn(__fmul_rn(g, g), vv)));
-        const float step = __fdiv_rn(__fmul_rn(sc.lr_t, mm), __fadd_rn(__fsqrt_rn(vv), 1e-7f));
-        m[i * DIM + c] = mm;
-        v[i * DIM + c] = vv;
-        y_next[i * DIM + c] = __fsub_rn(yi[c], step);
-        if (grad_out) grad_out[i * DIM + c] = g;
-      }
-      if (want_loss) row_loss[i] = lacc;
-    }
+    if (want_loss) p.row_loss[i] = lacc;
   }
+}
+
+template <int DIM>
+__global__ void __launch_bounds__(256) grad_adam_kernel(const GradArgs p, int itr) {
+  const Sched sc = p.sched[itr];
+  const int gl = threadIdx.x & (GRAD_G - 1);
+  const uint64_t groups = static_cast<uint64_t>(gridDim.x) * (blockDim.x / GRAD_G);
+  const unsigned gmask = ((1u << GRAD_G) - 1u) << ((threadIdx.x & 31) & ~(GRAD_G - 1));
+  for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * (blockDim.x / GRAD_G) + threadIdx.x / GRAD_G; i < p.n;
+       i += groups) {
+    const uint32_t s0 = p.rp[3 * i], s1 = p.rp[3 * i + 1], s2 = p.rp[3 * i + 2], s3 = p.rp[3 * i + 3];
+    if (s3 - s0 > GRAD_LONG) continue;  // grad_adam_long_kernel's
+    grad_adam_row<DIM, false>(p, sc, i, s0, s1, s2, s3, gl, gmask);
+  }
+}
+
+// Rows of more than GRAD_LONG entries (points that thousands of others drew as neighbour), a warp each, beside
+// grad_adam_kernel: walked by eight lanes, one such row outlasted all others together (60,000 image-like rows,
+// near-black images in up to ~7,000 lists: 120 us an iteration with eight lanes and two entries in flight, 54 us with
+// the warp). A kernel of its own: its registers in the other one cost the 1M x 128 fit 2 to 15 %.
+template <int DIM>
+__global__ void __launch_bounds__(256) grad_adam_long_kernel(const GradArgs p, int itr) {
+  const uint32_t q = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (q >= p.n_long) return;
+  const uint64_t i = p.long_rows[q];
+  const Sched sc = p.sched[itr];
+  grad_adam_row<DIM, true>(p, sc, i, p.rp[3 * i], p.rp[3 * i + 1], p.rp[3 * i + 2], p.rp[3 * i + 3], threadIdx.x & 31,
+                           0xFFFFFFFFu);
+}
+
+// The rows with more than GRAD_LONG entries, in any order (each is summed by itself).
+__global__ void long_rows_kernel(const uint32_t* __restrict__ rp, uint64_t n, uint32_t* __restrict__ rows,
+                                 uint32_t* __restrict__ count) {
+  const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i < n && rp[3 * i + 3] - rp[3 * i] > GRAD_LONG) rows[atomicAdd(count, 1u)] = static_cast<uint32_t>(i);
 }
 
 // Sum of the per-row losses in a fixed order; each pair was counted at both endpoints.
@@ -527,21 +634,22 @@ __global__ void __launch_bounds__(1024) loss_reduce_kernel(const float* __restri
   if (threadIdx.x == 0) *out = static_cast<float>(0.5 * red[0]);
 }
 
-using GradFn = void (*)(const float*, float*, float*, float*, const uint32_t*, const uint32_t*, uint64_t, const Sched*,
-                        int, float, float, float*, float*, int);
+using GradFn = void (*)(const GradArgs, int);
+struct GradFns {
+  GradFn rows, long_rows;
+};
 
-template <int G>
-GradFn pick_grad_kernel(uint64_t dim) {
+GradFns pick_grad_kernel(uint64_t dim) {
   switch (dim) {
-    case 1: return grad_adam_kernel<G, 1>;
-    case 2: return grad_adam_kernel<G, 2>;
-    case 3: return grad_adam_kernel<G, 3>;
-    case 4: return grad_adam_kernel<G, 4>;
-    case 5: return grad_adam_kernel<G, 5>;
-    case 6: return grad_adam_kernel<G, 6>;
-    case 7: return grad_adam_kernel<G, 7>;
-    case 8: return grad_adam_kernel<G, 8>;
-    default: return nullptr;
+    case 1: return {grad_adam_kernel<1>, grad_adam_long_kernel<1>};
+    case 2: return {grad_adam_kernel<2>, grad_adam_long_kernel<2>};
+    case 3: return {grad_adam_kernel<3>, grad_adam_long_kernel<3>};
+    case 4: return {grad_adam_kernel<4>, grad_adam_long_kernel<4>};
+    case 5: return {grad_adam_kernel<5>, grad_adam_long_kernel<5>};
+    case 6: return {grad_adam_kernel<6>, grad_adam_long_kernel<6>};
+    case 7: return {grad_adam_kernel<7>, grad_adam_long_kernel<7>};
+    case 8: return {grad_adam_kernel<8>, grad_adam_long_kernel<8>};
+    default: return {};
   }
 }
 
@@ -688,8 +796,15 @@ void build_csr(Ctx& c, uint64_t n, const uint32_t* d_pnn, uint64_t n_nn, const u
   seg_sort_small_kernel<<<g, SEG_WARPS * 32, 0, c.stream>>>(out.row_ptr.get(), skip, out.col.get(), nseg, big.get(),
                                                            big.get() + nseg);
   PM_LAUNCHED();
+  // at most 2 pairs / GRAD_LONG rows can be long
+  out.long_rows.alloc(c, total / GRAD_LONG + 2);
+  uint32_t* n_long = out.long_rows.get() + total / GRAD_LONG + 1;
+  PM_CUDA(cudaMemsetAsync(n_long, 0, sizeof(uint32_t), c.stream));
+  long_rows_kernel<<<ceil_div(n, 256), 256, 0, c.stream>>>(out.row_ptr.get(), n, out.long_rows.get(), n_long);
+  PM_LAUNCHED();
   uint32_t nbig = 0;
   PM_CUDA(cudaMemcpyAsync(&nbig, big.get() + nseg, sizeof(uint32_t), cudaMemcpyDeviceToHost, c.stream));
+  PM_CUDA(cudaMemcpyAsync(&out.n_long, n_long, sizeof(uint32_t), cudaMemcpyDeviceToHost, c.stream));
   PM_CUDA(cudaStreamSynchronize(c.stream));
   if (nbig > 0) {
     const size_t smem = SEG_MID * sizeof(uint32_t);
@@ -745,6 +860,40 @@ void init_random_device(Ctx& c, uint64_t n, uint64_t dim, uint64_t seed, float* 
   PM_LAUNCHED();
 }
 
+namespace {
+// A second stream that joins a capture: fork() makes it wait for the main stream, join() the main stream for it.
+// Both record their event while capturing, so the events only shape the graph.
+struct Branch {
+  cudaStream_t stream = nullptr;
+  cudaEvent_t ev[2] = {};
+  explicit Branch(bool on) {
+    if (!on) return;
+    cudaError_t e = cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking);
+    for (auto& x : ev)
+      if (e == cudaSuccess) e = cudaEventCreateWithFlags(&x, cudaEventDisableTiming);
+    if (e != cudaSuccess) {
+      release();
+      PM_CUDA(e);
+    }
+  }
+  bool fork(cudaStream_t main) {
+    return cudaEventRecord(ev[0], main) == cudaSuccess && cudaStreamWaitEvent(stream, ev[0], 0) == cudaSuccess;
+  }
+  bool join(cudaStream_t main) {
+    return cudaEventRecord(ev[1], stream) == cudaSuccess && cudaStreamWaitEvent(main, ev[1], 0) == cudaSuccess;
+  }
+  void release() {
+    for (auto& x : ev)
+      if (x) cudaEventDestroy(x);
+    if (stream) cudaStreamDestroy(stream);
+    stream = nullptr;
+  }
+  ~Branch() { release(); }
+  Branch(const Branch&) = delete;
+  Branch& operator=(const Branch&) = delete;
+};
+}  // namespace
+
 double& last_graph_setup_ms() {
   static thread_local double v = 0.0;
   return v;
@@ -754,8 +903,7 @@ void optimize_device(Ctx& c, const Csr& csr, const OptimizeArgs& a) {
   const uint64_t n = a.n, dim = a.dim;
   if (a.itr_end <= a.itr_begin || n == 0 || dim == 0) return;
   PM_REQUIRE(dim <= 8, PACMAP_ERR_UNSUPPORTED, "the optimiser supports embedding dimensions 1..8");
-  constexpr int G = 8;
-  GradFn fn = pick_grad_kernel<G>(dim);
+  const GradFns fns = pick_grad_kernel(dim);
   const uint64_t total_iters = a.p1 + a.p2 + a.p3;
   const uint64_t sched_len = std::max<uint64_t>(total_iters, a.itr_end);
   std::vector<Sched> hs(sched_len);
@@ -772,10 +920,23 @@ void optimize_device(Ctx& c, const Csr& csr, const OptimizeArgs& a) {
     loss_dev.alloc(c, iters);
   }
   int per_sm = 0;
-  PM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 256, 0));
-  const unsigned grid = static_cast<unsigned>(
-      std::max<uint64_t>(1, std::min<uint64_t>(ceil_div(n, 256 / G), static_cast<uint64_t>(c.sm_count) * std::max(per_sm, 1))));
+  PM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fns.rows, 256, 0));
+  const unsigned grid = static_cast<unsigned>(std::max<uint64_t>(
+      1, std::min<uint64_t>(ceil_div(n, 256 / GRAD_G), static_cast<uint64_t>(c.sm_count) * std::max(per_sm, 1))));
   float* bufs[2] = {a.d_y, yb.get()};
+  GradArgs ga{};
+  ga.m = a.d_m;
+  ga.v = a.d_v;
+  ga.rp = csr.row_ptr.get();
+  ga.col = csr.col.get();
+  ga.n = n;
+  ga.long_rows = csr.long_rows.get();
+  ga.n_long = csr.n_long;
+  ga.sched = sched.get();
+  ga.a1 = a1;
+  ga.a2 = a2;
+  ga.row_loss = a.h_loss ? row_loss.get() : nullptr;
+  Branch branch(csr.n_long > 0);  // the long rows run beside the others
 
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
@@ -786,10 +947,17 @@ void optimize_device(Ctx& c, const Csr& csr, const OptimizeArgs& a) {
   std::string capture_msg;
   for (uint64_t itr = a.itr_begin; itr < a.itr_end; ++itr) {
     const int src = static_cast<int>((itr - a.itr_begin) & 1), dst = src ^ 1;
-    fn<<<grid, 256, 0, c.stream>>>(bufs[src], bufs[dst], a.d_m, a.d_v, csr.row_ptr.get(), csr.col.get(), n,
-                                   sched.get(), static_cast<int>(itr), a1, a2, a.h_loss ? row_loss.get() : nullptr,
-                                   (itr + 1 == a.itr_end) ? a.d_grad_last : nullptr, 0);
+    ga.y_cur = bufs[src];
+    ga.y_next = bufs[dst];
+    ga.grad_out = (itr + 1 == a.itr_end) ? a.d_grad_last : nullptr;
+    if (csr.n_long > 0) {
+      capture_ok = branch.fork(c.stream) && capture_ok;
+      fns.long_rows<<<ceil_div(csr.n_long, 8), 256, 0, branch.stream>>>(ga, static_cast<int>(itr));
+      ++launches;
+    }
+    fns.rows<<<grid, 256, 0, c.stream>>>(ga, static_cast<int>(itr));
     ++launches;
+    if (csr.n_long > 0) capture_ok = branch.join(c.stream) && capture_ok;
     if (a.h_loss) {
       loss_reduce_kernel<<<1, 1024, 0, c.stream>>>(row_loss.get(), n, loss_dev.get() + (itr - a.itr_begin));
       ++launches;
@@ -836,15 +1004,26 @@ void gradient_device(Ctx& c, const Csr& csr, const float* d_y, uint64_t n, uint6
                      float w_fp, float* d_grad, float* h_loss) {
   if (n == 0 || dim == 0) return;
   PM_REQUIRE(dim <= 8, PACMAP_ERR_UNSUPPORTED, "the optimiser supports embedding dimensions 1..8");
-  constexpr int G = 8;
-  GradFn fn = pick_grad_kernel<G>(dim);
+  const GradFns fns = pick_grad_kernel(dim);
   const Sched hs{w_nn, w_mn, w_fp, 0.0f};
   DevBuf<Sched> sched(c, 1);
   DevBuf<float> row_loss(c, n), loss_dev(c, 1);
   PM_CUDA(cudaMemcpyAsync(sched.get(), &hs, sizeof(Sched), cudaMemcpyHostToDevice, c.stream));
-  const unsigned grid = static_cast<unsigned>(std::min<uint64_t>(ceil_div(n, 256 / G), c.sm_count * 8ull));
-  fn<<<grid, 256, 0, c.stream>>>(d_y, nullptr, nullptr, nullptr, csr.row_ptr.get(), csr.col.get(), n, sched.get(), 0,
-                                 0.0f, 0.0f, row_loss.get(), d_grad, 1);
+  const unsigned grid = static_cast<unsigned>(std::min<uint64_t>(ceil_div(n, 256 / GRAD_G), c.sm_count * 8ull));
+  GradArgs ga{};
+  ga.y_cur = d_y;
+  ga.rp = csr.row_ptr.get();
+  ga.col = csr.col.get();
+  ga.n = n;
+  ga.long_rows = csr.long_rows.get();
+  ga.n_long = csr.n_long;
+  ga.sched = sched.get();
+  ga.row_loss = row_loss.get();
+  ga.grad_out = d_grad;
+  ga.grad_only = 1;
+  fns.rows<<<grid, 256, 0, c.stream>>>(ga, 0);
+  PM_LAUNCHED();
+  if (csr.n_long > 0) fns.long_rows<<<ceil_div(csr.n_long, 8), 256, 0, c.stream>>>(ga, 0);
   PM_LAUNCHED();
   loss_reduce_kernel<<<1, 1024, 0, c.stream>>>(row_loss.get(), n, loss_dev.get());
   PM_LAUNCHED();
