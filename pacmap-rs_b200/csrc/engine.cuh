@@ -81,10 +81,19 @@ struct KnnShard {
 // mode PACMAP_KNN_APPROX searches approximately when n >= approx_threshold (exactly below it).
 void knn_exact_device(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint64_t kp, int mode, uint32_t* d_idx,
                       float* d_dist, const KnnShard& shard = KnnShard(), uint64_t approx_threshold = 0);
-// Exact kNN of a subset of rows (query ids in d_rows) against all rows.
+// The keys that each 32 query rows of a list are compared with: group g (rows 32 g to 32 g + 31 of the list) has
+// counts[g * slices + y] indices from cols[g * group_stride + y * slice_cols] on, for each slice y. d_idx and d_dist
+// hold, at the rows' own places, K points each that are among the keys: farther points are not kept.
+struct KnnKeyLists {
+  const uint32_t* cols = nullptr;
+  const int* counts = nullptr;
+  uint64_t slices = 1, slice_cols = 0, group_stride = 0;
+};
+// Exact kNN of a subset of rows (query ids in d_rows) against all rows, or against their key lists.
 // scatter: results go to the rows' own places (row r -> d_idx[r * kp]) instead of list order.
 void knn_rows_simt(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint64_t kp, const uint32_t* d_rows,
-                   uint64_t n_rows, uint32_t* d_idx, float* d_dist, bool scatter = false);
+                   uint64_t n_rows, uint32_t* d_idx, float* d_dist, bool scatter = false,
+                   const KnnKeyLists* lists = nullptr);
 
 // ---- pairs.cu ----
 void sigma_device(Ctx& c, const float* d_kd, uint64_t n, uint64_t kp, float* d_sig);

@@ -8,8 +8,8 @@
 //
 //   * knn_simt_kernel: every distance in the reference's exact f32 order (distance.rs:50-75) on CUDA
 //     cores, each block keeping the running k' best (distance key, index) of 32 query rows in shared
-//     memory. Used for small n, for any d, and as the fallback for rows the tensor-core filter
-//     (knn_tc.cu) cannot settle. When there are too few query rows to fill the GPU, the keys are split
+//     memory. Used for small n, for any d, and for rows the tensor-core filter (knn_tc.cu) cannot settle,
+//     against all rows or (LIST) against the columns that its second run left for the 32 rows. When there are too few query rows to fill the GPU, the keys are split
 //     into slices (grid y); each slice writes its own k' best per row and knn_merge_kernel merges
 //     them (the keys are totally ordered, so the merged lists are the same).
 #include "engine.cuh"
@@ -25,11 +25,13 @@ constexpr int SQ_LD = SQ_DC + 4;  // smem row stride (floats): 16-byte aligned, 
 constexpr int SQ_THREADS = 256;
 constexpr int SQ_MAX_K = 448;     // P = next_pow2(K + KT) <= 512
 
+template <bool LIST>
 __global__ void __launch_bounds__(SQ_THREADS) knn_simt_kernel(const float* __restrict__ x, uint64_t n, int d, int K,
                                                               int P, const uint32_t* __restrict__ rows,
                                                               uint64_t n_rows, uint32_t* __restrict__ out_idx,
                                                               float* __restrict__ out_dist, int scatter,
-                                                              uint64_t slice, uint64_t* __restrict__ part) {
+                                                              uint64_t slice, uint64_t* __restrict__ part,
+                                                              const KnnKeyLists kl) {
   extern __shared__ __align__(16) unsigned char smem[];
   float* qs = reinterpret_cast<float*>(smem);
   float* ks = qs + SQ_QB * SQ_LD;
@@ -37,6 +39,7 @@ __global__ void __launch_bounds__(SQ_THREADS) knn_simt_kernel(const float* __res
   __shared__ int stage_cnt[SQ_QB];
   __shared__ uint64_t theta[SQ_QB];
   __shared__ uint64_t qrow[SQ_QB];
+  __shared__ uint32_t kid[SQ_KT];  // LIST: the tile's keys
 
   const int tid = threadIdx.x;
   const int kt = tid & (SQ_KT - 1);
@@ -48,6 +51,10 @@ __global__ void __launch_bounds__(SQ_THREADS) knn_simt_kernel(const float* __res
     theta[tid] = ~0ull;
     const uint64_t s = slot0 + tid;
     qrow[tid] = (s < n_rows) ? (rows ? static_cast<uint64_t>(rows[s]) : s) : ~0ull;
+    if (LIST && s < n_rows) {  // keep what is not farther than the K-th of the points that the row already has
+      const uint64_t o = qrow[tid] * K + K - 1;
+      theta[tid] = ((static_cast<uint64_t>(total_key(out_dist[o])) << 32) | out_idx[o]) + 1;
+    }
   }
   for (int e = tid; e < SQ_QB * P; e += SQ_THREADS) lists[e] = ~0ull;
   __syncthreads();
@@ -56,8 +63,10 @@ __global__ void __launch_bounds__(SQ_THREADS) knn_simt_kernel(const float* __res
   // rows staged in 16-byte pieces when every row starts on a 16-byte boundary
   const bool vec4 = (d % 4 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15u) == 0);
   // keys [kbeg, kend) of this block's slice (slice is a multiple of SQ_KT)
-  const uint64_t kbeg = static_cast<uint64_t>(blockIdx.y) * slice;
-  const uint64_t kend = kbeg + slice < n ? kbeg + slice : n;
+  const uint64_t kbeg = LIST ? 0 : static_cast<uint64_t>(blockIdx.y) * slice;
+  const uint64_t kend = LIST ? static_cast<uint64_t>(kl.counts[blockIdx.x * kl.slices + blockIdx.y])
+                             : (kbeg + slice < n ? kbeg + slice : n);
+  const uint32_t* cols = LIST ? kl.cols + blockIdx.x * kl.group_stride + blockIdx.y * kl.slice_cols : nullptr;
   for (uint64_t key0 = kbeg; key0 < kend; key0 += SQ_KT) {
     float acc[8][8];
 #pragma unroll
@@ -65,6 +74,10 @@ __global__ void __launch_bounds__(SQ_THREADS) knn_simt_kernel(const float* __res
 #pragma unroll
       for (int l = 0; l < 8; ++l) acc[q][l] = 0.0f;
 
+    if (LIST) {  // the previous tile's last use of kid is behind its closing barrier
+      if (tid < SQ_KT) kid[tid] = key0 + tid < kend ? cols[key0 + tid] : 0u;
+      if (nc8 == 0) __syncthreads();
+    }
     for (int dbase = 0; dbase < nc8; dbase += SQ_DC) {
       const int dlen = min(SQ_DC, nc8 - dbase);
       __syncthreads();
@@ -82,9 +95,9 @@ __global__ void __launch_bounds__(SQ_THREADS) knn_simt_kernel(const float* __res
         for (int e = tid; e < SQ_KT * (SQ_DC / 4); e += SQ_THREADS) {
           const int kk = e / (SQ_DC / 4), c4 = e % (SQ_DC / 4);
           if (c4 >= q4) continue;
-          const uint64_t j = key0 + kk;
-          const float4 v = (j < kend) ? *reinterpret_cast<const float4*>(x + j * d + dbase + 4 * c4)
-                                      : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          const uint64_t j = LIST ? kid[kk] : key0 + kk;
+          const float4 v = (key0 + kk < kend) ? *reinterpret_cast<const float4*>(x + j * d + dbase + 4 * c4)
+                                              : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
           *reinterpret_cast<float4*>(&ks[kk * SQ_LD + 4 * c4]) = v;
         }
       } else {
@@ -95,8 +108,8 @@ __global__ void __launch_bounds__(SQ_THREADS) knn_simt_kernel(const float* __res
         }
         for (int e = tid; e < SQ_KT * dlen; e += SQ_THREADS) {
           const int kk = e / dlen, cc = e - kk * dlen;
-          const uint64_t j = key0 + kk;
-          ks[kk * SQ_LD + cc] = (j < kend) ? x[j * d + dbase + cc] : 0.0f;
+          const uint64_t j = LIST ? kid[kk] : key0 + kk;
+          ks[kk * SQ_LD + cc] = (key0 + kk < kend) ? x[j * d + dbase + cc] : 0.0f;
         }
       }
       __syncthreads();
@@ -119,7 +132,8 @@ __global__ void __launch_bounds__(SQ_THREADS) knn_simt_kernel(const float* __res
       }
     }
 
-    const uint64_t j = key0 + kt;
+    const uint64_t j = LIST ? kid[kt] : key0 + kt;
+    const bool have = key0 + kt < kend;
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
       const int qi = qg * 8 + q;
@@ -127,7 +141,7 @@ __global__ void __launch_bounds__(SQ_THREADS) knn_simt_kernel(const float* __res
       float t = 0.0f;
 #pragma unroll
       for (int l = 0; l < 8; ++l) t = __fadd_rn(t, acc[q][l]);
-      if (r == ~0ull || j >= kend || j == r) continue;
+      if (r == ~0ull || !have || j == r) continue;
       for (int e = nc8; e < d; ++e) {
         const float df = __fsub_rn(x[r * d + e], x[j * d + e]);
         t = __fadd_rn(t, __fmul_rn(df, df));
@@ -150,7 +164,7 @@ __global__ void __launch_bounds__(SQ_THREADS) knn_simt_kernel(const float* __res
       warp_bitonic_sort_u64(L, P);
       if (lane == 0) {
         stage_cnt[qi] = 0;
-        theta[qi] = L[K - 1];
+        theta[qi] = min(theta[qi], L[K - 1]);
       }
       __syncwarp();
     }
@@ -204,7 +218,7 @@ __global__ void __launch_bounds__(MG_WARPS * 32) knn_merge_kernel(const uint64_t
 }  // namespace
 
 void knn_rows_simt(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint64_t kp, const uint32_t* d_rows,
-                   uint64_t n_rows, uint32_t* d_idx, float* d_dist, bool scatter) {
+                   uint64_t n_rows, uint32_t* d_idx, float* d_dist, bool scatter, const KnnKeyLists* lists) {
   if (n_rows == 0 || kp == 0) return;
   PM_REQUIRE(kp <= SQ_MAX_K, PACMAP_ERR_UNSUPPORTED,
              "exact kNN supports at most " + std::to_string(SQ_MAX_K) + " neighbours per row");
@@ -212,11 +226,12 @@ void knn_rows_simt(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint64_t kp
   const int K = static_cast<int>(kp);
   const int P = next_pow2(K + SQ_KT);
   const size_t smem = static_cast<size_t>(SQ_QB + SQ_KT) * SQ_LD * sizeof(float) + static_cast<size_t>(SQ_QB) * P * 8;
-  PM_CUDA(cudaFuncSetAttribute(knn_simt_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  const auto kern = lists ? knn_simt_kernel<true> : knn_simt_kernel<false>;
+  PM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
   // Key slices: enough blocks for two waves when the query rows alone do not fill the GPU; every slice
   // keeps at least 4096 keys (a multiple of the key tile).
   int per_sm = 1;
-  PM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, knn_simt_kernel, SQ_THREADS, smem));
+  PM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, SQ_THREADS, smem));
   const uint64_t row_blocks = ceil_div(n_rows, SQ_QB);
   const uint64_t want = 2ull * c.sm_count * static_cast<uint64_t>(std::max(per_sm, 1));
   uint64_t slices = std::min<uint64_t>((want + row_blocks - 1) / row_blocks, std::max<uint64_t>(n / 4096, 1));
@@ -225,12 +240,13 @@ void knn_rows_simt(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint64_t kp
   uint64_t slice = (n + slices - 1) / slices;
   slice = (slice + SQ_KT - 1) / SQ_KT * SQ_KT;
   slices = (n + slice - 1) / slice;
+  if (lists) slices = lists->slices;
   DevBuf<uint64_t> part;
   if (slices > 1) part.alloc(c, n_rows * slices * static_cast<uint64_t>(K));
   const dim3 grid(static_cast<unsigned>(row_blocks), static_cast<unsigned>(slices));
-  knn_simt_kernel<<<grid, SQ_THREADS, smem, c.stream>>>(d_x, n, static_cast<int>(d), K, P, d_rows, n_rows, d_idx,
-                                                         d_dist, scatter ? 1 : 0, slice,
-                                                         slices > 1 ? part.get() : nullptr);
+  kern<<<grid, SQ_THREADS, smem, c.stream>>>(d_x, n, static_cast<int>(d), K, P, d_rows, n_rows, d_idx, d_dist,
+                                              scatter ? 1 : 0, slice, slices > 1 ? part.get() : nullptr,
+                                              lists ? *lists : KnnKeyLists());
   PM_LAUNCHED();
   if (slices > 1) {
     const int P2 = next_pow2(2 * K);

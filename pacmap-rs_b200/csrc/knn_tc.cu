@@ -23,8 +23,11 @@
 //  3. knn_rerank_kernel: the final threshold, then the reference's exact f32 distance of every
 //     survivor (gathered from a lane-grouped copy of x by 16-byte loads, each lane adding its terms in
 //     the reference's order), sorted by (distance, index): the rows of knn.rs.
-//  Rows whose candidate band does not fit the buffer (e.g. thousands of exact duplicates) are
-//  recomputed by the exact SIMT kernel.
+//  4. Rows whose candidate band does not fit the buffer (hundreds of exact duplicates, or distances small
+//     against the norms) go through the filter again in blocks of their own, with a fixed threshold from
+//     the exact distances of the candidates they had; every 32 of them keep one list of the columns that
+//     any of the 32 may have as neighbour, and the exact SIMT kernel runs over that list. Rows with non-finite
+//     data are recomputed by the exact SIMT kernel over all columns.
 //
 // Every mbarrier wait is bounded (2 s of %globaltimer): a kernel that gives up raises DEV_ERR_TIMEOUT
 // and returns after releasing its tensor memory. No TMA multicast is used anywhere.
@@ -557,15 +560,20 @@ __device__ int g_debug_stall_loads = 0;
 
 // K blocks of 64 elements: KP = 64 * KB (KB = 0: run-time kb_rt, MODE_STREAM only); candidate buffer
 // C = 32 * PER per row.
-template <int KB, int PER, int MODE>
+// WIDE: the rows are a gathered list (amap over their operand rows, nrm / ge by list position) whose thresholds are
+// given (resume_theta) and stay fixed. Grid y splits the column tiles, and each epilogue warp writes the columns (as
+// original indices) that pass for any of its 32 rows: group g = row / 32 has n_pad places in wide_cols, slice y's
+// from its first column on, and its count in cand_cnt[g * gridDim.y + y].
+template <int KB, int PER, int MODE, bool WIDE = false>
 __global__ void __launch_bounds__(TC_THREADS, 1) knn_filter_kernel(
-    const __grid_constant__ CUtensorMap hmap, const __grid_constant__ CUtensorMap gmap, uint64_t n, uint64_t n_pad,
+    const __grid_constant__ CUtensorMap hmap, const __grid_constant__ CUtensorMap gmap,
+    const __grid_constant__ CUtensorMap amap, uint64_t n, uint64_t n_pad,
     int kb_rt, uint32_t idesc, const float2* __restrict__ ge, const float* __restrict__ nrm,
     const uint32_t* __restrict__ perm, int rank, uint2* __restrict__ cand, int* __restrict__ cand_cnt,
     uint32_t* __restrict__ overflow_rows, uint32_t* __restrict__ n_overflow, uint32_t* __restrict__ err,
     int block_offset, const uint32_t* __restrict__ tile_ptr, const uint32_t* __restrict__ tile_list,
     const float* __restrict__ resume_theta, const uint32_t* __restrict__ e4max_bits,
-    unsigned long long* __restrict__ counters) {
+    unsigned long long* __restrict__ counters, uint32_t* __restrict__ wide_cols) {
   using L = FilterLayout<KB, MODE>;
   constexpr int NST = L::NST;
   constexpr int C = 32 * PER;
@@ -589,8 +597,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) knn_filter_kernel(
   const int ntiles = static_cast<int>(n_pad / TC_BN);
   // the column tiles this block visits: all of them in the sweep order, or (approximate kNN) its list
   const uint32_t lbase = tile_ptr ? tile_ptr[blk] : 0u;
-  const int nt = tile_ptr ? static_cast<int>(tile_ptr[blk + 1] - lbase) : ntiles;
+  const int per_slice = WIDE ? (ntiles + static_cast<int>(gridDim.y) - 1) / static_cast<int>(gridDim.y) : 0;
+  const int slice0 = WIDE ? min(static_cast<int>(blockIdx.y) * per_slice, ntiles) : 0;
+  const int nt = WIDE ? min(per_slice, ntiles - slice0)
+                      : (tile_ptr ? static_cast<int>(tile_ptr[blk + 1] - lbase) : ntiles);
   auto tile_at = [&](int t) -> int {
+    if (WIDE) return slice0 + t;
     return tile_ptr ? static_cast<int>(tile_list[lbase + t]) : sweep_tile(t, blk, ntiles);
   };
 
@@ -631,7 +643,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) knn_filter_kernel(
         mbar_expect_tx(&sh->a_full, L::A_RES);
         for (int h = 0; h < 2; ++h)
           for (int kb = 0; kb < KB; ++kb)
-            tma_load_2d(a_smem + (h * KB + kb) * KB_BYTES, &hmap, &sh->a_full, kb * 64, static_cast<int>(row0 + h * 128));
+            tma_load_2d(a_smem + (h * KB + kb) * KB_BYTES, &amap, &sh->a_full, kb * 64, static_cast<int>(row0 + h * 128));
       }
       const int total = nt * nch;
       int issued = 0, s = 0, ph = 0;
@@ -653,7 +665,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) knn_filter_kernel(
             tma_load_2d(st, &hmap, &sh->full[s], ch * 64, tile * TC_BN);
             if (MODE == MODE_STREAM)
               for (int h = 0; h < 2; ++h)
-                tma_load_2d(st + (1 + h) * KB_BYTES, &hmap, &sh->full[s], ch * 64, static_cast<int>(row0 + h * 128));
+                tma_load_2d(st + (1 + h) * KB_BYTES, &amap, &sh->full[s], ch * 64, static_cast<int>(row0 + h * 128));
           }
           if (ch == 0) tma_load_2d(g_smem + s * G_BYTES, &gmap, &sh->full[s], 0, tile * TC_BN);
           ++issued;
@@ -752,7 +764,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) knn_filter_kernel(
     const bool valid = row < n;
     float theta = valid ? 3.402823466e+38f : -__int_as_float(0x7f800000);
     int cnt = 0;
-    if (resume_theta && valid) {
+    if (WIDE) {
+      if (valid) theta = resume_theta[row];
+    } else if (resume_theta && valid) {
       // continue from an earlier pass over other tiles: its compacted buffer and threshold (an overflowed
       // row stays overflowed; it is already listed for the exact fallback)
       const int c0 = cand_cnt[row];
@@ -766,7 +780,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) knn_filter_kernel(
     const float n_i = valid ? nrm[row] : 0.0f;
     const float e4_i = valid ? ge[row].y : 0.0f;
     const uint64_t cbase = row * static_cast<uint64_t>(C);
-    const float e4max = __uint_as_float(*e4max_bits);
+    const float e4max = WIDE ? 0.0f : __uint_as_float(*e4max_bits);
+    const uint64_t wgroup = (row0 >> 5) + half * 4 + quad;
+    uint32_t* wide_out = WIDE ? wide_cols + wgroup * n_pad + static_cast<uint64_t>(slice0) * TC_BN : nullptr;
     bool ok = true;
     uint32_t n_ins = 0, n_comp = 0;  // this row's insertions and compactions (statistics)
     const int cnt0 = cnt;            // entries carried over from an earlier pass
@@ -780,6 +796,19 @@ __global__ void __launch_bounds__(TC_THREADS, 1) knn_filter_kernel(
       const float m = fmaxf(fmax3(m8[0], m8[1], m8[2]), m8[3]);
       // v = -2 D <= theta exactly when D >= -theta / 2 (both scalings by 2 are exact)
       const float hth = -0.5f * theta;
+      if (WIDE) {
+        if (!__any_sync(0xFFFFFFFFu, m >= hth)) return;
+        bool mine = false;  // lane c: does column c pass for any of the 32 rows?
+#pragma unroll
+        for (int c = 0; c < 32; ++c) {
+          const bool any = __any_sync(0xFFFFFFFFu, Dv[c] >= hth);
+          if (lane == c) mine = any;
+        }
+        const unsigned bal = __ballot_sync(0xFFFFFFFFu, mine);
+        if (mine) wide_out[cnt + __popc(bal & ((1u << lane) - 1u))] = perm[colb + lane];
+        cnt += __popc(bal);
+        return;
+      }
       if (__any_sync(0xFFFFFFFFu, m >= hth)) {
         // every column of the 32 without a branch: a predicated store of (j, v = -2 D) that also returns the
         // count (a divergent branch per column, or a vote per 8 columns, cost more than the column's work)
@@ -811,6 +840,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) knn_filter_kernel(
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&sh->tmem_empty[acc]);
+      if (WIDE) continue;  // a slice's places hold all of its columns
       // Compact full buffers so that the next tile (<= 128 insertions) always fits.
       // The next row's entries are loaded before the current row is compacted (their latency overlaps).
       unsigned need = __ballot_sync(0xFFFFFFFFu, cnt > C - TC_BN);
@@ -844,7 +874,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) knn_filter_kernel(
             if (cnt > C - TC_BN) {  // the band does not fit: exact recomputation later
               theta = -__int_as_float(0x7f800000);
               cnt = 0;
-              overflow_rows[atomicAdd(n_overflow, 1u)] = perm[row];
+              overflow_rows[atomicAdd(n_overflow, 1u)] = static_cast<uint32_t>(row);
             }
             n_ins += static_cast<uint32_t>(m - cnt);  // the entries this compaction dropped
           }
@@ -861,7 +891,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1) knn_filter_kernel(
       atomicOr(err, DEV_ERR_TIMEOUT);
       sh->abort_flag = 1;
     }
-    if (valid) cand_cnt[row] = (theta == -__int_as_float(0x7f800000)) ? -1 : cnt;
+    if (WIDE) {
+      if (lane == 0) cand_cnt[wgroup * gridDim.y + blockIdx.y] = cnt;
+    } else if (valid) {
+      cand_cnt[row] = (theta == -__int_as_float(0x7f800000)) ? -1 : cnt;
+    }
     n_ins += static_cast<uint32_t>(cnt - cnt0);  // dropped + left = inserted + present at the start
     if (counters) {
       const uint32_t wi = __reduce_add_sync(0xFFFFFFFFu, n_ins), wc = __reduce_add_sync(0xFFFFFFFFu, n_comp);
@@ -1083,6 +1117,95 @@ __global__ void __launch_bounds__(WARPS * 32) knn_rerank_kernel(
   }
 }
 
+// ---------------------------------------------------------------------------------------------
+// 4. rows whose band overflowed the filter's buffer: 60,000 x 784 image-like rows leave 14,000 to 16,000 of them, with
+//    3,000 exact ties (all-black images) and bands of 4,000 to 7,000 columns. Recomputed against all columns they took
+//    75 to 150 ms of the SIMT kernel; their second filter run and the SIMT kernel over the lists take 20 to 50
+//    (knn of 60,000 x 784: 182 -> 65 ms). Buffers of thousands of entries per row, re-ranked row by row, were no gain:
+//    the ties alone overflowed them, and each row gathered its own thousands of rows from L2.
+// ---------------------------------------------------------------------------------------------
+// An overflowed row's buffer still holds a band of more than C - TC_BN entries (>= rank of them): marked with
+// that count, the re-rank gives the row the K nearest of those, provisionally.
+__global__ void overflow_mark_kernel(const uint32_t* __restrict__ rows, const uint32_t* __restrict__ count, int entries,
+                                     int* __restrict__ cand_cnt) {
+  for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < *count; t += gridDim.x * blockDim.x)
+    cand_cnt[rows[t]] = entries;
+}
+
+// The operand rows, norms and thresholds of list rows [0, m) (padding up to the grid's rows is zeroed, with threshold
+// -inf). The threshold: the K-th provisional distance U is an exact distance of the reference, so a neighbour's
+// squared distance is at most U^2; in the scaled units of v, UB = (U s)^2, and theta_from(UB - n_i - 2 e_i) keeps every
+// column whose lower bound is within it. The f32 roundings of UB and of the subtraction are covered by widening UB by
+// 2^-20 and adding 2^-21 (UB + n_i).
+__global__ void __launch_bounds__(256) wide_gather_kernel(const uint32_t* __restrict__ rows, uint32_t m,
+                                                          const uint16_t* __restrict__ H, int KP,
+                                                          const float* __restrict__ nrm, const float2* __restrict__ ge,
+                                                          const uint32_t* __restrict__ perm,
+                                                          const float* __restrict__ dist, int K, float s,
+                                                          uint16_t* __restrict__ H2, float* __restrict__ nrm2,
+                                                          float2* __restrict__ ge2, float* __restrict__ theta) {
+  const uint32_t q = blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  const uint64_t r = q < m ? rows[q] : 0;
+  const uint4* src = reinterpret_cast<const uint4*>(H + r * KP);  // KP a multiple of 64
+  uint4* dst = reinterpret_cast<uint4*>(H2 + static_cast<uint64_t>(q) * KP);
+  for (int c = lane; c < KP / 8; c += 32) dst[c] = q < m ? src[c] : make_uint4(0u, 0u, 0u, 0u);
+  if (lane != 0) return;
+  float th = -__int_as_float(0x7f800000), n_i = 0.0f;
+  float2 g = make_float2(0.0f, 0.0f);
+  if (q < m) {
+    n_i = nrm[r];
+    g = ge[r];
+    const float u = dist[static_cast<uint64_t>(perm[r]) * K + K - 1] * s;
+    const float ub = (u * u) * (1.0f + 9.5367431640625e-07f);
+    th = theta_from((ub - n_i - 0.5f * g.y) + 4.76837158203125e-07f * (ub + n_i), n_i, g.y);
+    if (!(th < 3.402823466e+38f)) th = 3.402823466e+38f;  // distances beyond f32: every column (padding has v = +inf)
+  }
+  nrm2[q] = n_i;
+  ge2[q] = g;
+  theta[q] = th;
+}
+
+// The overflow list in ascending row order (the filter's atomics leave it in any): neighbouring rows share most of their
+// candidates, and each 32 rows of the list share one. Flags per row, counts per 1,024 rows, their offsets, placement.
+constexpr int OL_ROWS = 1024;
+__global__ void overflow_flag_kernel(const uint32_t* __restrict__ rows, uint32_t m, uint8_t* __restrict__ flags) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < m) flags[rows[t]] = 1;
+}
+__global__ void __launch_bounds__(OL_ROWS) overflow_count_kernel(const uint8_t* __restrict__ flags, uint64_t n,
+                                                                 uint32_t* __restrict__ counts) {
+  const uint64_t r = static_cast<uint64_t>(blockIdx.x) * OL_ROWS + threadIdx.x;
+  const int c = __syncthreads_count(r < n && flags[r]);
+  if (threadIdx.x == 0) counts[blockIdx.x] = c;
+}
+__global__ void __launch_bounds__(OL_ROWS) overflow_place_kernel(const uint8_t* __restrict__ flags, uint64_t n,
+                                                                 const uint32_t* __restrict__ counts,
+                                                                 uint32_t* __restrict__ rows) {
+  __shared__ uint32_t before, warp_cnt[OL_ROWS / 32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint32_t part = 0;
+  for (uint32_t b = threadIdx.x; b < blockIdx.x; b += OL_ROWS) part += counts[b];
+  if (threadIdx.x == 0) before = 0;
+  __syncthreads();
+  if (part) atomicAdd(&before, part);  // a count: any order
+  const uint64_t r = static_cast<uint64_t>(blockIdx.x) * OL_ROWS + threadIdx.x;
+  const bool f = r < n && flags[r];
+  const unsigned bal = __ballot_sync(0xFFFFFFFFu, f);
+  if (lane == 0) warp_cnt[warp] = __popc(bal);
+  __syncthreads();
+  uint32_t pos = before + __popc(bal & ((1u << lane) - 1u));
+  for (int w = 0; w < warp; ++w) pos += warp_cnt[w];
+  if (f) rows[pos] = static_cast<uint32_t>(r);
+}
+__global__ void original_ids_kernel(const uint32_t* __restrict__ rows, uint32_t m, const uint32_t* __restrict__ perm,
+                                    uint32_t* __restrict__ ids) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < m) ids[t] = perm[rows[t]];
+}
+
+constexpr uint64_t WIDE_COLS_MAX = 1ull << 28;  // places of the column lists in one launch (1 GB)
+
 }  // namespace
 
 bool knn_tc_supported(uint64_t n, uint64_t d, uint64_t kp) {
@@ -1252,17 +1375,8 @@ bool knn_tc_device(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint64_t kp
                                                           B.get(), ge.get(), gq.get(), e4max.get());
   PM_LAUNCHED();
 
-  CUtensorMap map;
-  std::memset(&map, 0, sizeof(map));
-  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(KP), static_cast<cuuint64_t>(n_pad)};
-  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(KP) * 2};
-  const cuuint32_t box[2] = {64, 128};
+  const CUtensorMap map = make_tmap_2d_16b(H.get(), n_pad, KP, 128, bf16);
   const cuuint32_t estr[2] = {1, 1};
-  const CUresult cr = detail::get_encode_fn()(&map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2,
-                                      H.get(), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                      CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  PM_REQUIRE(cr == CUDA_SUCCESS, PACMAP_ERR_CUDA, "cuTensorMapEncodeTiled failed: " + std::to_string(cr));
   // the column term: [n_pad][16] bf16, box 16 x 128, 32-byte swizzle (x is always 0)
   CUtensorMap gmap;
   std::memset(&gmap, 0, sizeof(gmap));
@@ -1299,10 +1413,10 @@ bool knn_tc_device(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint64_t kp
     auto launch = [&](auto kern, size_t smem) {
       PM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
       if (grid == 0) return;
-      kern<<<grid, TC_THREADS, smem, c.stream>>>(map, gmap, n, n_pad, KB, idesc, ge.get(), nrm.get(), perm.get(), rank,
-                                                 cand.get(), ccnt.get(), ovf_rows, n_ovf, c.d_err,
+      kern<<<grid, TC_THREADS, smem, c.stream>>>(map, gmap, map, n, n_pad, KB, idesc, ge.get(), nrm.get(), perm.get(),
+                                                 rank, cand.get(), ccnt.get(), ovf_rows, n_ovf, c.d_err,
                                                  static_cast<int>(blk0), lptr, llist, resume_theta, e4max.get(),
-                                                 counters.get());
+                                                 counters.get(), nullptr);
     };
     const bool p16 = PER == 16;
     if (mode == MODE_STREAM) {
@@ -1388,6 +1502,8 @@ bool knn_tc_device(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint64_t kp
   st.bound_ms = bms;
 
   compact(nullptr, nullptr, counters.get() + 2);
+  overflow_mark_kernel<<<c.sm_count, 256, 0, c.stream>>>(ovf.get(), ovf.get() + n, C - TC_BN + 1, ccnt.get());
+  PM_LAUNCHED();
   const int di = static_cast<int>(d), ki = static_cast<int>(kp);
   // the re-rank reads xperm with 16-byte loads
   PM_REQUIRE((reinterpret_cast<uintptr_t>(xperm.get()) & 15u) == 0, PACMAP_ERR_CUDA,
@@ -1411,23 +1527,77 @@ bool knn_tc_device(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint64_t kp
   }
   PM_LAUNCHED();
 
-  // Rows the filter could not settle: exact SIMT recomputation, scattered into place.
   uint32_t counts[2] = {0, 0};
   unsigned long long cv[3] = {0, 0, 0};
   PM_CUDA(cudaMemcpyAsync(&counts[0], ovf.get() + n, 4, cudaMemcpyDeviceToHost, c.stream));
   PM_CUDA(cudaMemcpyAsync(&counts[1], fbk.get() + n, 4, cudaMemcpyDeviceToHost, c.stream));
   PM_CUDA(cudaMemcpyAsync(cv, counters.get(), sizeof(cv), cudaMemcpyDeviceToHost, c.stream));
   PM_CUDA(cudaStreamSynchronize(c.stream));
-  st.fallback_rows = counts[0] + counts[1];
   st.insertions = cv[0];
   st.compactions = cv[1];
   st.band_entries = cv[2];
   st.rows = n;
-  const uint32_t* lists[2] = {ovf.get(), fbk.get()};
-  for (int q = 0; q < 2; ++q) {
-    if (!counts[q]) continue;
-    knn_rows_simt(c, d_x, n, d, kp, lists[q], counts[q], d_idx, d_dist, /*scatter=*/true);
+
+  // The overflowed rows: sorted, through the filter with fixed thresholds into column lists, exact distances over
+  // those. A launch takes at most one block per SM; fewer row blocks split the column tiles.
+  if (counts[0] > 0) {
+    const uint32_t total = counts[0];
+    const uint32_t fblocks = ceil_div(n, OL_ROWS);
+    DevBuf<uint8_t> flags(c, n);
+    DevBuf<uint32_t> fcounts(c, fblocks), ids(c, total);
+    PM_CUDA(cudaMemsetAsync(flags.get(), 0, n, c.stream));
+    overflow_flag_kernel<<<ceil_div(total, 256), 256, 0, c.stream>>>(ovf.get(), total, flags.get());
+    PM_LAUNCHED();
+    overflow_count_kernel<<<fblocks, OL_ROWS, 0, c.stream>>>(flags.get(), n, fcounts.get());
+    PM_LAUNCHED();
+    overflow_place_kernel<<<fblocks, OL_ROWS, 0, c.stream>>>(flags.get(), n, fcounts.get(), ovf.get());
+    PM_LAUNCHED();
+    original_ids_kernel<<<ceil_div(total, 256), 256, 0, c.stream>>>(ovf.get(), total, perm.get(), ids.get());
+    PM_LAUNCHED();
+    const uint64_t blocks_fit = std::max<uint64_t>(1, WIDE_COLS_MAX / (n_pad * (TC_BM / 32)));
+    const uint32_t blocks_max = static_cast<uint32_t>(
+        std::min<uint64_t>({ceil_div(total, TC_BM), static_cast<uint64_t>(c.sm_count), blocks_fit}));
+    const uint32_t slices = static_cast<uint32_t>(std::min<uint64_t>(c.sm_count / blocks_max, ntl));
+    const uint64_t m_max = static_cast<uint64_t>(blocks_max) * TC_BM, groups = m_max / 32;
+    DevBuf<uint16_t> H2(c, m_max * KP);
+    DevBuf<float> nrm2(c, m_max), theta2(c, m_max);
+    DevBuf<float2> ge2(c, m_max);
+    DevBuf<uint32_t> wcols(c, groups * n_pad);
+    DevBuf<int> wcnt(c, groups * slices);
+    const CUtensorMap amap = make_tmap_2d_16b(H2.get(), m_max, KP, 128, bf16);
+    for (uint64_t q0 = 0; q0 < total; q0 += m_max) {
+      const uint32_t m = static_cast<uint32_t>(std::min<uint64_t>(m_max, total - q0));
+      const uint32_t wblocks = ceil_div(m, TC_BM);
+      wide_gather_kernel<<<wblocks * (TC_BM / 8), 256, 0, c.stream>>>(ovf.get() + q0, m, H.get(), KP, nrm.get(),
+                                                                     ge.get(), perm.get(), d_dist, ki, s, H2.get(),
+                                                                     nrm2.get(), ge2.get(), theta2.get());
+      PM_LAUNCHED();
+      auto launch = [&](auto kern, size_t smem) {
+        PM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+        kern<<<dim3(wblocks, slices), TC_THREADS, smem, c.stream>>>(
+            map, gmap, amap, m, n_pad, KB, idesc, ge2.get(), nrm2.get(), perm.get(), rank, nullptr, wcnt.get(), nullptr,
+            nullptr, c.d_err, 0, nullptr, nullptr, theta2.get(), nullptr, nullptr, wcols.get());
+        PM_LAUNCHED();
+      };
+      if (mode == MODE_STREAM) launch(knn_filter_kernel<0, 16, MODE_STREAM, true>, FilterLayout<0, MODE_STREAM>::SMEM);
+      else if (KB == 1) launch(knn_filter_kernel<1, 16, MODE_TILE, true>, FilterLayout<1, MODE_TILE>::SMEM);
+      else if (KB == 2) launch(knn_filter_kernel<2, 16, MODE_TILE, true>, FilterLayout<2, MODE_TILE>::SMEM);
+      else if (KB == 3) launch(knn_filter_kernel<3, 16, MODE_KBLOCK, true>, FilterLayout<3, MODE_KBLOCK>::SMEM);
+      else launch(knn_filter_kernel<4, 16, MODE_KBLOCK, true>, FilterLayout<4, MODE_KBLOCK>::SMEM);
+      KnnKeyLists kl;
+      kl.cols = wcols.get();
+      kl.counts = wcnt.get();
+      kl.slices = slices;
+      kl.slice_cols = (ntl + slices - 1) / slices * TC_BN;
+      kl.group_stride = n_pad;
+      knn_rows_simt(c, d_x, n, d, kp, ids.get() + q0, m, d_idx, d_dist, /*scatter=*/true, &kl);
+    }
+    c.check_errors("tensor-core kNN wide rows");
   }
+  // Rows with fewer certified candidates than neighbours: exact SIMT recomputation, scattered into place.
+  st.wide_rows = counts[0];
+  st.fallback_rows = counts[1];
+  if (counts[1]) knn_rows_simt(c, d_x, n, d, kp, fbk.get(), counts[1], d_idx, d_dist, /*scatter=*/true);
   return true;
 }
 

@@ -16,6 +16,7 @@ struct KnnTcStats {
   double filter_ms = 0.0;       // device time of the filter launch that produced the candidates
   double bound_ms = 0.0;        // device time of the pruning's bound pass, statistics and tile lists
   uint64_t fallback_rows = 0;   // rows recomputed by the exact SIMT kernel
+  uint64_t wide_rows = 0;       // rows whose band overflowed, settled over their column lists
   uint64_t tiles_full = 0;      // (row block, column tile) pairs of the full sweep
   uint64_t tiles_visited = 0;   // pairs the filter computed
   uint64_t tiles_bound = 0;     // pairs the bound pass computed
