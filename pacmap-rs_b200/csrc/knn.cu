@@ -23,7 +23,14 @@ constexpr int SQ_KT = 64;   // keys per tile
 constexpr int SQ_DC = 64;   // dimensions staged per pass (multiple of 8)
 constexpr int SQ_LD = SQ_DC + 4;  // smem row stride (floats): 16-byte aligned, conflict-free float4 rows
 constexpr int SQ_THREADS = 256;
-constexpr int SQ_MAX_K = 448;     // P = next_pow2(K + KT) <= 512
+constexpr int SQ_MAX_K = 448;     // K + KT <= 512
+// Keys per query in shared memory: its K best, then staged candidates. A list is sorted only when the next tile's
+// candidates might not fit, so the more room the fewer sorts: at K <= 64, 256 places (5 sorts over 15,000 keys, the
+// threshold standing still between them lets in a third more candidates) instead of 128 (one after nearly every
+// tile with a candidate, about 140 sorts, which were most of the time at 64 columns).
+__host__ __device__ constexpr int sq_places(int K) { return K + SQ_KT <= 256 ? 256 : 512; }
+// A block's sorts, tail and merge cost about as much as this many keys of distances.
+constexpr double SQ_SLICE_KEYS = 300.0;
 
 template <bool LIST>
 __global__ void __launch_bounds__(SQ_THREADS) knn_simt_kernel(const float* __restrict__ x, uint64_t n, int d, int K,
@@ -154,11 +161,13 @@ __global__ void __launch_bounds__(SQ_THREADS) knn_simt_kernel(const float* __res
       }
     }
     __syncthreads();
-    // Merge the staged candidates of each query into its sorted list (one warp per query).
+    // Merge the staged candidates of each query into its sorted list (one warp per query) when the next tile's
+    // might not fit, and after the last tile.
+    const bool last = key0 + SQ_KT >= kend;
     const int warp = tid >> 5, lane = tid & 31;
     for (int qi = warp; qi < SQ_QB; qi += SQ_THREADS / 32) {
       const int cnt = stage_cnt[qi];
-      if (cnt == 0) continue;
+      if (cnt == 0 || (!last && K + cnt + SQ_KT <= P)) continue;
       uint64_t* L = lists + qi * P;
       for (int e = K + cnt + lane; e < P; e += 32) L[e] = ~0ull;
       warp_bitonic_sort_u64(L, P);
@@ -224,19 +233,26 @@ void knn_rows_simt(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint64_t kp
              "exact kNN supports at most " + std::to_string(SQ_MAX_K) + " neighbours per row");
   PM_REQUIRE(n < (1ull << 32) && d < (1ull << 31), PACMAP_ERR_UNSUPPORTED, "kNN needs n < 2^32 and d < 2^31");
   const int K = static_cast<int>(kp);
-  const int P = next_pow2(K + SQ_KT);
+  const int P = sq_places(K);
   const size_t smem = static_cast<size_t>(SQ_QB + SQ_KT) * SQ_LD * sizeof(float) + static_cast<size_t>(SQ_QB) * P * 8;
   const auto kern = lists ? knn_simt_kernel<true> : knn_simt_kernel<false>;
   PM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-  // Key slices: enough blocks for two waves when the query rows alone do not fill the GPU; every slice
-  // keeps at least 4096 keys (a multiple of the key tile).
+  // Key slices (at least 512 keys each): as many as shorten the row blocks' waves over the SMs most, a block's time
+  // being its keys plus SQ_SLICE_KEYS.
   int per_sm = 1;
   PM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, SQ_THREADS, smem));
   const uint64_t row_blocks = ceil_div(n_rows, SQ_QB);
-  const uint64_t want = 2ull * c.sm_count * static_cast<uint64_t>(std::max(per_sm, 1));
-  uint64_t slices = std::min<uint64_t>((want + row_blocks - 1) / row_blocks, std::max<uint64_t>(n / 4096, 1));
-  slices = std::min<uint64_t>(slices, 1024);
-  slices = std::max<uint64_t>(slices, 1);
+  const uint64_t slots = static_cast<uint64_t>(c.sm_count) * std::max(per_sm, 1);
+  uint64_t slices = 1;
+  double best = 1e300;
+  for (uint64_t q = 1; q <= 1024 && (q == 1 || (n / q >= 512 && row_blocks * q <= 8 * slots)); ++q) {
+    const double t = static_cast<double>(ceil_div(row_blocks * q, slots)) *
+                     (static_cast<double>(n) / static_cast<double>(q) + SQ_SLICE_KEYS);
+    if (t < best) {
+      best = t;
+      slices = q;
+    }
+  }
   uint64_t slice = (n + slices - 1) / slices;
   slice = (slice + SQ_KT - 1) / SQ_KT * SQ_KT;
   slices = (n + slice - 1) / slice;
