@@ -81,7 +81,7 @@ typedef enum pacmap_knn_mode {
   PACMAP_KNN_APPROX = 4,       /* approximate at n >= approx_threshold (the reference's rule,
                                 * src/neighbors.rs:71): each row block searches only the 16 of 256
                                 * pivot cells nearest its own; returned distances stay exact. Below
-                                * the threshold (or below 16,384 rows, where the SIMT path runs) exact;
+                                * the threshold, or below 16,384 rows, exact;
                                 * pacmap_knn_exact has no threshold: approximate whenever it can be. */
   PACMAP_KNN_TENSOR_F16_FULL = 5  /* as TENSOR_F16 with every column tile computed (no pruning)     */
 } pacmap_knn_mode;

@@ -31,6 +31,7 @@ constexpr int SQ_MAX_K = 448;     // K + KT <= 512
 __host__ __device__ constexpr int sq_places(int K) { return K + SQ_KT <= 256 ? 256 : 512; }
 // A block's sorts, tail and merge cost about as much as this many keys of distances.
 constexpr double SQ_SLICE_KEYS = 300.0;
+constexpr uint64_t TC_AUTO_ROWS = 5000, TC_APPROX_ROWS = 16384;
 
 template <bool LIST>
 __global__ void __launch_bounds__(SQ_THREADS) knn_simt_kernel(const float* __restrict__ x, uint64_t n, int d, int K,
@@ -286,14 +287,19 @@ void knn_exact_device(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint64_t
                       float* d_dist, const KnnShard& shard, uint64_t approx_threshold) {
   if (n == 0 || kp == 0) return;
   PM_REQUIRE(shard.count >= 1 && shard.index < shard.count, PACMAP_ERR_INVALID_ARGUMENT, "bad kNN shard");
-  // AUTO uses the tensor cores once the O(n^2) part dominates; the TENSOR modes force them.
-  const bool approx = mode == PACMAP_KNN_APPROX && n >= approx_threshold;
+  // AUTO uses the tensor cores once the O(n^2) part dominates; the TENSOR modes force them. At 5,000 rows the two
+  // paths take the same time at 16 columns and 15 neighbours (0.66 and 0.62 ms) and the tensor cores win everywhere else
+  // (100 columns: 0.85 against 1.05 ms at 15 neighbours, 1.05 against 1.43 at 72; 784 columns: 2.9 against 4.2); at
+  // 4,000 the SIMT kernel wins up to 128 columns (100: 0.63 against 0.78). At 14,000 x 64 it is 1.2 against 4.2 ms.
+  // The approximate search starts at 16,384 rows.
+  const bool approx = mode == PACMAP_KNN_APPROX && n >= approx_threshold && n >= TC_APPROX_ROWS;
   const bool want_tc = (mode == PACMAP_KNN_TENSOR_F16 || mode == PACMAP_KNN_TENSOR_BF16 ||
                         mode == PACMAP_KNN_TENSOR_F16_FULL) ||
-                       ((mode == PACMAP_KNN_AUTO || mode == PACMAP_KNN_APPROX) && n >= 16384);
+                       ((mode == PACMAP_KNN_AUTO || mode == PACMAP_KNN_APPROX) && n >= TC_AUTO_ROWS);
+  const bool forced = mode != PACMAP_KNN_AUTO && mode != PACMAP_KNN_APPROX;
   if (want_tc && knn_tc_supported(n, d, kp)) {
     if (knn_tc_device(c, d_x, n, d, kp, mode == PACMAP_KNN_TENSOR_BF16, d_idx, d_dist, shard, approx ? 16 : 0,
-                      /*prune=*/mode != PACMAP_KNN_TENSOR_F16_FULL))
+                      /*prune=*/mode != PACMAP_KNN_TENSOR_F16_FULL, /*any_scale=*/forced || n >= TC_APPROX_ROWS))
       return;
   }
   PM_REQUIRE(mode == PACMAP_KNN_AUTO || mode == PACMAP_KNN_SIMT_EXACT || mode == PACMAP_KNN_APPROX,

@@ -167,6 +167,10 @@ __global__ void __launch_bounds__(PV_BATCH * 32) pivot_draw_kernel(const float* 
   if (lane == 0) piv_rows[round * PV_BATCH + b] = static_cast<uint32_t>(sub_row(s, S, n));
 }
 
+__global__ void even_pivots_kernel(uint64_t n, uint32_t* __restrict__ piv_rows) {
+  piv_rows[threadIdx.x] = static_cast<uint32_t>(threadIdx.x * n / PIV);
+}
+
 // Per column tile (128 positions): its rows split by pivot cell into at most SEGS segments (cells are
 // contiguous in the locality order; cells past the fourth merge into the fourth, whose pivot stays its
 // first cell's). Per segment g: seg_cell, the radius seg_rad = max |x_i - p_cell| (rounded up), the
@@ -483,7 +487,12 @@ uint64_t build_probe_tile_lists(Ctx& c, const float* d_x, uint64_t d, const uint
   return total;
 }
 
-void select_pivots(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint32_t* d_piv_rows) {
+void select_pivots(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint32_t* d_piv_rows, bool seeded) {
+  if (!seeded) {
+    even_pivots_kernel<<<1, PIV, 0, c.stream>>>(n, d_piv_rows);
+    PM_LAUNCHED();
+    return;
+  }
   const uint32_t S = static_cast<uint32_t>(std::min<uint64_t>(n, PV_SUB_MAX));
   const int nchunks = static_cast<int>(ceil_div(S, PV_CHUNK));
   DevBuf<float> dmin(c, S);

@@ -4,8 +4,8 @@
 
 namespace pacmap {
 
-// PIV pivot rows of d_x (n x d) by k-means++ seeding in batches on a fixed subsample; deterministic.
-void select_pivots(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint32_t* d_piv_rows);
+// PIV pivot rows of d_x (n x d), deterministic: by k-means++ seeding in batches on a fixed subsample, or evenly spaced.
+void select_pivots(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint32_t* d_piv_rows, bool seeded);
 
 // Inputs of the tile test, all on the device and in the locality order unless noted:
 //   perm        position r -> original row

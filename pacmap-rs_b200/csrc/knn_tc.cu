@@ -511,7 +511,10 @@ __global__ void split_rows_kernel(const float* __restrict__ x, const uint32_t* _
 // part goes to e_j, the product part is split by AM-GM like eta. gq[j] stores -g_j / 4 as three bf16
 // parts with an exact sum, twice (elements 0..2 and 8..10, zero elsewhere), so that the all-ones row
 // operand sums them to -g_j / 2 whatever the swizzle order of the two 16-byte halves.
-__global__ void bound_kernel(uint64_t n, uint64_t n_pad, int d, int KP, float rho, const float* __restrict__ nrm,
+// abs_err covers what the reference's f32 products lose below the smallest normal number (d + 8 terms of 2^-150,
+// in the scaled units): it matters where coordinates differ by less than about 1e-19.
+__global__ void bound_kernel(uint64_t n, uint64_t n_pad, int d, int KP, float rho, float abs_err,
+                             const float* __restrict__ nrm,
                              const float* __restrict__ A, const float* __restrict__ B, float2* __restrict__ ge,
                              uint16_t* __restrict__ gq, uint32_t* __restrict__ e4max_bits) {
   const uint64_t j = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -529,7 +532,7 @@ __global__ void bound_kernel(uint64_t n, uint64_t n_pad, int d, int KP, float rh
     // and the epilogue's roundings: (2d + 64) 2^-24 + 2^-19.
     const float gamma = static_cast<float>(2 * d + 64) * 5.9604644775390625e-08f + 1.9073486328125e-06f;
     const float e0 = 0.5f * (rho * a + b / rho) + 0.5f * b + 0.5f * eta * a + gamma * nn;
-    const float e = e0 + 0.5f * eta_s * a + 0.5f * eta_s * (nn + 4.0f * e0) + 1e-30f;
+    const float e = e0 + 0.5f * eta_s * a + 0.5f * eta_s * (nn + 4.0f * e0) + abs_err;
     const float e_safe = e * (1.0f + 9.765625e-04f);  // 2^-10 relative margin on the bound itself
     const float g = nrm[j] - 2.0f * e_safe;
     ge[j] = make_float2(g, 4.0f * e_safe);
@@ -1227,7 +1230,7 @@ __global__ void mark_owned_kernel(const uint32_t* __restrict__ perm, uint64_t r0
 }
 
 bool knn_tc_device(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint64_t kp, bool bf16, uint32_t* d_idx,
-                   float* d_dist, const KnnShard& shard, int nprobe, bool prune) {
+                   float* d_dist, const KnnShard& shard, int nprobe, bool prune, bool any_scale) {
   if (!knn_tc_supported(n, d, kp)) return false;
   KnnTcStats& st = last_tc_stats();
   st = KnnTcStats();
@@ -1255,12 +1258,16 @@ bool knn_tc_device(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint64_t kp
   if (!(amx > 0.0f) || !std::isfinite(amx)) return false;  // all-zero or non-finite data: SIMT path
   int ex = 0;
   std::frexp(amx, &ex);  // amx in [2^(ex-1), 2^ex)
+  // Outside these scales the reference's f32 distances may overflow or vanish into ties that the filter does not see.
+  if (!any_scale && (ex < -30 || ex > 50)) return false;
   const float s = std::ldexp(1.0f, 13 - ex);
 
-  // locality order: pivots by k-means++ seeding, every point to its nearest pivot, a stable sort by cell
+  // locality order: pivots, every point to its nearest pivot, a stable sort by cell. Pruned and approximate searches
+  // need a pivot in every well-separated group (k-means++ seeding, 16 dependent rounds, 0.6 to 1.3 ms); a full sweep only
+  // wants near rows near each other, for which evenly spaced points do.
   const uint32_t chunks = ceil_div(n, PL_CHUNK);
   DevBuf<uint32_t> piv_rows(c, PIV), cell(c, n), cell_counts(c, static_cast<uint64_t>(chunks) * PIV), perm(c, n);
-  select_pivots(c, d_x, n, d, piv_rows.get());
+  select_pivots(c, d_x, n, d, piv_rows.get(), /*seeded=*/n >= PRUNE_MIN_ROWS || nprobe > 0);
   DevBuf<float> score, pnorm;
   if (prune) {
     score.alloc(c, n * PIV);
@@ -1369,9 +1376,10 @@ bool knn_tc_device(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint64_t kp
     sb += hpart[2 * b + 1];
   }
   const float rho = (sa > 0.0 && sb > 0.0) ? static_cast<float>(std::sqrt(sb / sa)) : 1e-4f;
+  const float abs_err = 1e-30f + static_cast<float>(std::ldexp(static_cast<double>(d + 8), -150) * s * s);
   DevBuf<uint32_t> e4max(c, 1);
   PM_CUDA(cudaMemsetAsync(e4max.get(), 0, sizeof(uint32_t), c.stream));
-  bound_kernel<<<ceil_div(n_pad, 256), 256, 0, c.stream>>>(n, n_pad, static_cast<int>(d), KP, rho, nrm.get(), A.get(),
+  bound_kernel<<<ceil_div(n_pad, 256), 256, 0, c.stream>>>(n, n_pad, static_cast<int>(d), KP, rho, abs_err, nrm.get(), A.get(),
                                                           B.get(), ge.get(), gq.get(), e4max.get());
   PM_LAUNCHED();
 

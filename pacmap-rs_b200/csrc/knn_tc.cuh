@@ -9,8 +9,10 @@ bool knn_tc_supported(uint64_t n, uint64_t d, uint64_t kp);
 // nprobe in 1..255: approximate -- each row block searches only the nprobe pivot cells nearest its own.
 // prune (exact mode, large n): column tiles that provably hold no neighbour of a row block are skipped
 // (knn_prune.cu); the result is the same.
+// any_scale false: also declines data whose largest magnitude is not within 2^-30 .. 2^50.
 bool knn_tc_device(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint64_t kp, bool bf16, uint32_t* d_idx,
-                   float* d_dist, const KnnShard& shard = KnnShard(), int nprobe = 0, bool prune = true);
+                   float* d_dist, const KnnShard& shard = KnnShard(), int nprobe = 0, bool prune = true,
+                   bool any_scale = true);
 // Counters of the last tensor-core kNN on this thread.
 struct KnnTcStats {
   double filter_ms = 0.0;       // device time of the filter launch that produced the candidates
