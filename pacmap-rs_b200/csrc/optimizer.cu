@@ -14,9 +14,10 @@
 //    group in a fixed butterfly, and applies the Adam step (adam.rs:45-57) to that point at once:
 //    y is ping-ponged between two buffers because other points read y_j during the iteration.
 //    Phase 3 has w_mn = 0: the MN segments are skipped (0 * finite = 0 adds nothing).
-// K9 optimize_device: all iterations are captured into one CUDA graph (one kernel node per iteration,
-//    snapshot copies as memcpy nodes); the per-iteration (w_nn, w_mn, w_fp, lr_t) schedule lives in a
-//    device table computed with the reference's f32 formulas.
+// K9 optimize_device: up to about 18,900 rows all iterations run in one launch (grad_adam_resident_kernel); above,
+//    or with losses asked for, they are captured into one CUDA graph (one kernel node per iteration, snapshot
+//    copies as memcpy nodes). The per-iteration (w_nn, w_mn, w_fp, lr_t) schedule lives in a device table computed
+//    with the reference's f32 formulas.
 #include <chrono>
 #include <cmath>
 #include <cstring>
@@ -24,6 +25,7 @@
 #include <type_traits>
 
 #include "engine.cuh"
+#include "ptx.cuh"
 
 namespace pacmap {
 namespace {
@@ -612,6 +614,148 @@ __global__ void __launch_bounds__(256) grad_adam_long_kernel(const GradArgs p, i
                            0xFFFFFFFFu);
 }
 
+// ------------------------------------------------------------------------------------------------
+// All iterations in one launch, for problems whose rows fit the GPU at once
+// ------------------------------------------------------------------------------------------------
+// y of a partner, which another block may have written before the last grid_arrive_wait: an ordinary load (L1 serves
+// repeated partners; the barrier's acquire keeps it from serving an earlier iteration's), never a read-only one.
+template <int DIM>
+__device__ __forceinline__ void load_y_shared(const float* y, uint32_t j, float (&out)[DIM]) {
+  if constexpr (DIM == 2) {
+    asm volatile("ld.global.v2.f32 {%0, %1}, [%2];"
+                 : "=f"(out[0]), "=f"(out[1])
+                 : "l"(y + static_cast<uint64_t>(j) * 2)
+                 : "memory");
+  } else {
+#pragma unroll
+    for (int c = 0; c < DIM; ++c)
+      asm volatile("ld.global.f32 %0, [%1];" : "=f"(out[c]) : "l"(y + static_cast<uint64_t>(j) * DIM + c) : "memory");
+  }
+}
+
+// accumulate_segment with RES_U entries of a lane in flight (the iteration is bound by latency here, not by the
+// gathers' rate).
+constexpr int RES_U = 4;
+template <int DIM, bool REPULSIVE>
+__device__ __forceinline__ void accumulate_resident(const float* y, const uint32_t* __restrict__ col, uint32_t s, uint32_t e, int gl, const float (&yi)[DIM], float c1,
+                                                    float c2, float w, float (&acc)[DIM]) {
+  constexpr uint32_t G = GRAD_G;
+  for (uint32_t j = s + static_cast<uint32_t>(gl); j < e; j += RES_U * G) {
+    uint32_t nj[RES_U];
+    float ya[RES_U][DIM];
+#pragma unroll
+    for (int u = 0; u < RES_U; ++u) nj[u] = j + u * G < e ? __ldg(col + j + u * G) : 0u;
+#pragma unroll
+    for (int u = 0; u < RES_U; ++u)
+      if (j + u * G < e) load_y_shared<DIM>(y, nj[u], ya[u]);
+#pragma unroll
+    for (int u = 0; u < RES_U; ++u) {
+      if (j + u * G >= e) break;
+      float term[DIM], loss;
+      pair_term<DIM, REPULSIVE>(yi, ya[u], c1, c2, w, term, loss, false);
+#pragma unroll
+      for (int c = 0; c < DIM; ++c) acc[c] = __fadd_rn(acc[c], term[c]);
+    }
+  }
+}
+
+struct ResidentArgs {
+  float* y[2];  // iteration itr0 reads y[0]
+  float *m, *v;
+  const uint32_t *rp, *col;
+  uint32_t n;
+  const Sched* sched;
+  const int* snap_slot;  // per iteration from itr0 on: the snapshot to write, or -1; may be null
+  float* snap;
+  int itr0, itr1;
+  float a1, a2;
+  uint32_t *arrived, *err;
+};
+
+// Waits until every block of the (cooperative) grid has arrived `round` times. False when it gave up (2 s).
+__device__ __forceinline__ bool grid_arrive_wait(uint32_t* arrived, uint32_t round, uint32_t* err) {
+  __shared__ int ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(arrived) : "memory");
+    const uint32_t want = round * gridDim.x;
+    const uint64_t t0 = globaltimer();
+    uint32_t seen;
+    int good = 1;
+    for (uint32_t it = 1;; ++it) {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(arrived) : "memory");
+      if (seen >= want) break;
+      if ((it & 255u) == 0 && globaltimer() - t0 > WAIT_LIMIT_NS) {
+        good = 0;
+        break;
+      }
+    }
+    if (!good) atomicOr(err, DEV_ERR_TIMEOUT);
+    ok = good;
+  }
+  __syncthreads();
+  return ok != 0;
+}
+
+// One row per eight lanes for all iterations: its y, m and v stay in registers (every lane of the group computes the same
+// Adam step), its partner indices in L1, and the blocks meet once per iteration. The sums are those of
+// grad_adam_kernel. Bound by that meeting and the latency of the gathers from L2: 2,000 rows in 2-D 4.4 us an iteration
+// against 8.1 for a graph node each, 9,000 rows 5.2 against 9.0, 18,000 rows 8.4 against 12.1; nothing to capture either
+// (0.5 ms a fit).
+template <int DIM>
+__global__ void __launch_bounds__(256, DIM <= 2 ? 4 : (DIM == 3 ? 3 : 1)) grad_adam_resident_kernel(const ResidentArgs p) {
+  const int gl = threadIdx.x & (GRAD_G - 1);
+  const unsigned gmask = ((1u << GRAD_G) - 1u) << ((threadIdx.x & 31) & ~(GRAD_G - 1));
+  const uint32_t i = blockIdx.x * (256 / GRAD_G) + threadIdx.x / GRAD_G;
+  const bool row = i < p.n;
+  const uint64_t at = static_cast<uint64_t>(i) * DIM;
+  uint32_t s[4] = {};
+  float yi[DIM] = {}, m[DIM] = {}, v[DIM] = {};
+  if (row) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) s[q] = p.rp[3 * static_cast<uint64_t>(i) + q];
+#pragma unroll
+    for (int c = 0; c < DIM; ++c) {
+      yi[c] = p.y[0][at + c];
+      m[c] = p.m[at + c];
+      v[c] = p.v[at + c];
+    }
+  }
+  for (int itr = p.itr0; itr < p.itr1; ++itr) {
+    const int from = (itr - p.itr0) & 1;
+    const Sched sc = p.sched[itr];
+    if (row) {
+      const float* y = p.y[from];
+      float acc[DIM] = {};
+      accumulate_resident<DIM, false>(y, p.col, s[0], s[1], gl, yi, 10.0f, 20.0f, sc.w_nn, acc);
+      if (sc.w_mn != 0.0f)
+        accumulate_resident<DIM, false>(y, p.col, s[1], s[2], gl, yi, 10000.0f, 20000.0f, sc.w_mn, acc);
+      accumulate_resident<DIM, true>(y, p.col, s[2], s[3], gl, yi, 1.0f, 2.0f, sc.w_fp, acc);
+#pragma unroll
+      for (int o = GRAD_G / 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int c = 0; c < DIM; ++c) acc[c] = __fadd_rn(acc[c], __shfl_xor_sync(gmask, acc[c], o, GRAD_G));
+      const int slot = p.snap_slot ? p.snap_slot[itr - p.itr0] : -1;
+#pragma unroll
+      for (int c = 0; c < DIM; ++c) {
+        yi[c] = adam_coord(acc[c], yi[c], &m[c], &v[c], p.a1, p.a2, sc.lr_t);
+        if (gl == 0) {
+          p.y[from ^ 1][at + c] = yi[c];
+          if (slot >= 0) p.snap[static_cast<uint64_t>(slot) * p.n * DIM + at + c] = yi[c];
+        }
+      }
+    }
+    if (itr + 1 < p.itr1 && !grid_arrive_wait(p.arrived, static_cast<uint32_t>(itr + 1 - p.itr0), p.err)) return;
+  }
+  if (row && gl == 0) {
+#pragma unroll
+    for (int c = 0; c < DIM; ++c) {
+      p.m[at + c] = m[c];
+      p.v[at + c] = v[c];
+    }
+  }
+}
+
 // The rows with more than GRAD_LONG entries, in any order (each is summed by itself).
 __global__ void long_rows_kernel(const uint32_t* __restrict__ rp, uint64_t n, uint32_t* __restrict__ rows,
                                  uint32_t* __restrict__ count) {
@@ -635,20 +779,22 @@ __global__ void __launch_bounds__(1024) loss_reduce_kernel(const float* __restri
 }
 
 using GradFn = void (*)(const GradArgs, int);
+using ResidentFn = void (*)(const ResidentArgs);
 struct GradFns {
   GradFn rows, long_rows;
+  ResidentFn resident;
 };
 
 GradFns pick_grad_kernel(uint64_t dim) {
   switch (dim) {
-    case 1: return {grad_adam_kernel<1>, grad_adam_long_kernel<1>};
-    case 2: return {grad_adam_kernel<2>, grad_adam_long_kernel<2>};
-    case 3: return {grad_adam_kernel<3>, grad_adam_long_kernel<3>};
-    case 4: return {grad_adam_kernel<4>, grad_adam_long_kernel<4>};
-    case 5: return {grad_adam_kernel<5>, grad_adam_long_kernel<5>};
-    case 6: return {grad_adam_kernel<6>, grad_adam_long_kernel<6>};
-    case 7: return {grad_adam_kernel<7>, grad_adam_long_kernel<7>};
-    case 8: return {grad_adam_kernel<8>, grad_adam_long_kernel<8>};
+    case 1: return {grad_adam_kernel<1>, grad_adam_long_kernel<1>, grad_adam_resident_kernel<1>};
+    case 2: return {grad_adam_kernel<2>, grad_adam_long_kernel<2>, grad_adam_resident_kernel<2>};
+    case 3: return {grad_adam_kernel<3>, grad_adam_long_kernel<3>, grad_adam_resident_kernel<3>};
+    case 4: return {grad_adam_kernel<4>, grad_adam_long_kernel<4>, grad_adam_resident_kernel<4>};
+    case 5: return {grad_adam_kernel<5>, grad_adam_long_kernel<5>, grad_adam_resident_kernel<5>};
+    case 6: return {grad_adam_kernel<6>, grad_adam_long_kernel<6>, grad_adam_resident_kernel<6>};
+    case 7: return {grad_adam_kernel<7>, grad_adam_long_kernel<7>, grad_adam_resident_kernel<7>};
+    case 8: return {grad_adam_kernel<8>, grad_adam_long_kernel<8>, grad_adam_resident_kernel<8>};
     default: return {};
   }
 }
@@ -892,6 +1038,57 @@ struct Branch {
   Branch(const Branch&) = delete;
   Branch& operator=(const Branch&) = delete;
 };
+
+// optimize_device for rows that fit the GPU at once, eight lanes each; false when they do not, or when the call wants
+// what only the other path gives (losses, the last gradient, long rows beside the others).
+bool optimize_resident(Ctx& c, const Csr& csr, const OptimizeArgs& a, ResidentFn fn, const Sched* sched, float* yb,
+                       float a1, float a2) {
+  if (a.h_loss || a.d_grad_last || csr.n_long > 0 || a.n >= (1ull << 24)) return false;
+  int per_sm = 0;
+  PM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 256, 0));
+  const unsigned blocks = ceil_div(a.n, 256 / GRAD_G);
+  if (blocks > static_cast<unsigned>(c.sm_count * per_sm)) return false;
+  const uint64_t iters = a.itr_end - a.itr_begin;
+  DevBuf<uint32_t> arrived(c, 1);
+  PM_CUDA(cudaMemsetAsync(arrived.get(), 0, sizeof(uint32_t), c.stream));
+  DevBuf<int> slots;
+  std::vector<int> hslots;
+  if (a.d_snap && a.snapshots) {
+    hslots.assign(iters, -1);
+    for (uint64_t t = 0; t < iters; ++t)
+      for (uint64_t q = 0; q < a.n_snapshots; ++q)
+        if (a.snapshots[q] == a.itr_begin + t + 1) {
+          hslots[t] = static_cast<int>(q);
+          break;
+        }
+    upload(c, slots, hslots.data(), iters);
+  }
+  ResidentArgs ra{};
+  ra.y[0] = a.d_y;
+  ra.y[1] = yb;
+  ra.m = a.d_m;
+  ra.v = a.d_v;
+  ra.rp = csr.row_ptr.get();
+  ra.col = csr.col.get();
+  ra.n = static_cast<uint32_t>(a.n);
+  ra.sched = sched;
+  ra.snap_slot = slots.get();
+  ra.snap = a.d_snap;
+  ra.itr0 = static_cast<int>(a.itr_begin);
+  ra.itr1 = static_cast<int>(a.itr_end);
+  ra.a1 = a1;
+  ra.a2 = a2;
+  ra.arrived = arrived.get();
+  ra.err = c.d_err;
+  void* params[] = {&ra};
+  PM_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(fn), dim3(blocks), dim3(256), params, 0, c.stream));
+  count_launch();
+  if (iters & 1)
+    PM_CUDA(cudaMemcpyAsync(a.d_y, yb, a.n * a.dim * sizeof(float), cudaMemcpyDeviceToDevice, c.stream));
+  PM_CUDA(cudaStreamSynchronize(c.stream));
+  last_graph_setup_ms() = 0.0;
+  return true;
+}
 }  // namespace
 
 double& last_graph_setup_ms() {
@@ -919,6 +1116,7 @@ void optimize_device(Ctx& c, const Csr& csr, const OptimizeArgs& a) {
     row_loss.alloc(c, n);
     loss_dev.alloc(c, iters);
   }
+  if (optimize_resident(c, csr, a, fns.resident, sched.get(), yb.get(), a1, a2)) return;
   int per_sm = 0;
   PM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fns.rows, 256, 0));
   const unsigned grid = static_cast<unsigned>(std::max<uint64_t>(
