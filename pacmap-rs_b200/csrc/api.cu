@@ -432,9 +432,9 @@ pacmap_status pacmap_fit_transform(const float* x, uint64_t n, uint64_t d, const
     const bool snaps = out_snapshots && cfg->snapshots && cfg->n_snapshots > 0;
     if (snaps) ds.alloc(c, cfg->n_snapshots * n * dim);
     fit_transform_impl(c, dx.get(), n, d, *cfg, dy.get(), snaps ? ds.get() : nullptr);
-    if (dim) PM_CUDA(cudaMemcpyAsync(out_embedding, dy.get(), n * dim * sizeof(float), cudaMemcpyDeviceToHost, c.stream));
+    if (dim) copy_to_host(c, out_embedding, dy.get(), n * dim * sizeof(float));
     if (snaps)
-      PM_CUDA(cudaMemcpyAsync(out_snapshots, ds.get(), ds.bytes(), cudaMemcpyDeviceToHost, c.stream));
+      copy_to_host(c, out_snapshots, ds.get(), ds.bytes());
     PM_CUDA(cudaStreamSynchronize(c.stream));
   });
 }
@@ -470,8 +470,8 @@ pacmap_status pacmap_fit_transform_learned(const float* x, uint64_t n, uint64_t 
                "target_mean and target_std go together");
     fit_transform_impl(c, dx.get(), n, d, *cfg, dy.get(), snaps ? ds.get() : nullptr, mlp_params, target_mean,
                        target_std);
-    PM_CUDA(cudaMemcpyAsync(out_embedding, dy.get(), n * dim * sizeof(float), cudaMemcpyDeviceToHost, c.stream));
-    if (snaps) PM_CUDA(cudaMemcpyAsync(out_snapshots, ds.get(), ds.bytes(), cudaMemcpyDeviceToHost, c.stream));
+    copy_to_host(c, out_embedding, dy.get(), n * dim * sizeof(float));
+    if (snaps) copy_to_host(c, out_snapshots, ds.get(), ds.bytes());
     PM_CUDA(cudaStreamSynchronize(c.stream));
   });
 }
@@ -537,7 +537,7 @@ pacmap_status pacmap_mlp_apply(const float* params, uint64_t d, uint64_t dim, co
     DevBuf<float> dx, dy(c, n * dim);
     upload(c, dx, xp, n * d);
     mlp_apply_device(c, params, d, dim, dx.get(), n, dy.get());
-    PM_CUDA(cudaMemcpyAsync(out, dy.get(), dy.bytes(), cudaMemcpyDeviceToHost, c.stream));
+    copy_to_host(c, out, dy.get(), dy.bytes());
     PM_CUDA(cudaStreamSynchronize(c.stream));
   });
 }
@@ -596,7 +596,7 @@ pacmap_status pacmap_transform(const float* x, uint64_t n, uint64_t d, uint64_t 
     DevBuf<float> dx, dy(c, n * dim);
     upload(c, dx, x, n * d);
     transform_device(c, dx.get(), n, d, dim, params, pre_min, pre_max, pre_mean, target_mean, target_std, dy.get());
-    PM_CUDA(cudaMemcpyAsync(out_embedding, dy.get(), dy.bytes(), cudaMemcpyDeviceToHost, c.stream));
+    copy_to_host(c, out_embedding, dy.get(), dy.bytes());
     PM_CUDA(cudaStreamSynchronize(c.stream));
   });
 }
@@ -628,8 +628,8 @@ pacmap_status pacmap_knn_exact(const float* x, uint64_t n, uint64_t d, uint64_t 
     DevBuf<uint32_t> di(c, n * kp);
     upload(c, dx, x, n * d);
     knn_exact_device(c, dx.get(), n, d, kp, knn_mode, di.get(), dd.get());
-    PM_CUDA(cudaMemcpyAsync(out_idx, di.get(), di.bytes(), cudaMemcpyDeviceToHost, c.stream));
-    PM_CUDA(cudaMemcpyAsync(out_dist, dd.get(), dd.bytes(), cudaMemcpyDeviceToHost, c.stream));
+    copy_to_host(c, out_idx, di.get(), di.bytes());
+    copy_to_host(c, out_dist, dd.get(), dd.bytes());
     PM_CUDA(cudaStreamSynchronize(c.stream));
     c.check_errors("knn");
   });
@@ -659,10 +659,10 @@ pacmap_status pacmap_knn_exact_shard(const float* x, uint64_t n, uint64_t d, uin
       sh.count = n_shards;
       sh.d_owned = own.get();
       knn_exact_device(c, dx.get(), n, d, kp, knn_mode, di.get(), dd.get(), sh);
-      PM_CUDA(cudaMemcpyAsync(out_idx, di.get(), di.bytes(), cudaMemcpyDeviceToHost, c.stream));
-      PM_CUDA(cudaMemcpyAsync(out_dist, dd.get(), dd.bytes(), cudaMemcpyDeviceToHost, c.stream));
+      copy_to_host(c, out_idx, di.get(), di.bytes());
+      copy_to_host(c, out_dist, dd.get(), dd.bytes());
     }
-    PM_CUDA(cudaMemcpyAsync(out_owned, own.get(), n, cudaMemcpyDeviceToHost, c.stream));
+    copy_to_host(c, out_owned, own.get(), n);
     PM_CUDA(cudaStreamSynchronize(c.stream));
     c.check_errors("knn shard");
   });
@@ -704,8 +704,8 @@ pacmap_status pacmap_preprocess(const float* x, uint64_t n, uint64_t d, int32_t 
     DevBuf<float> dx, dout(c, n * d), dmean(c, d);
     upload(c, dx, x, n * d);
     preprocess_device(c, dx.get(), n, d, dout.get(), out_min, out_max, dmean.get());
-    PM_CUDA(cudaMemcpyAsync(out, dout.get(), dout.bytes(), cudaMemcpyDeviceToHost, c.stream));
-    if (out_mean) PM_CUDA(cudaMemcpyAsync(out_mean, dmean.get(), dmean.bytes(), cudaMemcpyDeviceToHost, c.stream));
+    copy_to_host(c, out, dout.get(), dout.bytes());
+    if (out_mean) copy_to_host(c, out_mean, dmean.get(), dmean.bytes());
     PM_CUDA(cudaStreamSynchronize(c.stream));
   });
 }
@@ -731,9 +731,9 @@ pacmap_status pacmap_generate_pairs(const float* x, uint64_t n, uint64_t d, cons
     DevPairs pairs;
     generate_pairs_device(c, xp.get(), n, dw, pc, cfg->has_seed ? cfg->seed : entropy_seed(), cfg->knn_mode, pairs,
                           nullptr, cfg->approx_threshold);
-    if (out_pnn) PM_CUDA(cudaMemcpyAsync(out_pnn, pairs.nn.get(), pairs.nn.bytes(), cudaMemcpyDeviceToHost, c.stream));
-    if (out_pmn) PM_CUDA(cudaMemcpyAsync(out_pmn, pairs.mn.get(), pairs.mn.bytes(), cudaMemcpyDeviceToHost, c.stream));
-    if (out_pfp) PM_CUDA(cudaMemcpyAsync(out_pfp, pairs.fp.get(), pairs.fp.bytes(), cudaMemcpyDeviceToHost, c.stream));
+    if (out_pnn) copy_to_host(c, out_pnn, pairs.nn.get(), pairs.nn.bytes());
+    if (out_pmn) copy_to_host(c, out_pmn, pairs.mn.get(), pairs.mn.bytes());
+    if (out_pfp) copy_to_host(c, out_pfp, pairs.fp.get(), pairs.fp.bytes());
     PM_CUDA(cudaStreamSynchronize(c.stream));
   });
 }
@@ -751,8 +751,8 @@ pacmap_status pacmap_reselect_neighbors(const uint32_t* knn_idx, const float* kn
     upload(c, dd, knn_dist, n * kp);
     sigma_device(c, dd.get(), n, kp, ds.get());
     reselect_device(c, di.get(), dd.get(), ds.get(), n, kp, k, dp.get());
-    PM_CUDA(cudaMemcpyAsync(out_pnn, dp.get(), dp.bytes(), cudaMemcpyDeviceToHost, c.stream));
-    if (out_sigma) PM_CUDA(cudaMemcpyAsync(out_sigma, ds.get(), ds.bytes(), cudaMemcpyDeviceToHost, c.stream));
+    copy_to_host(c, out_pnn, dp.get(), dp.bytes());
+    if (out_sigma) copy_to_host(c, out_sigma, ds.get(), ds.bytes());
     PM_CUDA(cudaStreamSynchronize(c.stream));
   });
 }
@@ -769,7 +769,7 @@ pacmap_status pacmap_sample_pairs(const float* xp, uint64_t n, uint64_t d, const
       DevBuf<uint32_t> dm(c, n * n_mn * 2);
       upload(c, dx, xp, n * d);
       sample_mn_device(c, dx.get(), n, d, n_mn, seed, dm.get());
-      PM_CUDA(cudaMemcpyAsync(out_pmn, dm.get(), dm.bytes(), cudaMemcpyDeviceToHost, c.stream));
+      copy_to_host(c, out_pmn, dm.get(), dm.bytes());
       PM_CUDA(cudaStreamSynchronize(c.stream));
     }
     if (out_pfp && n_fp) {
@@ -777,7 +777,7 @@ pacmap_status pacmap_sample_pairs(const float* xp, uint64_t n, uint64_t d, const
       DevBuf<uint32_t> dn, df(c, n * n_fp * 2);
       upload(c, dn, pair_neighbors, n * k * 2);
       sample_fp_device(c, dn.get(), n, k, n_fp, seed, df.get());
-      PM_CUDA(cudaMemcpyAsync(out_pfp, df.get(), df.bytes(), cudaMemcpyDeviceToHost, c.stream));
+      copy_to_host(c, out_pfp, df.get(), df.bytes());
       PM_CUDA(cudaStreamSynchronize(c.stream));
     }
     c.check_errors("pair sampling");
@@ -824,11 +824,11 @@ pacmap_status pacmap_optimize_steps(float* y, float* m, float* v, uint64_t n, ui
     }
     optimize_device(c, csr, oa);
     c.check_errors("optimiser");
-    PM_CUDA(cudaMemcpyAsync(y, dy.get(), dy.bytes(), cudaMemcpyDeviceToHost, c.stream));
-    PM_CUDA(cudaMemcpyAsync(m, dm.get(), dm.bytes(), cudaMemcpyDeviceToHost, c.stream));
-    PM_CUDA(cudaMemcpyAsync(v, dv.get(), dv.bytes(), cudaMemcpyDeviceToHost, c.stream));
+    copy_to_host(c, y, dy.get(), dy.bytes());
+    copy_to_host(c, m, dm.get(), dm.bytes());
+    copy_to_host(c, v, dv.get(), dv.bytes());
     if (oa.d_grad_last)
-      PM_CUDA(cudaMemcpyAsync(out_grad, dg.get(), dg.bytes(), cudaMemcpyDeviceToHost, c.stream));
+      copy_to_host(c, out_grad, dg.get(), dg.bytes());
     PM_CUDA(cudaStreamSynchronize(c.stream));
     if (oa.d_grad_last) {
       out_grad[n * dim] = loss.back();
@@ -855,7 +855,7 @@ pacmap_status pacmap_gradient(const float* y, uint64_t n, uint64_t dim, const ui
     build_csr(c, n, a.get(), n_nn, b.get(), n_mn, e.get(), n_fp, csr);
     float loss = 0.0f;
     gradient_device(c, csr, dy.get(), n, dim, w_nn, w_mn, w_fp, dg.get(), &loss);
-    PM_CUDA(cudaMemcpyAsync(out_grad, dg.get(), dg.bytes(), cudaMemcpyDeviceToHost, c.stream));
+    copy_to_host(c, out_grad, dg.get(), dg.bytes());
     PM_CUDA(cudaStreamSynchronize(c.stream));
     out_grad[n * dim] = loss;
     for (uint64_t cc = 1; cc < dim; ++cc) out_grad[n * dim + cc] = 0.0f;
@@ -870,7 +870,7 @@ pacmap_status pacmap_init_value(const float* v, uint64_t n, uint64_t dim, int32_
     DevBuf<float> dv, dy(c, n * dim);
     upload(c, dv, v, n * dim);
     init_value_device(c, dv.get(), n, dim, dy.get());
-    PM_CUDA(cudaMemcpyAsync(out, dy.get(), dy.bytes(), cudaMemcpyDeviceToHost, c.stream));
+    copy_to_host(c, out, dy.get(), dy.bytes());
     PM_CUDA(cudaStreamSynchronize(c.stream));
   });
 }
@@ -882,7 +882,7 @@ pacmap_status pacmap_init_random(uint64_t n, uint64_t dim, uint64_t seed, int32_
     Ctx& c = dl.ctx;
     DevBuf<float> dy(c, n * dim);
     init_random_device(c, n, dim, seed, dy.get());
-    PM_CUDA(cudaMemcpyAsync(out, dy.get(), dy.bytes(), cudaMemcpyDeviceToHost, c.stream));
+    copy_to_host(c, out, dy.get(), dy.bytes());
     PM_CUDA(cudaStreamSynchronize(c.stream));
   });
 }

@@ -1,6 +1,7 @@
 // Host-side engine plumbing: per-call context, stream-ordered device buffers, stage launchers.
 #pragma once
 
+#include <memory>
 #include <vector>
 
 #include "common.cuh"
@@ -55,11 +56,17 @@ struct DevBuf {
   size_t bytes() const { return count * sizeof(T); }
 };
 
+// ---- hostcopy.cu ----
+// Copies on the call's stream between the device and a caller's host memory, which the call may let go of (to_device) or
+// read (to_host, after a synchronisation of the stream) once the function has returned, as with cudaMemcpyAsync.
+void copy_to_device(Ctx& c, void* d_dst, const void* src, size_t bytes);
+void copy_to_host(Ctx& c, void* dst, const void* d_src, size_t bytes);
+
 // dst = a device copy of count host values (stream-ordered).
 template <typename T>
 void upload(Ctx& c, DevBuf<T>& dst, const T* src, size_t count) {
   dst.alloc(c, count);
-  if (count) PM_CUDA(cudaMemcpyAsync(dst.get(), src, count * sizeof(T), cudaMemcpyHostToDevice, c.stream));
+  copy_to_device(c, dst.get(), src, count * sizeof(T));
 }
 
 // ---- preprocess.cu ----
