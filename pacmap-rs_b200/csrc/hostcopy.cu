@@ -1,11 +1,11 @@
 // Copies between a caller's ordinary (pageable) host memory and the device.
 //
-// The driver moves pageable memory through its own staging buffers on the calling thread, about 10 GB/s each way, and an
-// output's pages are first touched there, one by one; the PCIe link takes 55 GB/s from page-locked memory. Copies of
-// at least COPY_MIN bytes are therefore cut into one range per worker: each worker moves its range piece by piece
-// through two page-locked slots of its own, copying one piece on a core while the other is on the link. The threads live
-// for one copy; the slots (32 MB) stay with the device until the library is unloaded. Calls on a device hold its lock,
-// so one copy uses them at a time. Memory that the caller page-locked goes to the link directly, as before.
+// The driver moves pageable memory through its own staging buffers on the calling thread, and an output's pages are first
+// touched there, one by one: 64 MB take it 4.7 ms up and 13.6 down, where the link needs 1.2. Larger copies are cut into
+// one range per worker: each worker moves its range piece by piece through two page-locked slots of its own, copying
+// one piece on a core while the other is on the link (64 MB: 3.0 and 3.1 ms). The threads live for one copy; the slots
+// (32 MB) stay with the device until the library is unloaded. Calls on a device hold its lock, so one copy uses them at a
+// time. Memory that the caller page-locked goes to the link directly.
 #include <algorithm>
 #include <cstring>
 #include <system_error>
@@ -17,7 +17,10 @@ namespace pacmap {
 namespace {
 
 constexpr int COPY_WORKERS = 8;
-constexpr size_t COPY_PIECE = 2u << 20, COPY_MIN = 4u << 20;
+constexpr size_t COPY_SLOT = 2u << 20;
+// Downloads are staged from 1 MB (0.11 against 0.23 ms; 4 MB 0.45 against 0.63), uploads from 32 MB (1.6 against 1.9; at
+// 16 MB the two are equal). A worker is worth starting for 8 MB: smaller shares made 4 MB downloads 0.7 to 1.2 ms.
+constexpr size_t DOWN_MIN = 1u << 20, UP_MIN = 32u << 20, COPY_SHARE = 8u << 20;
 
 }  // namespace
 
@@ -25,7 +28,7 @@ struct HostStaging {
   char* buf = nullptr;
   cudaEvent_t ev[COPY_WORKERS][2] = {};
   HostStaging() {
-    PM_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&buf), 2 * COPY_WORKERS * COPY_PIECE, cudaHostAllocDefault));
+    PM_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&buf), 2 * COPY_WORKERS * COPY_SLOT, cudaHostAllocDefault));
     for (auto& w : ev)
       for (auto& e : w)
         if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
@@ -53,10 +56,11 @@ std::unique_ptr<HostStaging> g_staging[64];  // by device, used under the device
 cudaError_t move_range(HostStaging& st, int w, int device, cudaStream_t stream, char* dst, const char* src, size_t lo,
                        size_t hi, bool to_device) {
   cudaError_t e = cudaSetDevice(device);
-  char* slots[2] = {st.buf + (2 * w) * COPY_PIECE, st.buf + (2 * w + 1) * COPY_PIECE};
-  const size_t pieces = (hi - lo + COPY_PIECE - 1) / COPY_PIECE;
-  auto at = [&](size_t p) { return lo + p * COPY_PIECE; };
-  auto len = [&](size_t p) { return std::min(COPY_PIECE, hi - at(p)); };
+  char* slots[2] = {st.buf + (2 * w) * COPY_SLOT, st.buf + (2 * w + 1) * COPY_SLOT};
+  const size_t piece = std::min(COPY_SLOT, std::max<size_t>((hi - lo) / 4, 128u << 10));
+  const size_t pieces = (hi - lo + piece - 1) / piece;
+  auto at = [&](size_t p) { return lo + p * piece; };
+  auto len = [&](size_t p) { return std::min(piece, hi - at(p)); };
   for (size_t p = 0; p < pieces + (to_device ? 0 : 1) && e == cudaSuccess; ++p) {
     const int s = static_cast<int>(p & 1);
     if (to_device) {
@@ -84,7 +88,7 @@ void copy_host(Ctx& c, void* dst, const void* src, size_t bytes, bool to_device)
   if (!bytes) return;
   const cudaMemcpyKind kind = to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
   cudaPointerAttributes at{};
-  const bool pageable = bytes >= COPY_MIN && cudaPointerGetAttributes(&at, to_device ? src : dst) == cudaSuccess &&
+  const bool pageable = bytes >= (to_device ? UP_MIN : DOWN_MIN) && cudaPointerGetAttributes(&at, to_device ? src : dst) == cudaSuccess &&
                         at.type == cudaMemoryTypeUnregistered;
   if (!pageable) {
     PM_CUDA(cudaMemcpyAsync(dst, src, bytes, kind, c.stream));
@@ -94,7 +98,7 @@ void copy_host(Ctx& c, void* dst, const void* src, size_t bytes, bool to_device)
   HostStaging& st = *g_staging[c.device];
   const int cores = static_cast<int>(std::max(1u, std::thread::hardware_concurrency()));
   const int workers = static_cast<int>(
-      std::min<size_t>(std::min(COPY_WORKERS, std::max(1, cores / 2)), std::max<size_t>(1, bytes / COPY_PIECE)));
+      std::min<size_t>(std::min(COPY_WORKERS, std::max(1, cores / 2)), std::max<size_t>(1, bytes / COPY_SHARE)));
   const size_t share = (bytes / workers + 4095) & ~static_cast<size_t>(4095);
   cudaError_t err[COPY_WORKERS] = {};
   std::thread th[COPY_WORKERS];

@@ -14,10 +14,10 @@ def _rows(n, d, seed):
     return np.random.default_rng(seed).uniform(-2, 3, size=(n, d)).astype(np.float32)
 
 
-# bytes: just below 4 MiB, exactly, one row above; one piece more than two; ranges that are no multiple of a piece or of
-# 4 KiB; more than all slots hold
-@pytest.mark.parametrize("n,d", [(1048575, 1), (1048576, 1), (1048577, 1), (174763, 9), (100003, 33), (30011, 301),
-                                 (170001, 67)])
+# bytes: around the rules of 1 MiB (down) and 32 MiB (up), one to eight workers, ranges that are no multiple of a piece or
+# of 4 KiB, more than all slots hold
+@pytest.mark.parametrize("n,d", [(262143, 1), (262144, 1), (262145, 1), (1048577, 1), (174763, 9), (100003, 33),
+                                 (8388607, 1), (262144, 32), (262145, 32), (30011, 301), (170001, 97)])
 def test_copies_are_complete(lib, orc, n, d):
     x = _rows(n, d, n)
     got, mn, mx, mean = lib.stages.preprocess(x)
@@ -26,15 +26,16 @@ def test_copies_are_complete(lib, orc, n, d):
 
 
 def test_copies_from_unaligned_memory(lib, orc):
-    raw = np.zeros(60001 * 31 * 4 + 64, np.uint8)
-    x = raw[12:12 + 60001 * 31 * 4].view(np.float32).reshape(60001, 31)
-    x[:] = _rows(60001, 31, 4)
+    n = 300001
+    raw = np.zeros(n * 31 * 4 + 64, np.uint8)
+    x = raw[12:12 + n * 31 * 4].view(np.float32).reshape(n, 31)
+    x[:] = _rows(n, 31, 4)
     got = lib.stages.preprocess(x)[0]
     assert np.array_equal(got, orc.preprocess(x)[0])
 
 
 def test_copies_from_several_threads(lib, orc):
-    xs = [_rows(40001 + 7 * t, 50, t) for t in range(4)]
+    xs = [_rows(170001 + 7 * t, 50, t) for t in range(4)]
     want = [orc.preprocess(x)[0] for x in xs]
     bad = []
 
@@ -52,10 +53,10 @@ def test_copies_from_several_threads(lib, orc):
 def test_page_locked_memory(lib, orc):
     import torch
 
-    x = _rows(60000, 40, 8)
+    x = _rows(240000, 40, 8)
     px = torch.empty(x.shape, dtype=torch.float32, pin_memory=True)
     px.copy_(torch.from_numpy(x))
     out = torch.empty_like(px, pin_memory=True)
     mn, mx = C.c_float(0), C.c_float(0)
-    lib._check(lib._abi.lib().pacmap_preprocess(px.data_ptr(), 60000, 40, 0, out.data_ptr(), C.byref(mn), C.byref(mx), None))
+    lib._check(lib._abi.lib().pacmap_preprocess(px.data_ptr(), 240000, 40, 0, out.data_ptr(), C.byref(mn), C.byref(mx), None))
     assert np.array_equal(out.numpy(), orc.preprocess(x)[0])
