@@ -333,6 +333,10 @@ uint64_t pacmap_take_launch_count(void);
  * of hanging; on = 0 restores normal operation. The caller's current device is kept. */
 pacmap_status pacmap_debug_stall_knn_loads(int32_t device, int32_t on);
 
+/* Test hook (no reference analogue): out[i] = num / x[i] on the device with the division that the optimiser's tiled
+ * gradient uses for its pair factors. x, out: n values of host memory. */
+pacmap_status pacmap_debug_divide(float num, const float* x, uint64_t n, int32_t device, float* out);
+
 /* The message of the last failure on this thread ("" after success). */
 const char* pacmap_last_error(void);
 

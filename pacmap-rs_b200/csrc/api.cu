@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "engine.cuh"
+#include "grad.cuh"
 #include "knn_tc.cuh"
 #include "mlp.cuh"
 
@@ -819,8 +820,9 @@ pacmap_status pacmap_optimize_steps(float* y, float* m, float* v, uint64_t n, ui
     if (out_grad && itr_end > itr_begin) {
       dg.alloc(c, n * dim);
       oa.d_grad_last = dg.get();
-      loss.resize(itr_end - itr_begin);
+      loss.resize(1);
       oa.h_loss = loss.data();
+      oa.last_loss_only = true;
     }
     optimize_device(c, csr, oa);
     c.check_errors("optimiser");
@@ -882,6 +884,19 @@ pacmap_status pacmap_init_random(uint64_t n, uint64_t dim, uint64_t seed, int32_
     Ctx& c = dl.ctx;
     DevBuf<float> dy(c, n * dim);
     init_random_device(c, n, dim, seed, dy.get());
+    copy_to_host(c, out, dy.get(), dy.bytes());
+    PM_CUDA(cudaStreamSynchronize(c.stream));
+  });
+}
+
+pacmap_status pacmap_debug_divide(float num, const float* x, uint64_t n, int32_t device, float* out) {
+  return guarded([&] {
+    PM_REQUIRE(x && out, PACMAP_ERR_INVALID_ARGUMENT, "NULL buffer");
+    DeviceLock dl(device);
+    Ctx& c = dl.ctx;
+    DevBuf<float> dx, dy(c, n);
+    upload(c, dx, x, n);
+    if (n) debug_divide(c, num, dx.get(), n, dy.get());
     copy_to_host(c, out, dy.get(), dy.bytes());
     PM_CUDA(cudaStreamSynchronize(c.stream));
   });

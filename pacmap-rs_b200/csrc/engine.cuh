@@ -155,6 +155,7 @@ struct OptimizeArgs {
   uint64_t n_snapshots = 0;
   float* d_snap = nullptr;              // n_snapshots x n x dim (slot 0 pre-filled by the caller)
   float* h_loss = nullptr;              // per-iteration loss (host, itr_end - itr_begin values), may be NULL
+  bool last_loss_only = false;          // h_loss receives one value, the last iteration's (no snapshots then)
   float* d_grad_last = nullptr;         // (n+1) x dim gradient of the last iteration, may be NULL
 };
 void optimize_device(Ctx& c, const Csr& csr, const OptimizeArgs& a);

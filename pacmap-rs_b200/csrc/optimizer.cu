@@ -25,6 +25,7 @@
 #include <type_traits>
 
 #include "engine.cuh"
+#include "grad.cuh"
 #include "ptx.cuh"
 
 namespace pacmap {
@@ -392,92 +393,6 @@ __global__ void random_init_kernel(uint64_t total, uint64_t seed, float* __restr
 // ------------------------------------------------------------------------------------------------
 // K8: fused gradient + Adam
 // ------------------------------------------------------------------------------------------------
-struct Sched {
-  float w_nn, w_mn, w_fp, lr_t;
-};
-
-constexpr int GRAD_G = 8;  // lanes per row
-
-// What one iteration reads and writes: y_cur -> y_next, m and v in place (grad_only: none of them written).
-struct GradArgs {
-  const float* y_cur;
-  float *y_next, *m, *v;
-  const uint32_t *rp, *col;
-  uint64_t n;
-  const uint32_t* long_rows;
-  uint32_t n_long;
-  const Sched* sched;
-  float a1, a2;
-  float *row_loss, *grad_out;  // may be null
-  int grad_only;
-};
-
-// y of partner j (DIM consecutive floats; one 8-byte load for 2-D).
-template <int DIM>
-__device__ __forceinline__ void load_y(const float* __restrict__ y, uint32_t j, float (&out)[DIM]) {
-  if constexpr (DIM == 2) {
-    const float2 v = *reinterpret_cast<const float2*>(y + static_cast<uint64_t>(j) * 2);
-    out[0] = v.x;
-    out[1] = v.y;
-  } else {
-#pragma unroll
-    for (int c = 0; c < DIM; ++c) out[c] = y[static_cast<uint64_t>(j) * DIM + c];
-  }
-}
-
-// The force of partner yj on yi (per-pair arithmetic of gradient.rs:120-147) and the pair's loss.
-template <int DIM, bool REPULSIVE>
-__device__ __forceinline__ void pair_term(const float (&yi)[DIM], const float (&yj)[DIM], float c1, float c2, float w,
-                                          float (&term)[DIM], float& loss, bool want_loss) {
-  float df[DIM];
-  float dsq = 1.0f;
-#pragma unroll
-  for (int c = 0; c < DIM; ++c) {
-    df[c] = __fsub_rn(yi[c], yj[c]);
-    dsq = __fadd_rn(dsq, __fmul_rn(df[c], df[c]));
-  }
-  const float tt = __fadd_rn(c1, dsq);
-  const float w1 = __fmul_rn(w, __fdiv_rn(c2, __fmul_rn(tt, tt)));
-#pragma unroll
-  for (int c = 0; c < DIM; ++c) {
-    const float gterm = __fmul_rn(w1, df[c]);
-    term[c] = REPULSIVE ? -gterm : gterm;
-  }
-  if (want_loss)
-    loss = REPULSIVE ? __fmul_rn(w, __fdiv_rn(1.0f, __fadd_rn(1.0f, dsq))) : __fmul_rn(w, __fdiv_rn(dsq, tt));
-}
-
-// One segment (one pair type) of a row: lane gl of a G-lane group takes entries s + gl, s + gl + G, ...
-// in that order, with the partner index and y of the next entry loaded ahead (two-deep pipeline; four entries in
-// flight need 74 registers instead of 48 and made the 1M x 128 iterations 2 % slower).
-// The type's constants (c1, c2, weight, sign) are fixed for the whole segment.
-template <int DIM, bool REPULSIVE>
-__device__ __forceinline__ void accumulate_segment(const float* __restrict__ y, const uint32_t* __restrict__ col,
-                                                   uint32_t s, uint32_t e, int gl, int G, const float (&yi)[DIM],
-                                                   float c1, float c2, float w, float (&acc)[DIM], float& lacc,
-                                                   bool want_loss) {
-  uint32_t j = s + static_cast<uint32_t>(gl);
-  if (j >= e) return;
-  const uint32_t g = static_cast<uint32_t>(G);
-  uint32_t ja = col[j];
-  uint32_t jb = j + g < e ? col[j + g] : 0u;
-  float ya[DIM];
-  load_y<DIM>(y, ja, ya);
-  for (; j < e; j += g) {
-    float yb[DIM];
-    if (j + g < e) load_y<DIM>(y, jb, yb);
-    const uint32_t jc = j + 2 * g < e ? col[j + 2 * g] : 0u;
-    float term[DIM], loss = 0.0f;
-    pair_term<DIM, REPULSIVE>(yi, ya, c1, c2, w, term, loss, want_loss);
-#pragma unroll
-    for (int c = 0; c < DIM; ++c) acc[c] = __fadd_rn(acc[c], term[c]);
-    if (want_loss) lacc += loss;
-#pragma unroll
-    for (int c = 0; c < DIM; ++c) ya[c] = yb[c];
-    jb = jc;
-  }
-}
-
 // The same segment by a whole warp, for rows of more than GRAD_LONG entries: each lane forms the terms of its own
 // entries (LONG_U x 32 in flight), and lane l then adds, from the four lanes l % 8 + 8 r in turn, the entries
 // that lane l % 8 of an eight-lane group would have added, in the same order: the sums are the same bits. (Entry t of
@@ -541,18 +456,6 @@ __device__ __forceinline__ void accumulate_row(const float* __restrict__ y, cons
       accumulate_segment<DIM, false>(y, col, s1, s2, gl, G, yi, 10000.0f, 20000.0f, sc.w_mn, acc, lacc, want_loss);
     accumulate_segment<DIM, true>(y, col, s2, s3, gl, G, yi, 1.0f, 2.0f, sc.w_fp, acc, lacc, want_loss);
   }
-}
-
-// Adam (adam.rs:45-57) of one coordinate: updates m and v, returns the new y.
-__device__ __forceinline__ float adam_coord(float g, float yi, float* __restrict__ m, float* __restrict__ v, float a1,
-                                            float a2, float lr_t) {
-  float mm = *m, vv = *v;
-  mm = __fadd_rn(mm, __fmul_rn(a1, __fsub_rn(g, mm)));
-  vv = __fadd_rn(vv, __fmul_rn(a2, __fsub_rn(__fmul_rn(g, g), vv)));
-  const float step = __fdiv_rn(__fmul_rn(lr_t, mm), __fadd_rn(__fsqrt_rn(vv), 1e-7f));
-  *m = mm;
-  *v = vv;
-  return __fsub_rn(yi, step);
 }
 
 // One row's iteration by the lanes gl of an eight-lane group (gmask: its lanes), or by a whole warp.
@@ -840,6 +743,17 @@ Sched schedule_at(uint64_t itr, uint64_t p1, uint64_t p2, float lr) {
 
 }  // namespace
 
+void exclusive_scan_u32(Ctx& c, const uint32_t* d_in, uint64_t len, uint32_t* d_out) {
+  const uint64_t tiles = ceil_div(len, SCAN_TILE);
+  DevBuf<uint32_t> sums(c, tiles);
+  scan_tiles_kernel<<<static_cast<unsigned>(tiles), SCAN_T, 0, c.stream>>>(d_in, len, d_out, sums.get());
+  PM_LAUNCHED();
+  scan_sums_kernel<<<1, SCAN_T, 0, c.stream>>>(sums.get(), tiles);
+  PM_LAUNCHED();
+  scan_add_kernel<<<ceil_div(len, 256), 256, 0, c.stream>>>(d_out, len, sums.get());
+  PM_LAUNCHED();
+}
+
 void build_csr(Ctx& c, uint64_t n, const uint32_t* d_pnn, uint64_t n_nn, const uint32_t* d_pmn, uint64_t n_mn,
                const uint32_t* d_pfp, uint64_t n_fp, Csr& out, bool grouped_known) {
   PM_REQUIRE(n < (1ull << 32), PACMAP_ERR_UNSUPPORTED, "pair indices are u32: n must be < 2^32");
@@ -894,15 +808,7 @@ void build_csr(Ctx& c, uint64_t n, const uint32_t* d_pnn, uint64_t n_nn, const u
   }
   c.check_errors("pair lists");
   out.row_ptr.alloc(c, nseg + 1);
-  const uint64_t tiles = ceil_div(nseg + 1, SCAN_TILE);
-  DevBuf<uint32_t> sums(c, tiles);
-  scan_tiles_kernel<<<static_cast<unsigned>(tiles), SCAN_T, 0, c.stream>>>(cnt.get(), nseg + 1, out.row_ptr.get(),
-                                                                          sums.get());
-  PM_LAUNCHED();
-  scan_sums_kernel<<<1, SCAN_T, 0, c.stream>>>(sums.get(), tiles);
-  PM_LAUNCHED();
-  scan_add_kernel<<<ceil_div(nseg + 1, 256), 256, 0, c.stream>>>(out.row_ptr.get(), nseg + 1, sums.get());
-  PM_LAUNCHED();
+  exclusive_scan_u32(c, cnt.get(), nseg + 1, out.row_ptr.get());
   uint32_t total = 0;
   PM_CUDA(cudaMemcpyAsync(&total, out.row_ptr.get() + nseg, sizeof(uint32_t), cudaMemcpyDeviceToHost, c.stream));
   PM_CUDA(cudaStreamSynchronize(c.stream));
@@ -1100,6 +1006,18 @@ void optimize_device(Ctx& c, const Csr& csr, const OptimizeArgs& a) {
   const uint64_t n = a.n, dim = a.dim;
   if (a.itr_end <= a.itr_begin || n == 0 || dim == 0) return;
   PM_REQUIRE(dim <= 8, PACMAP_ERR_UNSUPPORTED, "the optimiser supports embedding dimensions 1..8");
+  if (a.h_loss && a.last_loss_only && a.itr_end - a.itr_begin > 1) {
+    // the iterations before the last without losses, which every form of the optimiser takes
+    OptimizeArgs b = a;
+    b.itr_end = a.itr_end - 1;
+    b.h_loss = nullptr;
+    b.d_grad_last = nullptr;
+    optimize_device(c, csr, b);
+    b = a;
+    b.itr_begin = a.itr_end - 1;
+    optimize_device(c, csr, b);
+    return;
+  }
   const GradFns fns = pick_grad_kernel(dim);
   const uint64_t total_iters = a.p1 + a.p2 + a.p3;
   const uint64_t sched_len = std::max<uint64_t>(total_iters, a.itr_end);
@@ -1134,7 +1052,16 @@ void optimize_device(Ctx& c, const Csr& csr, const OptimizeArgs& a) {
   ga.a1 = a1;
   ga.a2 = a2;
   ga.row_loss = a.h_loss ? row_loss.get() : nullptr;
-  Branch branch(csr.n_long > 0);  // the long rows run beside the others
+  // Many rows: the partners through shared memory, tile by tile (not with losses, which need every pair's term by row).
+  TileGrad tg;
+  // The tiles are copied 16 bytes at a time: y is the caller's buffer.
+  const bool tiled = !a.h_loss && (reinterpret_cast<uintptr_t>(a.d_y) & 15u) == 0 &&
+                     build_tile_grad(c, csr, n, dim, iters, tg);
+  if (tiled) {
+    ga.long_rows = tg.long_rows.get();
+    ga.n_long = tg.n_long;
+  }
+  Branch branch(ga.n_long > 0);  // the long rows run beside the others
 
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
@@ -1148,14 +1075,19 @@ void optimize_device(Ctx& c, const Csr& csr, const OptimizeArgs& a) {
     ga.y_cur = bufs[src];
     ga.y_next = bufs[dst];
     ga.grad_out = (itr + 1 == a.itr_end) ? a.d_grad_last : nullptr;
-    if (csr.n_long > 0) {
+    if (ga.n_long > 0) {
       capture_ok = branch.fork(c.stream) && capture_ok;
-      fns.long_rows<<<ceil_div(csr.n_long, 8), 256, 0, branch.stream>>>(ga, static_cast<int>(itr));
+      fns.long_rows<<<ceil_div(ga.n_long, 8), 256, 0, branch.stream>>>(ga, static_cast<int>(itr));
       ++launches;
     }
-    fns.rows<<<grid, 256, 0, c.stream>>>(ga, static_cast<int>(itr));
-    ++launches;
-    if (csr.n_long > 0) capture_ok = branch.join(c.stream) && capture_ok;
+    if (tiled) {
+      launch_tile_grad(tg, ga, dim, static_cast<int>(itr), c.stream);
+      launches += 2;
+    } else {
+      fns.rows<<<grid, 256, 0, c.stream>>>(ga, static_cast<int>(itr));
+      ++launches;
+    }
+    if (ga.n_long > 0) capture_ok = branch.join(c.stream) && capture_ok;
     if (a.h_loss) {
       loss_reduce_kernel<<<1, 1024, 0, c.stream>>>(row_loss.get(), n, loss_dev.get() + (itr - a.itr_begin));
       ++launches;
