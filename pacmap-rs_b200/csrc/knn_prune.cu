@@ -16,8 +16,9 @@
 // final comparison by a relative margin of 1e-4 that also covers the reference's own f32 distance sum.
 //
 // Pivots: k-means++ seeding (Arthur & Vassilvitskii, SODA 2007) in batches of 16 draws on a subsample of
-// at most 65,536 rows, so that every well-separated group of points receives a pivot and the cells stay
-// compact; the draws come from a Philox4x32-10 stream with a fixed key (the same pivots on every call).
+// at most 16,384 rows, then 16 times the point farthest from every pivot (Gonzalez, Theor. Comput. Sci. 38, 1985), so
+// that every well-separated group of points receives a pivot and the cells stay compact; the draws come from
+// a Philox4x32-10 stream with a fixed key (the same pivots on every call).
 #include <algorithm>
 #include <cmath>
 
@@ -29,8 +30,13 @@ namespace pacmap {
 namespace {
 
 constexpr int PV_BATCH = 16;             // pivots drawn per round
-constexpr uint32_t PV_SUB_MAX = 65536;   // subsample size limit
-constexpr int PV_CHUNK = 256;            // subsample points per block (and per prefix-sum entry)
+// The last pivots go to the farthest points: random draws alone left one or two of 200 groups without a pivot, whose
+// points then spread over other cells and spoiled their bounds (400,000 x 256 from 200 Gaussians: 788,000 of 4,886,000
+// tile pairs kept with 256 draws, 28,000 with 240 and 16 farthest).
+constexpr int PV_FAR = 16;
+// 64 points per pivot; four times as many took 0.8 ms longer on that data and pruned no better.
+constexpr uint32_t PV_SUB_MAX = 16384;   // subsample size limit
+constexpr int PV_CHUNK = 64;             // subsample points per block (and per prefix-sum entry)
 constexpr uint32_t TAG_PIVOT = 0x50495654u;  // 'PIVT'
 constexpr int SEGS = 4;                  // cell segments kept per tile (further cells merge into the last)
 constexpr float PRUNE_MARGIN = 1e-4f;    // relative margin of the skip test
@@ -57,7 +63,7 @@ __global__ void __launch_bounds__(256) pivot_dmin_kernel(const float* __restrict
   double ws = 0.0;
   // four subsample rows at a time (their loads in flight together); each row's sums and the order of
   // the block's double sum are those of one row at a time
-  static_assert(PER_WARP % 4 == 0, "rows are taken four at a time");
+  static_assert(PER_WARP % 4 == 0 && (PIV - PV_FAR) % PV_BATCH == 0, "rows are taken four at a time");
   for (int t0 = 0; t0 < PER_WARP; t0 += 4) {
     const uint32_t s0 = blockIdx.x * PV_CHUNK + warp * PER_WARP + t0;
     if (s0 >= S) break;  // warp-uniform
@@ -165,6 +171,53 @@ __global__ void __launch_bounds__(PV_BATCH * 32) pivot_draw_kernel(const float* 
     if (pick != 0xFFFFFFFFu) s = pick;
   }
   if (lane == 0) piv_rows[round * PV_BATCH + b] = static_cast<uint32_t>(sub_row(s, S, n));
+}
+
+// Step k of PV_FAR: dmin takes in the pivot that step k - 1 found (best[k - 1], written to piv_rows here), and best[k] the
+// largest dmin with its point: the distance's bits above, the complement of the point below (ties to the lower one).
+__device__ __forceinline__ uint32_t far_point(unsigned long long key) { return ~static_cast<uint32_t>(key); }
+__global__ void __launch_bounds__(256) pivot_far_kernel(const float* __restrict__ x, uint64_t n, int d, uint32_t S, int k,
+                                                        float* __restrict__ dmin,
+                                                        unsigned long long* __restrict__ best,
+                                                        uint32_t* __restrict__ piv_rows) {
+  __shared__ unsigned long long wbest[8];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint64_t q = 0;
+  if (k > 0) {
+    q = sub_row(far_point(best[k - 1]), S, n);
+    if (blockIdx.x == 0 && threadIdx.x == 0) piv_rows[PIV - PV_FAR + k - 1] = static_cast<uint32_t>(q);
+  }
+  unsigned long long mine = 0;
+  for (int t = 0; t < PV_CHUNK / 8; ++t) {
+    const uint32_t s = blockIdx.x * PV_CHUNK + warp * (PV_CHUNK / 8) + t;
+    if (s >= S) break;  // warp-uniform
+    float v = dmin[s];
+    if (k > 0) {
+      const float *a = x + sub_row(s, S, n) * d, *b = x + q * d;
+      float acc = 0.0f;
+      for (int col = lane; col < d; col += 32) {
+        const float df = a[col] - b[col];
+        acc = fmaf(df, df, acc);
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, o);
+      v = fminf(v, acc);
+      if (lane == 0) dmin[s] = v;
+    }
+    if (!(v < 3.0e38f)) v = 0.0f;
+    const unsigned long long key = (static_cast<unsigned long long>(__float_as_uint(v)) << 32) | ~s;
+    mine = key > mine ? key : mine;
+  }
+  if (lane == 0) wbest[warp] = mine;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) mine = wbest[w] > mine ? wbest[w] : mine;
+    atomicMax(&best[k], mine);
+  }
+}
+__global__ void pivot_far_last_kernel(uint64_t n, uint32_t S, const unsigned long long* __restrict__ best,
+                                      uint32_t* __restrict__ piv_rows) {
+  piv_rows[PIV - 1] = static_cast<uint32_t>(sub_row(far_point(best[PV_FAR - 1]), S, n));
 }
 
 __global__ void even_pivots_kernel(uint64_t n, uint32_t* __restrict__ piv_rows) {
@@ -501,13 +554,23 @@ void select_pivots(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint32_t* d
   PM_CUDA(cudaFuncSetAttribute(pivot_dmin_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
   pivot_draw_kernel<<<1, PV_BATCH * 32, 0, c.stream>>>(dmin.get(), S, n, csum.get(), nchunks, 0, d_piv_rows);
   PM_LAUNCHED();
-  for (int r = 1; r < PIV / PV_BATCH; ++r) {
+  constexpr int ROUNDS = (PIV - PV_FAR) / PV_BATCH;
+  for (int r = 1; r <= ROUNDS; ++r) {
     pivot_dmin_kernel<<<nchunks, 256, smem, c.stream>>>(d_x, n, static_cast<int>(d), S, d_piv_rows, (r - 1) * PV_BATCH,
                                                         dmin.get(), csum.get());
     PM_LAUNCHED();
+    if (r == ROUNDS) break;
     pivot_draw_kernel<<<1, PV_BATCH * 32, 0, c.stream>>>(dmin.get(), S, n, csum.get(), nchunks, r, d_piv_rows);
     PM_LAUNCHED();
   }
+  DevBuf<unsigned long long> best(c, PV_FAR);
+  PM_CUDA(cudaMemsetAsync(best.get(), 0, best.bytes(), c.stream));
+  for (int k = 0; k < PV_FAR; ++k) {
+    pivot_far_kernel<<<nchunks, 256, 0, c.stream>>>(d_x, n, static_cast<int>(d), S, k, dmin.get(), best.get(), d_piv_rows);
+    PM_LAUNCHED();
+  }
+  pivot_far_last_kernel<<<1, 1, 0, c.stream>>>(n, S, best.get(), d_piv_rows);
+  PM_LAUNCHED();
 }
 
 uint64_t build_pruned_tile_lists(Ctx& c, const PruneInputs& in, DevBuf<uint32_t>& ptr, DevBuf<uint32_t>& list) {
