@@ -211,6 +211,7 @@ __global__ void __launch_bounds__(MG_WARPS * 32) knn_merge_kernel(const uint64_t
   const uint64_t* src = part + s * static_cast<uint64_t>(slices) * K;
   for (int e = lane; e < K; e += 32) buf[e] = src[e];
   for (int q = 1; q < slices; ++q) {
+    if (src[static_cast<uint64_t>(q) * K] == ~0ull) continue;  // an empty list
     __syncwarp();
     for (int e = lane; e < K; e += 32) buf[K + e] = src[static_cast<uint64_t>(q) * K + e];
     for (int e = 2 * K + lane; e < P2; e += 32) buf[e] = ~0ull;

@@ -925,7 +925,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) knn_filter_kernel(
 //     bound of the reference's squared distance (scaled by s^2) over the columns the row met, u + n_i + 2 e_i
 //     rounded up -- an upper bound of its k'-th neighbour distance, since k' of those rank columns are
 //     other points;
-//     +inf when the row met fewer than rank columns or overflowed.
+//     +inf when the row met fewer than rank columns; 0 for a row that overflowed (no tile is visited for it: it is
+//     settled over its own column list).
 constexpr int RC_WARPS = 4;
 
 template <int PER>
@@ -940,7 +941,7 @@ __global__ void __launch_bounds__(RC_WARPS * 32) knn_compact_kernel(
        r += static_cast<uint64_t>(gridDim.x) * RC_WARPS) {
     const int m0 = min(cand_cnt[r], C);
     if (m0 <= 0 || (ub && m0 < rank)) {
-      if (ub && lane == 0) ub[r] = __int_as_float(0x7f800000);
+      if (ub && lane == 0) ub[r] = m0 < 0 ? 0.0f : __int_as_float(0x7f800000);
       if (theta_out && lane == 0) theta_out[r] = 3.402823466e+38f;  // every column met is still kept
       continue;
     }
@@ -1132,7 +1133,45 @@ __global__ void __launch_bounds__(WARPS * 32) knn_rerank_kernel(
 __global__ void overflow_mark_kernel(const uint32_t* __restrict__ rows, const uint32_t* __restrict__ count, int entries,
                                      int* __restrict__ cand_cnt) {
   for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < *count; t += gridDim.x * blockDim.x)
-    cand_cnt[rows[t]] = entries;
+    if (cand_cnt[rows[t]] < 0) cand_cnt[rows[t]] = entries;  // far rows keep their bound pass's band
+}
+
+// Far rows: after the bound pass, the few rows of a block whose bound is more than FAR_RATIO times (in squared distance) the
+// block's median bound, points apart from their cell. The tiles are chosen by a block's largest bounds, so six such
+// blocks of 400,000 rows in 256 columns visited 2,500 tiles each where the others visit 18, and the whole pass waited
+// for them: 6.0 ms, 0.3 without them. They join the overflowed rows instead: their bound no longer counts for their
+// block, their threshold lets nothing more in, and their bound pass's band gives them provisional neighbours.
+// Not when more than a quarter of a block would go (two cells of different density), or more than n / 64 in all.
+constexpr float FAR_RATIO = 4.0f;
+constexpr int FAR_BLOCK_MAX = TC_BM / 4;
+// Settling far rows apart takes about 0.6 ms; from 1,024 column tiles on a block that visits them all takes longer. (90,000
+// rows, 704 tiles: 4.4 ms without, 4.9 with.)
+constexpr uint64_t FAR_MIN_TILES = 1024;
+__global__ void __launch_bounds__(TC_BM) far_rows_kernel(uint64_t n, int rank, int blk0, const int* __restrict__ cand_cnt,
+                                                         const float* __restrict__ ub, uint32_t* __restrict__ rows,
+                                                         uint32_t* __restrict__ count) {
+  __shared__ float u_s[TC_BM];
+  __shared__ float median;
+  const uint64_t r = (static_cast<uint64_t>(blockIdx.x) + blk0) * TC_BM + threadIdx.x;
+  const bool in = r < n && cand_cnt[r] >= rank;
+  const float u = in ? ub[r] : __int_as_float(0x7f800000);
+  u_s[threadIdx.x] = u;
+  const int live = __syncthreads_count(in);
+  int below = 0;
+  for (int t = 0; t < TC_BM; ++t) below += (u_s[t] < u || (u_s[t] == u && t < static_cast<int>(threadIdx.x))) ? 1 : 0;
+  if (live > 0 && below == (live - 1) / 2) median = u;
+  __syncthreads();
+  const bool far = in && u <= 3.4e38f && u > FAR_RATIO * median;
+  const int total = __syncthreads_count(far);
+  if (far && total <= FAR_BLOCK_MAX) rows[atomicAdd(count, 1u)] = static_cast<uint32_t>(r);
+}
+__global__ void far_apply_kernel(const uint32_t* __restrict__ rows, uint32_t m, float* __restrict__ ub,
+                                 float* __restrict__ theta, uint32_t* __restrict__ ovf, uint32_t* __restrict__ n_ovf) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= m) return;
+  ub[rows[t]] = 0.0f;
+  theta[rows[t]] = -3.402823466e+38f;  // finite: the row is not an overflowed one
+  ovf[atomicAdd(n_ovf, 1u)] = rows[t];
 }
 
 // The operand rows, norms and thresholds of list rows [0, m) (padding up to the grid's rows is zeroed, with threshold
@@ -1481,6 +1520,21 @@ bool knn_tc_device(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint64_t kp
     DevBuf<float> ub(c, n_pad);
     resume.alloc(c, n_pad);
     compact(ub.get(), resume.get(), nullptr);
+    if (grid > 0 && ntl >= FAR_MIN_TILES) {
+      DevBuf<uint32_t> far(c, n + 1);
+      uint32_t n_far = 0;
+      PM_CUDA(cudaMemsetAsync(far.get() + n, 0, sizeof(uint32_t), c.stream));
+      far_rows_kernel<<<grid, TC_BM, 0, c.stream>>>(n, rank, static_cast<int>(blk0), ccnt.get(), ub.get(), far.get(),
+                                                    far.get() + n);
+      PM_LAUNCHED();
+      PM_CUDA(cudaMemcpyAsync(&n_far, far.get() + n, sizeof(uint32_t), cudaMemcpyDeviceToHost, c.stream));
+      PM_CUDA(cudaStreamSynchronize(c.stream));
+      if (n_far > 0 && n_far <= n / 64) {
+        far_apply_kernel<<<ceil_div(n_far, 256), 256, 0, c.stream>>>(far.get(), n_far, ub.get(), resume.get(), ovf.get(),
+                                                                    ovf.get() + n);
+        PM_LAUNCHED();
+      }
+    }
     PruneInputs in;
     in.perm = perm.get();
     in.cell = cell.get();
@@ -1565,7 +1619,7 @@ bool knn_tc_device(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint64_t kp
     const uint64_t blocks_fit = std::max<uint64_t>(1, WIDE_COLS_MAX / (n_pad * (TC_BM / 32)));
     const uint32_t blocks_max = static_cast<uint32_t>(
         std::min<uint64_t>({ceil_div(total, TC_BM), static_cast<uint64_t>(c.sm_count), blocks_fit}));
-    const uint32_t slices = static_cast<uint32_t>(std::min<uint64_t>(c.sm_count / blocks_max, ntl));
+    const uint32_t slices = static_cast<uint32_t>(std::min<uint64_t>(c.sm_count / blocks_max, ceil_div(ntl, 64)));
     const uint64_t m_max = static_cast<uint64_t>(blocks_max) * TC_BM, groups = m_max / 32;
     DevBuf<uint16_t> H2(c, m_max * KP);
     DevBuf<float> nrm2(c, m_max), theta2(c, m_max);
