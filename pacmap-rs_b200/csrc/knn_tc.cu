@@ -567,7 +567,9 @@ __device__ int g_debug_stall_loads = 0;
 // given (resume_theta) and stay fixed. Grid y splits the column tiles, and each epilogue warp writes the columns (as
 // original indices) that pass for any of its 32 rows: group g = row / 32 has n_pad places in wide_cols, slice y's
 // from its first column on, and its count in cand_cnt[g * gridDim.y + y].
-template <int KB, int PER, int MODE, bool WIDE = false>
+// RESUME: continues an earlier pass (resume_theta): without the chunks of a row's first tiles, whose code made the main
+// pass of 1,000,000 x 128 1.5 ms slower.
+template <int KB, int PER, int MODE, bool WIDE = false, bool RESUME = false>
 __global__ void __launch_bounds__(TC_THREADS, 1) knn_filter_kernel(
     const __grid_constant__ CUtensorMap hmap, const __grid_constant__ CUtensorMap gmap,
     const __grid_constant__ CUtensorMap amap, uint64_t n, uint64_t n_pad,
@@ -769,7 +771,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) knn_filter_kernel(
     int cnt = 0;
     if (WIDE) {
       if (valid) theta = resume_theta[row];
-    } else if (resume_theta && valid) {
+    } else if (RESUME && valid) {
       // continue from an earlier pass over other tiles: its compacted buffer and threshold (an overflowed
       // row stays overflowed; it is already listed for the exact fallback)
       const int c0 = cand_cnt[row];
@@ -789,6 +791,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) knn_filter_kernel(
     bool ok = true;
     uint32_t n_ins = 0, n_comp = 0;  // this row's insertions and compactions (statistics)
     const int cnt0 = cnt;            // entries carried over from an earlier pass
+    // no row of this warp has a threshold yet (warp-uniform; it stays false once one has)
+    bool open = !WIDE && !RESUME && __all_sync(0xFFFFFFFFu, theta == 3.402823466e+38f);
     auto screen = [&](const uint32_t (&r)[32], int colb) {
       const float* Dv = reinterpret_cast<const float*>(r);
       float m8[4];
@@ -811,6 +815,28 @@ __global__ void __launch_bounds__(TC_THREADS, 1) knn_filter_kernel(
         if (mine) wide_out[cnt + __popc(bal & ((1u << lane) - 1u))] = perm[colb + lane];
         cnt += __popc(bal);
         return;
+      }
+      if (!WIDE && !RESUME && open) {
+        // Before a row's first compaction every column passes: when that is so for all 32 rows and columns, each lane
+        // writes its 32 entries as eight whole sectors (its count is a multiple of 4: so far only whole chunks were
+        // written). Entry by entry they are four partial writes of each sector, and the first four tiles of every row
+        // made the bound pass wait for L2 (with its lists 20.0 ms for 1,000,000 x 128, 18.7 with whole sectors; 6.2 and
+        // 5.3 for 400,000 x 256).
+        float lo[4];
+#pragma unroll
+        for (int g = 0; g < 4; ++g)
+          lo[g] = fminf(fminf(fminf(Dv[8 * g], Dv[8 * g + 1]), fminf(Dv[8 * g + 2], Dv[8 * g + 3])),
+                        fminf(fminf(Dv[8 * g + 4], Dv[8 * g + 5]), fminf(Dv[8 * g + 6], Dv[8 * g + 7])));
+        if (__all_sync(0xFFFFFFFFu, fminf(fminf(lo[0], lo[1]), fminf(lo[2], lo[3])) >= hth && (cnt & 3) == 0)) {
+          uint2* out = cand + cbase + cnt;
+#pragma unroll
+          for (int c = 0; c < 32; c += 4)
+            st_global_v8(out + c, colb + c, __float_as_uint(-2.0f * Dv[c]), colb + c + 1,
+                         __float_as_uint(-2.0f * Dv[c + 1]), colb + c + 2, __float_as_uint(-2.0f * Dv[c + 2]),
+                         colb + c + 3, __float_as_uint(-2.0f * Dv[c + 3]));
+          cnt += 32;
+          return;
+        }
       }
       if (__any_sync(0xFFFFFFFFu, m >= hth)) {
         // every column of the 32 without a branch: a predicated store of (j, v = -2 D) that also returns the
@@ -848,6 +874,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) knn_filter_kernel(
       // The next row's entries are loaded before the current row is compacted (their latency overlaps).
       unsigned need = __ballot_sync(0xFFFFFFFFu, cnt > C - TC_BN);
       if (need) {
+        open = false;
         int L = __ffs(need) - 1;
         need &= need - 1;
         RowRegs<PER> cur;
@@ -1465,28 +1492,24 @@ bool knn_tc_device(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint64_t kp
                                                  static_cast<int>(blk0), lptr, llist, resume_theta, e4max.get(),
                                                  counters.get(), nullptr);
     };
-    const bool p16 = PER == 16;
-    if (mode == MODE_STREAM) {
-      constexpr size_t sm = FilterLayout<0, MODE_STREAM>::SMEM;
-      if (p16) launch(knn_filter_kernel<0, 16, MODE_STREAM>, sm);
-      else launch(knn_filter_kernel<0, 32, MODE_STREAM>, sm);
-    } else if (KB == 1) {
-      constexpr size_t sm = FilterLayout<1, MODE_TILE>::SMEM;
-      if (p16) launch(knn_filter_kernel<1, 16, MODE_TILE>, sm);
-      else launch(knn_filter_kernel<1, 32, MODE_TILE>, sm);
-    } else if (KB == 2) {
-      constexpr size_t sm = FilterLayout<2, MODE_TILE>::SMEM;
-      if (p16) launch(knn_filter_kernel<2, 16, MODE_TILE>, sm);
-      else launch(knn_filter_kernel<2, 32, MODE_TILE>, sm);
-    } else if (KB == 3) {
-      constexpr size_t sm = FilterLayout<3, MODE_KBLOCK>::SMEM;
-      if (p16) launch(knn_filter_kernel<3, 16, MODE_KBLOCK>, sm);
-      else launch(knn_filter_kernel<3, 32, MODE_KBLOCK>, sm);
-    } else {
-      constexpr size_t sm = FilterLayout<4, MODE_KBLOCK>::SMEM;
-      if (p16) launch(knn_filter_kernel<4, 16, MODE_KBLOCK>, sm);
-      else launch(knn_filter_kernel<4, 32, MODE_KBLOCK>, sm);
-    }
+    // the kernel for this data width and buffer size, starting or resuming
+    auto pick = [&](auto kb, auto md) {
+      constexpr int K = decltype(kb)::value, M = decltype(md)::value;
+      constexpr size_t sm = FilterLayout<K, M>::SMEM;
+      if (PER == 16) {
+        if (resume_theta) launch(knn_filter_kernel<K, 16, M, false, true>, sm);
+        else launch(knn_filter_kernel<K, 16, M>, sm);
+      } else {
+        if (resume_theta) launch(knn_filter_kernel<K, 32, M, false, true>, sm);
+        else launch(knn_filter_kernel<K, 32, M>, sm);
+      }
+    };
+    using std::integral_constant;
+    if (mode == MODE_STREAM) pick(integral_constant<int, 0>(), integral_constant<int, MODE_STREAM>());
+    else if (KB == 1) pick(integral_constant<int, 1>(), integral_constant<int, MODE_TILE>());
+    else if (KB == 2) pick(integral_constant<int, 2>(), integral_constant<int, MODE_TILE>());
+    else if (KB == 3) pick(integral_constant<int, 3>(), integral_constant<int, MODE_KBLOCK>());
+    else pick(integral_constant<int, 4>(), integral_constant<int, MODE_KBLOCK>());
     PM_LAUNCHED();
   };
   const unsigned cgrid = std::min<unsigned>(ceil_div(n, RC_WARPS), c.sm_count * 16);
