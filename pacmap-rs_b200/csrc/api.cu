@@ -299,8 +299,10 @@ void fit_transform_impl(Ctx& c, const float* d_x, uint64_t n, uint64_t d, const 
   if (mlp_params && t_mean && t_std) {
     // learned initialiser in the training embedding's coordinates: MLP(x') * std + mean, where the plain
     // schedule would have placed the points (the network predicts standardised coordinates)
-    mlp_apply_device(c, mlp_params, d, dim, xp.get(), n, d_out);
-    destandardise_device(c, d_out, n, dim, t_mean, t_std);
+    MlpAffine around;
+    around.t_mean = t_mean;
+    around.t_std = t_std;
+    mlp_apply_device(c, mlp_params, d, dim, xp.get(), n, d_out, around);
   } else if (mlp_params) {
     // learned initialiser: MLP(x') as Initialization::Value (lib.rs:753-766 z-scores it to std 1e-4)
     DevBuf<float> raw(c, n * dim);

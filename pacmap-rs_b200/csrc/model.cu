@@ -37,27 +37,6 @@ uint64_t fnv1a(const unsigned char* p, size_t n) {
   return h;
 }
 
-// x' = ((x - min) / max) - mean[c] in preprocess_x's three f32 roundings (src/lib.rs:500-511).
-__global__ void apply_preprocess_kernel(const float* __restrict__ x, uint64_t n, uint64_t d, float mn, float mx,
-                                        const float* __restrict__ mean, float* __restrict__ out) {
-  const uint64_t total = n * d;
-  const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-  for (uint64_t t = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; t < total; t += stride) {
-    const uint64_t c = t % d;
-    out[t] = __fsub_rn(__fdiv_rn(__fsub_rn(x[t], mn), mx), mean[c]);
-  }
-}
-
-// y = z * std + mean per dimension (ms: mean[dim] then std[dim]).
-__global__ void destandardise_kernel(float* __restrict__ y, uint64_t n, uint64_t dim, const float* __restrict__ ms) {
-  const uint64_t total = n * dim;
-  const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-  for (uint64_t t = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; t < total; t += stride) {
-    const uint64_t c = t % dim;
-    y[t] = __fadd_rn(__fmul_rn(y[t], ms[dim + c]), ms[c]);
-  }
-}
-
 struct Writer {
   std::vector<unsigned char> buf;
   template <typename T>
@@ -164,42 +143,13 @@ void model_load(const char* path, uint64_t* d_out, uint64_t* dim_out, float* par
   r.get_f32(params, count);
 }
 
-void destandardise_device(Ctx& c, float* d_y, uint64_t n, uint64_t dim, const float* t_mean, const float* t_std) {
-  std::vector<float> ms(2 * dim);
-  for (uint64_t k = 0; k < dim; ++k) {
-    ms[k] = t_mean[k];
-    ms[dim + k] = t_std[k];
-  }
-  DevBuf<float> dms;
-  upload(c, dms, ms.data(), 2 * dim);
-  const unsigned g = static_cast<unsigned>(std::min<uint64_t>(ceil_div(n * dim, 256), c.sm_count * 16ull));
-  destandardise_kernel<<<g, 256, 0, c.stream>>>(d_y, n, dim, dms.get());
-  PM_LAUNCHED();
-}
-
 void transform_device(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint64_t dim, const float* params,
                       float pre_min, float pre_max, const float* pre_mean, const float* t_mean, const float* t_std,
                       float* d_out) {
   if (n == 0) return;
   PM_REQUIRE(d >= 1 && d <= kMaxD && dim >= 1 && dim <= kMaxDim, PACMAP_ERR_UNSUPPORTED,
              "models support d <= 4096 and dim <= 16");
-  DevBuf<float> xp(c, n * d), consts;
-  upload(c, consts, pre_mean, d);
-  std::vector<float> ms(2 * dim);
-  for (uint64_t k = 0; k < dim; ++k) {
-    ms[k] = t_mean[k];
-    ms[dim + k] = t_std[k];
-  }
-  DevBuf<float> dms;
-  upload(c, dms, ms.data(), 2 * dim);
-  const unsigned g = static_cast<unsigned>(std::min<uint64_t>(ceil_div(n * d, 256), c.sm_count * 16ull));
-  apply_preprocess_kernel<<<g, 256, 0, c.stream>>>(d_x, n, d, pre_min, pre_max, consts.get(), xp.get());
-  PM_LAUNCHED();
-  mlp_apply_device(c, params, d, dim, xp.get(), n, d_out);
-  const unsigned g2 = static_cast<unsigned>(std::min<uint64_t>(ceil_div(n * dim, 256), c.sm_count * 16ull));
-  destandardise_kernel<<<g2, 256, 0, c.stream>>>(d_out, n, dim, dms.get());
-  PM_LAUNCHED();
-  c.check_errors("transform");
+  mlp_apply_device(c, params, d, dim, d_x, n, d_out, MlpAffine{pre_min, pre_max, pre_mean, t_mean, t_std});
 }
 
 }  // namespace pacmap
