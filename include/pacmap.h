@@ -337,6 +337,12 @@ pacmap_status pacmap_debug_stall_knn_loads(int32_t device, int32_t on);
  * gradient uses for its pair factors. x, out: n values of host memory. */
 pacmap_status pacmap_debug_divide(float num, const float* x, uint64_t n, int32_t device, float* out);
 
+/* Test hook (no reference analogue): the k <= 8 leading eigenvectors of a symmetric d x d matrix, 2 <= d <= 160, by
+ * the one-block Jacobi kernel that the Pca initialisation uses. *found = 0, out_axes untouched, where that kernel
+ * leaves the matrix to the host (eigenvalues too close together, or not finite). cov, out_axes: host memory. */
+pacmap_status pacmap_debug_small_axes(const double* cov, uint64_t d, uint64_t k, int32_t device, double* out_axes,
+                                      int32_t* found);
+
 /* The message of the last failure on this thread ("" after success). */
 const char* pacmap_last_error(void);
 

@@ -560,6 +560,15 @@ pacmap_status pacmap_pca_axes_device(const double* cov, uint64_t d, uint64_t k, 
   });
 }
 
+pacmap_status pacmap_debug_small_axes(const double* cov, uint64_t d, uint64_t k, int32_t device, double* out_axes,
+                                      int32_t* out_found) {
+  return guarded([&] {
+    PM_REQUIRE(cov && out_axes && out_found, PACMAP_ERR_INVALID_ARGUMENT, "NULL buffer");
+    DeviceLock dl(device);
+    *out_found = pca_small_axes_device(dl.ctx, cov, d, k, out_axes) ? 1 : 0;
+  });
+}
+
 pacmap_status pacmap_model_target_stats(const float* y, uint64_t n, uint64_t dim, float* out_mean, float* out_std) {
   return guarded([&] {
     PM_REQUIRE(y && out_mean && out_std, PACMAP_ERR_INVALID_ARGUMENT, "NULL buffer");

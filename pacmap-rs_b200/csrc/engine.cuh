@@ -139,6 +139,9 @@ void pca_project_device(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint64
 void pca_top_axes(const double* cov, uint64_t d, uint64_t k, double* axes);
 // The same axes, bit for bit, from the device's subspace iteration (160 < d <= 1024, k <= 128).
 void pca_top_axes_device(Ctx& c, const double* cov, uint64_t d, uint64_t k, double* axes);
+// The axes from one block's Jacobi sweeps (2 <= d <= 160, k <= 8; cov in host memory); false, with axes untouched,
+// where the host's sweeps have to decide.
+bool pca_small_axes_device(Ctx& c, const double* cov, uint64_t d, uint64_t k, double* axes);
 // d_out (n x k) = scale * x[:, :k] for x (n x w).
 void leading_columns(Ctx& c, const float* d_x, uint64_t n, uint64_t w, uint64_t k, float scale, float* d_out);
 void init_random_device(Ctx& c, uint64_t n, uint64_t dim, uint64_t seed, float* d_y);

@@ -7,10 +7,11 @@
 //   1. column means (f64, fixed-order two-level sums);
 //   2. the d x d covariance of the centred rows in f64: at most 64 row chunks (of at least 16,384 rows)
 //      write 32 x 32 partial tiles, reduced over the chunks in order (deterministic, no atomics);
-//   3. the top-k axes (f64): cyclic Jacobi of the whole matrix on the host for d <= 160, above that
-//      subspace iteration on k + 24 vectors with a Rayleigh-Ritz step (the power iteration the
-//      reference's randomized SVD uses), on the GPU when the data is there (top_axes_device) and on the
-//      host for pacmap_pca_axes, with the same operations in the same order: the axes are the same bits;
+//   3. the top-k axes (f64): for d <= 160 Jacobi of the whole matrix, in one block for k <= 8 well separated axes
+//      (jacobi_kernel) and cyclic on the host otherwise; above that subspace iteration on k + 24 vectors with a
+//      Rayleigh-Ritz step (the power iteration the reference's randomized SVD uses), on the GPU when the data
+//      is there (top_axes_device) and on the host for pacmap_pca_axes, with the same operations in the same
+//      order: the axes are the same bits;
 //      axes by descending variance, each axis's largest-magnitude loading made positive (the reference's
 //      SVD sign is LAPACK's and unpinned);
 //   4. the projection (x - mean) V_k by a tiled f32 kernel with f64 accumulation.
@@ -445,6 +446,206 @@ std::vector<double> top_axes_device(Ctx& c, const double* d_cov, int d, int k) {
   return leading_axes(vecs, w, d, m, k);
 }
 
+// Jacobi's method for a symmetric d x d matrix, 2 <= d <= 160, and up to eight leading eigenvectors: one block, the
+// matrix in shared memory (zero-padded to an even order n, row length ld odd so that a column's elements fall in
+// different banks; only the upper triangle is kept up to date). A sweep is n - 1 steps of n / 2 rotations on disjoint
+// index pairs (the round-robin order of Brent and Luk, SIAM J. Sci. Stat. Comput. 6, 1985): a thread per pair finds
+// the rotation, then a thread per two pairs turns their 2 x 2 block of the matrix. The rotations go to rot; the
+// wanted eigenvectors are unit vectors taken back through them, so that the full eigenvector matrix is never formed.
+// out: status (1: converged and the leading k + 1 eigenvalues lie JACOBI_GAP of the largest apart), the k leading
+// eigenvalues, the eigenvectors (d x k, row-major). Bound by each step's serial chain: two divisions, a square root
+// and a reciprocal square root in f64, then the block's products, with a barrier after either (1.2 us a step, 890
+// steps at d = 100). A 2,000 x 100 fit from the principal axes: 12.1 ms with the host's sweeps, 4.4 ms so.
+constexpr int JACOBI_THREADS = 1024, JACOBI_MAX_K = 8, JACOBI_SWEEPS = 20, JACOBI_AHEAD = 8;
+constexpr int JACOBI_BLOCKS = ((JACOBI_MAX_D / 2) * (JACOBI_MAX_D / 2 - 1) / 2 + JACOBI_THREADS - 1) / JACOBI_THREADS;
+// The device from 32 columns on: 216 us against the host's 255 at 32 (copies in and out included), 162 against 123
+// at 24, 1.12 ms against 6.9 at 100, 3.0 against 63 at 160. Its residuals are the smaller (2e-15 of the largest
+// eigenvalue against 1e-14 at 100), and the f32 axes of 120 covariances of both kinds came out the same.
+// JACOBI_GAP: axes whose eigenvalues lie closer than this (of the largest) depend on the order of the rotations in
+// digits that f32 keeps, and equal eigenvalues leave the choice of basis to it, so the host's cyclic order stays
+// for those; above it the two methods' axes differ by about 1e-12, far below f32. Eight axes: the start's dim; the
+// 100 axes of the wide data's reduction have closer pairs among them as a rule.
+constexpr int JACOBI_MIN_D = 32;
+constexpr double JACOBI_GAP = 1e-3;
+static_assert(JACOBI_MAX_K * JACOBI_MAX_D / 2 <= JACOBI_THREADS, "a thread per vector and pair");
+size_t jacobi_smem(int d) {
+  const int n = d + (d & 1);
+  return (static_cast<size_t>(n) * (n | 1) + n) * sizeof(double) + static_cast<size_t>(n) * sizeof(int) +
+         static_cast<size_t>(n / 2) * sizeof(double2);
+}
+
+// Pair number i of step s, 0 <= i < n / 2, 0 <= s < n - 1 = m: (s, m) for i = 0, else s + i and s - i modulo m.
+__device__ __forceinline__ void jacobi_pair(int i, int s, int m, int& p, int& q) {
+  p = s + i < m ? s + i : s + i - m;
+  q = i == 0 ? m : (s - i >= 0 ? s - i : s - i + m);
+}
+
+__global__ void __launch_bounds__(JACOBI_THREADS)
+    jacobi_kernel(const double* __restrict__ cov, int d, int k, double2* __restrict__ rot, double* __restrict__ out) {
+  extern __shared__ __align__(16) char jacobi_shared[];
+  __shared__ double part[JACOBI_THREADS / 32];
+  __shared__ double sum;
+  __shared__ int ok;
+  const int tid = threadIdx.x, n = d + (d & 1), m = n - 1, h = n / 2, ld = n | 1;
+  double2* cs = reinterpret_cast<double2*>(jacobi_shared);  // [h] this step's cosines and sines
+  double* a = reinterpret_cast<double*>(cs + h);            // [n][ld]
+  double* w = a + static_cast<size_t>(n) * ld;              // [n] eigenvalues
+  int* order = reinterpret_cast<int*>(w + n);               // [n] columns by descending eigenvalue
+  auto at = [&](int i, int j) -> double& { return i < j ? a[i * ld + j] : a[j * ld + i]; };
+  // the sum of v over the block's threads, in a fixed order
+  auto block_sum = [&](double v) {
+#pragma unroll
+    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if ((tid & 31) == 0) part[tid >> 5] = v;
+    __syncthreads();
+    if (tid < 32) {
+      double t = part[tid];
+#pragma unroll
+      for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if (tid == 0) sum = t;
+    }
+    __syncthreads();
+    return sum;
+  };
+  double sq = 0.0;
+  for (int e = tid; e < n * n; e += JACOBI_THREADS) {
+    const int i = e / n, j = e % n;
+    const double v = i < d && j < d ? cov[i * d + j] : 0.0;
+    a[i * ld + j] = v;
+    sq += v * v;
+  }
+  if (tid < n) order[tid] = tid;  // every entry a column, whatever the comparisons below make of a NaN
+  const double total = block_sum(sq);
+  // this thread's two pairs of pairs I < J (the same numbers in every step)
+  int bi[JACOBI_BLOCKS], bj[JACOBI_BLOCKS];
+#pragma unroll
+  for (int b = 0; b < JACOBI_BLOCKS; ++b) {
+    int e = tid + b * JACOBI_THREADS, i = 0;
+    bi[b] = -1;
+    bj[b] = 0;
+    if (e < h * (h - 1) / 2) {
+      while (e >= h - 1 - i) e -= h - 1 - i++;
+      bi[b] = i;
+      bj[b] = i + 1 + e;
+    }
+  }
+  int sweep = 0;
+  bool done = false;
+  for (;; ++sweep) {
+    double off = 0.0;
+    for (int e = tid; e < n * n; e += JACOBI_THREADS) {
+      const int i = e / n, j = e % n;
+      if (i < j) off += a[i * ld + j] * a[i * ld + j];
+    }
+    off = block_sum(off);
+    done = off <= 1e-30 * total;  // false for NaN
+    if (done || sweep == JACOBI_SWEEPS) break;
+    for (int s = 0; s < m; ++s) {
+      if (tid < h) {
+        int p, q;
+        jacobi_pair(tid, s, m, p, q);
+        double& apq = at(p, q);
+        double c = 1.0, t = 0.0;
+        if (fabs(apq) >= 1e-300) {
+          double &app = a[p * ld + p], &aqq = a[q * ld + q];
+          const double theta = (aqq - app) / (2.0 * apq);
+          t = (theta >= 0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
+          c = rsqrt(t * t + 1.0);
+          app -= t * apq;
+          aqq += t * apq;
+          apq = 0.0;
+        }
+        cs[tid] = make_double2(c, t * c);
+        rot[(static_cast<size_t>(sweep) * m + s) * h + tid] = cs[tid];
+      }
+      __syncthreads();
+#pragma unroll
+      for (int b = 0; b < JACOBI_BLOCKS; ++b) {
+        if (bi[b] < 0) continue;
+        int p, q, r, u;
+        jacobi_pair(bi[b], s, m, p, q);
+        jacobi_pair(bj[b], s, m, r, u);
+        const double2 x = cs[bi[b]], y = cs[bj[b]];
+        double &e00 = at(p, r), &e01 = at(p, u), &e10 = at(q, r), &e11 = at(q, u);
+        const double f00 = x.x * e00 - x.y * e10, f01 = x.x * e01 - x.y * e11;
+        const double f10 = x.y * e00 + x.x * e10, f11 = x.y * e01 + x.x * e11;
+        e00 = y.x * f00 - y.y * f01;
+        e01 = y.y * f00 + y.x * f01;
+        e10 = y.x * f10 - y.y * f11;
+        e11 = y.y * f10 + y.x * f11;
+      }
+      __syncthreads();
+    }
+  }
+  // the order of the eigenvalues, descending, equal ones by column
+  if (tid < d) w[tid] = a[tid * ld + tid];
+  if (tid == 0) ok = done;
+  __syncthreads();
+  if (!ok) {
+    if (tid == 0) out[0] = 0.0;
+    return;
+  }
+  if (tid < d) {
+    int rank = 0;
+    for (int j = 0; j < d; ++j) rank += w[j] > w[tid] || (w[j] == w[tid] && j < tid);
+    order[rank] = tid;
+  }
+  __syncthreads();
+  if (tid < k && tid + 1 < d && !(w[order[tid]] - w[order[tid + 1]] > JACOBI_GAP * w[order[0]])) ok = 0;
+  __syncthreads();
+  if (!ok) {
+    if (tid == 0) out[0] = 0.0;
+    return;
+  }
+  if (tid == 0) out[0] = 1.0;
+  if (tid < k) out[1 + tid] = w[order[tid]];
+  // eigenvector v is J_1 J_2 ... e_{order[v]}: vector v's pair i belongs to thread v * h + i; a is reused, [k][n]
+  const int v = tid / h, i = tid % h;
+  __syncthreads();
+  for (int e = tid; e < k * n; e += JACOBI_THREADS) a[e] = e % n == order[e / n] ? 1.0 : 0.0;
+  __syncthreads();
+  for (int step = sweep * m - 1; step >= 0;) {
+    const int batch = min(JACOBI_AHEAD, step + 1);
+    double2 r[JACOBI_AHEAD];
+#pragma unroll
+    for (int b = 0; b < JACOBI_AHEAD; ++b)
+      if (b < batch && v < k) r[b] = rot[static_cast<size_t>(step - b) * h + i];
+#pragma unroll
+    for (int b = 0; b < JACOBI_AHEAD; ++b) {
+      if (b < batch && v < k) {
+        int p, q;
+        jacobi_pair(i, (step - b) % m, m, p, q);
+        const double xp = a[v * n + p], xq = a[v * n + q];
+        a[v * n + p] = r[b].x * xp + r[b].y * xq;
+        a[v * n + q] = r[b].x * xq - r[b].y * xp;
+      }
+      __syncthreads();
+    }
+    step -= batch;
+  }
+  for (int e = tid; e < d * k; e += JACOBI_THREADS) out[1 + k + e] = a[(e % k) * n + e / k];
+}
+
+// top_axes for d <= JACOBI_MAX_D and k <= JACOBI_MAX_K with the covariance on the device; empty when the host's
+// sequence of rotations has to decide (see JACOBI_GAP) or the sweeps ran out (a NaN or an infinity in the matrix).
+std::vector<double> small_axes_device(Ctx& c, const double* d_cov, int d, int k) {
+  PM_REQUIRE(d >= 2 && d <= JACOBI_MAX_D && k >= 1 && k <= std::min(d, JACOBI_MAX_K), PACMAP_ERR_UNSUPPORTED,
+             "the one-block Jacobi takes 2 <= d <= 160 and k <= 8");
+  const int n = d + (d & 1);
+  DevBuf<double2> rot(c, static_cast<uint64_t>(JACOBI_SWEEPS) * (n - 1) * (n / 2));
+  DevBuf<double> out(c, 1 + static_cast<uint64_t>(k) + static_cast<uint64_t>(d) * k);
+  const size_t smem = jacobi_smem(d);
+  PM_CUDA(cudaFuncSetAttribute(jacobi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  jacobi_kernel<<<1, JACOBI_THREADS, smem, c.stream>>>(d_cov, d, k, rot.get(), out.get());
+  PM_LAUNCHED();
+  std::vector<double> h(out.count);
+  PM_CUDA(cudaMemcpyAsync(h.data(), out.get(), out.bytes(), cudaMemcpyDeviceToHost, c.stream));
+  PM_CUDA(cudaStreamSynchronize(c.stream));
+  if (h[0] != 1.0) return {};
+  const std::vector<double> w(h.begin() + 1, h.begin() + 1 + k), vecs(h.begin() + 1 + k, h.end());
+  return leading_axes(vecs, w, d, k, k);
+}
+
 // out (n x k) = scale * x[:, :k] for x (n x w).
 __global__ void leading_columns_kernel(const float* __restrict__ x, uint64_t n, uint64_t w, uint64_t k, float scale,
                                        float* __restrict__ out) {
@@ -473,6 +674,16 @@ void pca_top_axes_device(Ctx& c, const double* cov, uint64_t d, uint64_t k, doub
   upload(c, dc, cov, d * d);
   const std::vector<double> V = top_axes_device(c, dc.get(), static_cast<int>(d), static_cast<int>(k));
   std::copy(V.begin(), V.end(), axes);
+}
+
+bool pca_small_axes_device(Ctx& c, const double* cov, uint64_t d, uint64_t k, double* axes) {
+  PM_REQUIRE(d <= static_cast<uint64_t>(JACOBI_MAX_D) && k <= static_cast<uint64_t>(JACOBI_MAX_K),
+             PACMAP_ERR_UNSUPPORTED, "the one-block Jacobi takes 2 <= d <= 160 and k <= 8");
+  DevBuf<double> dc;
+  upload(c, dc, cov, d * d);
+  const std::vector<double> V = small_axes_device(c, dc.get(), static_cast<int>(d), static_cast<int>(k));
+  std::copy(V.begin(), V.end(), axes);
+  return !V.empty();
 }
 
 void leading_columns(Ctx& c, const float* d_x, uint64_t n, uint64_t w, uint64_t k, float scale, float* d_out) {
@@ -507,7 +718,10 @@ void pca_project_device(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint64
   std::vector<double> V64;
   if (d > static_cast<uint64_t>(JACOBI_MAX_D)) {
     V64 = top_axes_device(c, cov.get(), static_cast<int>(d), static_cast<int>(k));
-  } else {
+  } else if (d >= static_cast<uint64_t>(JACOBI_MIN_D) && k <= static_cast<uint64_t>(JACOBI_MAX_K)) {
+    V64 = small_axes_device(c, cov.get(), static_cast<int>(d), static_cast<int>(k));
+  }
+  if (V64.empty()) {
     std::vector<double> a(d * d);
     PM_CUDA(cudaMemcpyAsync(a.data(), cov.get(), d * d * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
     PM_CUDA(cudaStreamSynchronize(c.stream));
