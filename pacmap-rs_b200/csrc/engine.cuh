@@ -131,7 +131,7 @@ void normalize_rows_device(Ctx& c, float* d_x, uint64_t n, uint64_t d);
 
 // ---- pca.cu: Initialization::Pca ----
 // d_out (n x k) = scale * (x - column mean) V_k with V_k the k leading principal axes of x (n x d);
-// axes_out (optional) receives V_k (d x k, row-major). k <= 128, d <= 1024.
+// axes_out (optional) receives V_k (d x k, row-major). k <= 104, d <= 1024.
 void pca_project_device(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint64_t k, float scale, float* d_out,
                         std::vector<float>* axes_out);
 // The k leading eigenvectors of a symmetric d x d matrix (host, f64): axes (d x k, row-major), by

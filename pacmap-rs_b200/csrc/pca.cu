@@ -6,7 +6,7 @@
 //
 //   1. column means (f64, fixed-order two-level sums);
 //   2. the d x d covariance of the centred rows in f64: at most 64 row chunks (of at least 16,384 rows)
-//      write 32 x 32 partial tiles, reduced over the chunks in order (deterministic, no atomics);
+//      write partial tiles, reduced over the chunks in order (deterministic, no atomics);
 //   3. the top-k axes (f64): for d <= 160 Jacobi of the whole matrix, in one block for k <= 8 well separated axes
 //      (jacobi_kernel) and cyclic on the host otherwise; above that subspace iteration on k + 24 vectors with a
 //      Rayleigh-Ritz step (the power iteration the reference's randomized SVD uses), on the GPU when the data
@@ -27,9 +27,8 @@
 namespace pacmap {
 namespace {
 
-constexpr int PCA_T = 32;           // covariance tile (32 x 32 outputs)
 constexpr uint64_t PCA_MAX_CHUNKS = 64;  // partial covariances (row chunks of at least 16,384 rows)
-constexpr int MEAN_BLOCKS = 256;
+constexpr int MEAN_BLOCKS = 256, MEAN_AHEAD = 16;  // row ranges of the mean; loads in flight per thread
 
 __global__ void __launch_bounds__(256) col_sum_partial_kernel(const float* __restrict__ x, uint64_t n, uint64_t d,
                                                               double* __restrict__ partial) {
@@ -38,7 +37,15 @@ __global__ void __launch_bounds__(256) col_sum_partial_kernel(const float* __res
   const uint64_t r0 = static_cast<uint64_t>(blockIdx.x) * rpb, r1 = r0 + rpb < n ? r0 + rpb : n;
   for (uint64_t c = threadIdx.x; c < d; c += blockDim.x) {
     double s = 0.0;
-    for (uint64_t r = r0; r < r1; ++r) s += x[r * d + c];
+    uint64_t r = r0;
+    for (; r + MEAN_AHEAD <= r1; r += MEAN_AHEAD) {
+      float v[MEAN_AHEAD];
+#pragma unroll
+      for (int q = 0; q < MEAN_AHEAD; ++q) v[q] = x[(r + q) * d + c];
+#pragma unroll
+      for (int q = 0; q < MEAN_AHEAD; ++q) s += v[q];
+    }
+    for (; r < r1; ++r) s += x[r * d + c];
     partial[static_cast<uint64_t>(blockIdx.x) * d + c] = s;
   }
 }
@@ -48,94 +55,147 @@ __global__ void col_mean_final_kernel(const double* __restrict__ partial, int pa
   const uint64_t c = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (c >= d) return;
   double s = 0.0;
+#pragma unroll 16
   for (int b = 0; b < parts; ++b) s += partial[static_cast<uint64_t>(b) * d + c];
   mean[c] = s / static_cast<double>(n);
 }
 
-// Partial covariance of one row chunk for one 32 x 32 tile (ti, tj): thread (ty, tx) of a 32 x 8 block
-// owns outputs (ti * 32 + ty, tj * 32 + tx + 8q), q < 4.
-__global__ void __launch_bounds__(256) cov_partial_kernel(const float* __restrict__ x, uint64_t n, uint64_t d,
+// Partial covariance of one row chunk (blockIdx.y) for one pair of column tiles ti <= tj (blockIdx.x): E x E threads
+// of R x R outputs, slabs of centred rows in two buffers, the next slab's values in registers meanwhile. Each output
+// is one chain of fused multiply-adds over the chunk's rows in order, whatever the tile; the products commute, so the
+// tiles below the diagonal would hold the same bits and are not computed. Bound by the operands' way out of shared
+// memory: 32 R cycles a row of a 16 R wide tile, against 4 R^2 in the f64 units (64 fused multiply-adds per clock and
+// SM). 60,000 x 784: 11.1 ms with 32 x 32 tiles over the whole square, one output of a row by four columns a thread
+// and nothing in flight; 2.9 ms so.
+template <int R, int E>
+__global__ void __launch_bounds__(E * E) cov_partial_kernel(const float* __restrict__ x, uint64_t n, uint64_t d,
                                                           uint64_t rows_per_chunk, const double* __restrict__ mean,
                                                           double* __restrict__ partial) {
-  __shared__ double a[PCA_T][PCA_T + 1], b[PCA_T][PCA_T + 1];  // [row][column]
-  const int ti = blockIdx.x, tj = blockIdx.y;
-  const uint64_t chunk = blockIdx.z;
+  constexpr int T = E * R, S = R == 4 ? 16 : 32, PASS = E * E / T, LOADS = S / PASS;
+  __shared__ __align__(16) double a[2][S][T], b[2][S][T];  // [buffer][row][column]
+  int ti = 0, rest = blockIdx.x;
+  for (const int tiles = static_cast<int>((d + T - 1) / T); rest >= tiles - ti;) rest -= tiles - ti++;
+  const int tj = ti + rest;
+  const uint64_t chunk = blockIdx.y;
   const uint64_t r0 = chunk * rows_per_chunk, r1 = r0 + rows_per_chunk < n ? r0 + rows_per_chunk : n;
-  const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;  // ty 0..31
-  double acc[4] = {0.0, 0.0, 0.0, 0.0};
-  for (uint64_t rb = r0; rb < r1; rb += PCA_T) {
-    __syncthreads();
-    for (int e = threadIdx.x; e < PCA_T * PCA_T; e += 256) {
-      const int rr = e / PCA_T, cc = e % PCA_T;
-      const uint64_t r = rb + rr;
-      const uint64_t ci = static_cast<uint64_t>(ti) * PCA_T + cc, cj = static_cast<uint64_t>(tj) * PCA_T + cc;
-      a[rr][cc] = (r < r1 && ci < d) ? static_cast<double>(x[r * d + ci]) - mean[ci] : 0.0;
-      b[rr][cc] = (r < r1 && cj < d) ? static_cast<double>(x[r * d + cj]) - mean[cj] : 0.0;
-    }
-    __syncthreads();
-#pragma unroll 4
-    for (int rr = 0; rr < PCA_T; ++rr) {
-      const double av = a[rr][ty];
+  const int lc = threadIdx.x % T, lr = threadIdx.x / T;  // this thread's staged column and first row
+  const uint64_t ci = static_cast<uint64_t>(ti) * T + lc, cj = static_cast<uint64_t>(tj) * T + lc;
+  const double mi = ci < d ? mean[ci] : 0.0, mj = cj < d ? mean[cj] : 0.0;
+  float fa[LOADS], fb[LOADS];
+  auto load = [&](uint64_t rb) {
 #pragma unroll
-      for (int q = 0; q < 4; ++q) acc[q] = fma(av, b[rr][tx + 8 * q], acc[q]);
+    for (int q = 0; q < LOADS; ++q) {
+      const uint64_t r = rb + lr + q * PASS;
+      fa[q] = r < r1 && ci < d ? x[r * d + ci] : 0.0f;
+      fb[q] = r < r1 && cj < d ? x[r * d + cj] : 0.0f;
     }
+  };
+  auto store = [&](uint64_t rb, int buf) {
+#pragma unroll
+    for (int q = 0; q < LOADS; ++q) {
+      const int rr = lr + q * PASS;
+      a[buf][rr][lc] = rb + rr < r1 && ci < d ? static_cast<double>(fa[q]) - mi : 0.0;
+      b[buf][rr][lc] = rb + rr < r1 && cj < d ? static_cast<double>(fb[q]) - mj : 0.0;
+    }
+  };
+  const int tx = threadIdx.x % E, ty = threadIdx.x / E;
+  double acc[R][R] = {};
+  load(r0);
+  store(r0, 0);
+  __syncthreads();
+  int buf = 0;
+  for (uint64_t rb = r0; rb < r1; rb += S, buf ^= 1) {
+    const bool more = rb + S < r1;
+    if (more) load(rb + S);
+#pragma unroll 8
+    for (int rr = 0; rr < S; ++rr) {
+      double av[R], bv[R];
+#pragma unroll
+      for (int h = 0; h < R / 2; ++h) {
+        const double2 u = *reinterpret_cast<const double2*>(&a[buf][rr][2 * ty + 2 * E * h]);
+        const double2 v = *reinterpret_cast<const double2*>(&b[buf][rr][2 * tx + 2 * E * h]);
+        av[2 * h] = u.x, av[2 * h + 1] = u.y;
+        bv[2 * h] = v.x, bv[2 * h + 1] = v.y;
+      }
+#pragma unroll
+      for (int p = 0; p < R; ++p)
+#pragma unroll
+        for (int q = 0; q < R; ++q) acc[p][q] = fma(av[p], bv[q], acc[p][q]);
+    }
+    if (more) store(rb + S, buf ^ 1);
+    __syncthreads();
   }
-  const uint64_t i = static_cast<uint64_t>(ti) * PCA_T + ty;
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const uint64_t j = static_cast<uint64_t>(tj) * PCA_T + tx + 8 * q;
-    if (i < d && j < d) partial[(chunk * d + i) * d + j] = acc[q];
+  for (int p = 0; p < R; ++p) {
+    const uint64_t i = static_cast<uint64_t>(ti) * T + 2 * ty + (p & 1) + 2 * E * (p >> 1);
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      const uint64_t j = static_cast<uint64_t>(tj) * T + 2 * tx + (q & 1) + 2 * E * (q >> 1);
+      if (i < d && j < d) partial[(chunk * d + i) * d + j] = acc[p][q];
+    }
   }
 }
 
-__global__ void cov_reduce_kernel(const double* __restrict__ partial, uint64_t chunks, uint64_t dd,
+__global__ void cov_reduce_kernel(const double* __restrict__ partial, uint64_t chunks, uint64_t d,
                                   double* __restrict__ cov) {
   const uint64_t e = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (e >= dd) return;
+  if (e >= d * d) return;
+  const uint64_t i = e / d, j = e % d, src = i <= j ? e : j * d + i;
   double s = 0.0;
-  for (uint64_t c = 0; c < chunks; ++c) s += partial[c * dd + e];
+  for (uint64_t c = 0; c < chunks; ++c) s += partial[c * d * d + src];
   cov[e] = s;
 }
 
-// out (n x k, f32) = scale * (x - mean) V for V (d x k, f32, row-major), k <= 128: 64 rows per block,
-// d in slices of 32 staged in shared memory, f64 accumulation.
-constexpr int PJ_ROWS = 64, PJ_D = 32, PJ_K = 128;
+// out (n x k, f32) = scale * (x - mean) V for V (d x k, f32, row-major), k <= 8 NQ: 64 rows per block, thread (tr, tc)
+// rows tr and tr + 32, columns tc + 8 q; d in slices staged in shared memory as f64, f64 accumulation over the columns
+// in order. Bound by the operands' way out of shared memory. 60,000 x 784 -> 100: 1.76 ms when every form was 128
+// columns wide and converted V at each product, 1.09 so.
+constexpr int PJ_ROWS = 64, PJ_K = 104;  // the widest form's columns
+template <int NQ>
 __global__ void __launch_bounds__(256) project_kernel(const float* __restrict__ x, uint64_t n, uint64_t d,
                                                       const double* __restrict__ mean, const float* __restrict__ V,
                                                       int k, float scale, float* __restrict__ out) {
-  __shared__ float xs[PJ_ROWS][PJ_D + 1];
-  __shared__ float vs[PJ_D][PJ_K];
+  constexpr int D = NQ > 8 ? 16 : 32, K = 8 * NQ;
+  __shared__ double xs[PJ_ROWS][D + 1];
+  __shared__ double vs[D][K];
   const uint64_t row0 = static_cast<uint64_t>(blockIdx.x) * PJ_ROWS;
-  // thread t: rows (t / 4) + 64 * 0, columns (t % 4) + 4 q for q < k / 4 (rounded up)
-  const int tr = threadIdx.x >> 2, tc = threadIdx.x & 3;
-  double acc[PJ_K / 4];
-#pragma unroll
-  for (int q = 0; q < PJ_K / 4; ++q) acc[q] = 0.0;
-  for (uint64_t c0 = 0; c0 < d; c0 += PJ_D) {
+  const int tr = threadIdx.x >> 3, tc = threadIdx.x & 7;
+  double acc[2][NQ] = {};
+  for (uint64_t c0 = 0; c0 < d; c0 += D) {
     __syncthreads();
-    for (int e = threadIdx.x; e < PJ_ROWS * PJ_D; e += 256) {
-      const int rr = e / PJ_D, cc = e % PJ_D;
+#pragma unroll
+    for (int e = threadIdx.x; e < PJ_ROWS * D; e += 256) {
+      const int rr = e / D, cc = e % D;
       const uint64_t r = row0 + rr, c = c0 + cc;
-      xs[rr][cc] = (r < n && c < d) ? static_cast<float>(static_cast<double>(x[r * d + c]) - mean[c]) : 0.0f;
+      xs[rr][cc] =
+          (r < n && c < d) ? static_cast<double>(static_cast<float>(static_cast<double>(x[r * d + c]) - mean[c])) : 0.0;
     }
-    for (int e = threadIdx.x; e < PJ_D * PJ_K; e += 256) {
-      const int rr = e / PJ_K, cc = e % PJ_K;
+    for (int e = threadIdx.x; e < D * K; e += 256) {
+      const int rr = e / K, cc = e % K;
       const uint64_t c = c0 + rr;
-      vs[rr][cc] = (c < d && cc < k) ? V[c * k + cc] : 0.0f;
+      vs[rr][cc] = (c < d && cc < k) ? static_cast<double>(V[c * k + cc]) : 0.0;
     }
     __syncthreads();
-    for (int cc = 0; cc < PJ_D; ++cc) {
-      const double xv = xs[tr][cc];
+#pragma unroll 4
+    for (int cc = 0; cc < D; ++cc) {
+      const double x0 = xs[tr][cc], x1 = xs[tr + 32][cc];
 #pragma unroll
-      for (int q = 0; q < PJ_K / 4; ++q) acc[q] = fma(xv, static_cast<double>(vs[cc][tc + 4 * q]), acc[q]);
+      for (int q = 0; q < NQ; ++q) {
+        const double v = vs[cc][tc + 8 * q];
+        acc[0][q] = fma(x0, v, acc[0][q]);
+        acc[1][q] = fma(x1, v, acc[1][q]);
+      }
     }
   }
-  const uint64_t r = row0 + tr;
-  if (r >= n) return;
 #pragma unroll
-  for (int q = 0; q < PJ_K / 4; ++q) {
-    const int c = tc + 4 * q;
-    if (c < k) out[r * k + c] = static_cast<float>(acc[q] * scale);
+  for (int p = 0; p < 2; ++p) {
+    const uint64_t r = row0 + tr + 32 * p;
+    if (r >= n) continue;
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+      const int c = tc + 8 * q;
+      if (c < k) out[r * k + c] = static_cast<float>(acc[p][q] * scale);
+    }
   }
 }
 
@@ -198,6 +258,7 @@ void orthonormalise(std::vector<double>& q, int d, int m) {
 }
 
 constexpr int JACOBI_MAX_D = 160;    // whole-matrix Jacobi up to here, subspace iteration above
+constexpr int SUBSPACE_MAX_K = 128;  // axes the device's form takes (columns in mgs_kernel's shared memory)
 constexpr int SUBSPACE_EXTRA = 24;   // vectors iterated beyond the k wanted
 constexpr int SUBSPACE_ITERS = 20;
 
@@ -294,8 +355,8 @@ std::vector<double> top_axes(std::vector<double>& a, int d, int k) {
 // The subspace iteration on the GPU. Every sum runs over its index in ascending order with separately rounded
 // multiplications and additions, as the host's loops do, so each element is the host's bit for bit: the
 // parallelism is over elements only, and what bounds it is the serial chain of d additions per element.
-// 784 columns, 100 axes: 620-720 ms on a host core, 46 ms here (21 orthonormalisations 32 ms, 22 products 5 ms,
-// the rest the host's Ritz problem and copies); a 60,000 x 784 fit from the default start 759 -> 172 ms.
+// 784 columns, 100 axes: 620-720 ms on a host core; here 21 orthonormalisations of 1.36 ms, 22 products of 35 us,
+// and the host's Ritz problem.
 // ------------------------------------------------------------------------------------------------
 __global__ void subspace_start_kernel(double* __restrict__ q, uint64_t count) {
   const uint64_t e = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -303,42 +364,69 @@ __global__ void subspace_start_kernel(double* __restrict__ q, uint64_t count) {
     q[e] = __dsub_rn(__dmul_rn(static_cast<double>(start_bits(e)), 2.0 / 9007199254740992.0), 1.0);
 }
 
-// out (rows x m) = A (rows x inner) B (inner x m), all row-major: block = AP_ROWS rows x every column (m <= 160,
-// one thread per column), the block's rows of A in shared memory, B's rows read once per block from L2. Four rows a
-// block: 196 blocks for 784 rows (eight rows would leave a third of the SMs without one).
-constexpr int AP_ROWS = 4, AP_COLS = 160;
-__global__ void __launch_bounds__(AP_COLS) block_apply_kernel(const double* __restrict__ A, int rows, int inner,
-                                                              const double* __restrict__ B, int m,
-                                                              double* __restrict__ out) {
-  extern __shared__ double as[];  // [AP_ROWS][inner]
-  const int r0 = blockIdx.x * AP_ROWS, nr = min(AP_ROWS, rows - r0);
-  for (int e = threadIdx.x; e < AP_ROWS * inner; e += AP_COLS)
-    as[e] = e < nr * inner ? A[static_cast<size_t>(r0) * inner + e] : 0.0;
-  __syncthreads();
-  const int j = threadIdx.x;
-  if (j >= m) return;
-  double acc[AP_ROWS] = {};
-#pragma unroll 8
-  for (int l = 0; l < inner; ++l) {
-    const double b = B[static_cast<size_t>(l) * m + j];
+// out (rows x m) = A B for B (inner x m) and A rows x inner, or its transpose (inner x rows) when TRANS; all row-major.
+// 32 x 32 outputs a block, 2 x 2 a thread, slabs of 32 inner indices in two shared-memory buffers with the next slab's
+// values in registers meanwhile. 784 x 784 times 784 x 124 (100 blocks): 229 us when each thread read B's rows from
+// L2 one after another, 35 so; q^T (A q) of that size 119 -> 33 us.
+constexpr int AP_T = 32;
+template <bool TRANS>
+__global__ void __launch_bounds__(256) block_apply_kernel(const double* __restrict__ A, int rows, int inner,
+                                                          const double* __restrict__ B, int m,
+                                                          double* __restrict__ out) {
+  __shared__ __align__(16) double as[2][AP_T][AP_T + 2], bs[2][AP_T][AP_T];  // [buffer][inner][row or column]
+  const int r0 = blockIdx.x * AP_T, j0 = blockIdx.y * AP_T;
+  const int lo = threadIdx.x & 31, hi = threadIdx.x >> 5;  // staging: 8 values of 32 per pass
+  double fa[4], fb[4];
+  auto load = [&](int l0) {
 #pragma unroll
-    for (int r = 0; r < AP_ROWS; ++r) acc[r] = __dadd_rn(acc[r], __dmul_rn(as[r * inner + l], b));
+    for (int q = 0; q < 4; ++q) {
+      const int h = hi + 8 * q;
+      if (TRANS) fa[q] = l0 + h < inner && r0 + lo < rows ? A[static_cast<size_t>(l0 + h) * rows + r0 + lo] : 0.0;
+      else fa[q] = r0 + h < rows && l0 + lo < inner ? A[static_cast<size_t>(r0 + h) * inner + l0 + lo] : 0.0;
+      fb[q] = l0 + h < inner && j0 + lo < m ? B[static_cast<size_t>(l0 + h) * m + j0 + lo] : 0.0;
+    }
+  };
+  auto store = [&](int buf) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int h = hi + 8 * q;
+      as[buf][TRANS ? h : lo][TRANS ? lo : h] = fa[q];
+      bs[buf][h][lo] = fb[q];
+    }
+  };
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  double acc[2][2] = {};
+  load(0);
+  store(0);
+  __syncthreads();
+  int buf = 0;
+  for (int l0 = 0; l0 < inner; l0 += AP_T, buf ^= 1) {
+    const bool more = l0 + AP_T < inner;
+    if (more) load(l0 + AP_T);
+    auto term = [&](int l) {
+      const double2 u = *reinterpret_cast<const double2*>(&as[buf][l][2 * ty]);
+      const double2 v = *reinterpret_cast<const double2*>(&bs[buf][l][2 * tx]);
+      acc[0][0] = __dadd_rn(acc[0][0], __dmul_rn(u.x, v.x));
+      acc[0][1] = __dadd_rn(acc[0][1], __dmul_rn(u.x, v.y));
+      acc[1][0] = __dadd_rn(acc[1][0], __dmul_rn(u.y, v.x));
+      acc[1][1] = __dadd_rn(acc[1][1], __dmul_rn(u.y, v.y));
+    };
+    if (l0 + AP_T <= inner) {
+#pragma unroll 16
+      for (int l = 0; l < AP_T; ++l) term(l);
+    } else {
+      for (int l = 0; l < inner - l0; ++l) term(l);
+    }
+    if (more) store(buf ^ 1);
+    __syncthreads();
   }
 #pragma unroll
-  for (int r = 0; r < AP_ROWS; ++r)
-    if (r < nr) out[static_cast<size_t>(r0 + r) * m + j] = acc[r];
-}
-
-// proj (m x m) = q^T aq over the d rows in order; one thread per element.
-__global__ void ritz_project_kernel(const double* __restrict__ q, const double* __restrict__ aq, int d, int m,
-                                    double* __restrict__ proj) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y;
-  if (j >= m) return;
-  double s = 0.0;
-#pragma unroll 8
-  for (int r = 0; r < d; ++r)
-    s = __dadd_rn(s, __dmul_rn(q[static_cast<size_t>(r) * m + i], aq[static_cast<size_t>(r) * m + j]));
-  proj[static_cast<size_t>(i) * m + j] = s;
+  for (int p = 0; p < 2; ++p)
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int r = r0 + 2 * ty + p, j = j0 + 2 * tx + q;
+      if (r < rows && j < m) out[static_cast<size_t>(r) * m + j] = acc[p][q];
+    }
 }
 
 // Modified Gram-Schmidt of the columns of a d x m matrix (row-major in and out; in == out allowed) by one cluster of
@@ -346,19 +434,35 @@ __global__ void ritz_project_kernel(const double* __restrict__ q, const double* 
 // copies it over distributed shared memory, and takes its part out of the later columns it owns. For each column
 // the projections onto the earlier ones are removed in ascending order, as in the host's column-by-column loop.
 // Bound by two serial chains of d additions per column (the norm, then the dot products: those of a block's columns
-// run side by side in the lanes of one warp): 12 us per column of 784 rows, about 14 cycles an addition; forming
-// the next products ahead of the additions did not change it. The columns lie an odd number of doubles apart, so
+// run side by side in the lanes of one warp), 8.3 cycles an addition: 7 of the 11 us per column of 784 rows. With the
+// products formed 16 rows ahead of the additions 1.36 ms for 124 columns, with the loop only unrolled (8) 1.83. The columns lie an odd number of doubles apart, so
 // that the lanes' reads fall in different banks. At most 152 columns of 1024 rows: 19 columns per block, 164 KB.
-constexpr int MGS_BLOCKS = 8, MGS_THREADS = 512;
+constexpr int MGS_BLOCKS = 8, MGS_THREADS = 512, CHAIN_AHEAD = 16;
 __host__ __device__ __forceinline__ int mgs_ld(int d) { return d | 1; }
 size_t mgs_smem(int d, int m) {
   return (static_cast<size_t>((m + MGS_BLOCKS - 1) / MGS_BLOCKS) * mgs_ld(d) + d) * sizeof(double);
 }
 
+// The products of the next CHAIN_AHEAD rows are formed while this batch's are added up.
 __device__ __forceinline__ double chain_dot(const double* a, const double* b, int d) {
-  double s = 0.0;
-#pragma unroll 8
-  for (int r = 0; r < d; ++r) s = __dadd_rn(s, __dmul_rn(a[r], b[r]));
+  double s = 0.0, p[CHAIN_AHEAD];
+  int r = 0;
+  if (d >= CHAIN_AHEAD) {
+#pragma unroll
+    for (int q = 0; q < CHAIN_AHEAD; ++q) p[q] = __dmul_rn(a[q], b[q]);
+    for (r = CHAIN_AHEAD; r + CHAIN_AHEAD <= d; r += CHAIN_AHEAD) {
+      double t[CHAIN_AHEAD];
+#pragma unroll
+      for (int q = 0; q < CHAIN_AHEAD; ++q) t[q] = __dmul_rn(a[r + q], b[r + q]);
+#pragma unroll
+      for (int q = 0; q < CHAIN_AHEAD; ++q) s = __dadd_rn(s, p[q]);
+#pragma unroll
+      for (int q = 0; q < CHAIN_AHEAD; ++q) p[q] = t[q];
+    }
+#pragma unroll
+    for (int q = 0; q < CHAIN_AHEAD; ++q) s = __dadd_rn(s, p[q]);
+  }
+  for (; r < d; ++r) s = __dadd_rn(s, __dmul_rn(a[r], b[r]));
   return s;
 }
 
@@ -410,8 +514,7 @@ __global__ void __cluster_dims__(MGS_BLOCKS, 1, 1) __launch_bounds__(MGS_THREADS
 // diagonal by then) stays on the host.
 std::vector<double> top_axes_device(Ctx& c, const double* d_cov, int d, int k) {
   const int m = std::min(d, k + SUBSPACE_EXTRA);
-  PM_REQUIRE(m <= AP_COLS && (m + MGS_BLOCKS - 1) / MGS_BLOCKS <= 32, PACMAP_ERR_UNSUPPORTED,
-             "PCA supports at most 128 components");
+  PM_REQUIRE(k <= SUBSPACE_MAX_K, PACMAP_ERR_UNSUPPORTED, "PCA supports at most 128 components");
   const uint64_t dm = static_cast<uint64_t>(d) * m;
   DevBuf<double> q(c, dm), t(c, dm), proj(c, static_cast<uint64_t>(m) * m), z(c, static_cast<uint64_t>(m) * m);
   const size_t ms = mgs_smem(d, m);
@@ -421,8 +524,7 @@ std::vector<double> top_axes_device(Ctx& c, const double* d_cov, int d, int k) {
     PM_LAUNCHED();
   };
   auto apply = [&](const double* A, int inner, const double* B, double* out) {
-    block_apply_kernel<<<(d + AP_ROWS - 1) / AP_ROWS, AP_COLS, static_cast<size_t>(AP_ROWS) * inner * sizeof(double),
-                         c.stream>>>(A, d, inner, B, m, out);
+    block_apply_kernel<false><<<dim3(ceil_div(d, AP_T), ceil_div(m, AP_T)), 256, 0, c.stream>>>(A, d, inner, B, m, out);
     PM_LAUNCHED();
   };
   subspace_start_kernel<<<ceil_div(dm, 256), 256, 0, c.stream>>>(q.get(), dm);
@@ -433,7 +535,9 @@ std::vector<double> top_axes_device(Ctx& c, const double* d_cov, int d, int k) {
     mgs(t.get(), q.get());
   }
   apply(d_cov, d, q.get(), t.get());
-  ritz_project_kernel<<<dim3(ceil_div(m, 64), m), 64, 0, c.stream>>>(q.get(), t.get(), d, m, proj.get());
+  // q^T (A q)
+  block_apply_kernel<true><<<dim3(ceil_div(m, AP_T), ceil_div(m, AP_T)), 256, 0, c.stream>>>(q.get(), m, d, t.get(), m,
+                                                                                           proj.get());
   PM_LAUNCHED();
   std::vector<double> hp(proj.count), w, hz, vecs(dm);
   PM_CUDA(cudaMemcpyAsync(hp.data(), proj.get(), proj.bytes(), cudaMemcpyDeviceToHost, c.stream));
@@ -667,7 +771,7 @@ void pca_top_axes(const double* cov, uint64_t d, uint64_t k, double* axes) {
 }
 
 void pca_top_axes_device(Ctx& c, const double* cov, uint64_t d, uint64_t k, double* axes) {
-  PM_REQUIRE(k >= 1 && k <= static_cast<uint64_t>(PJ_K) && k <= d && d <= 1024 &&
+  PM_REQUIRE(k >= 1 && k <= static_cast<uint64_t>(SUBSPACE_MAX_K) && k <= d && d <= 1024 &&
                  d > static_cast<uint64_t>(JACOBI_MAX_D),
              PACMAP_ERR_UNSUPPORTED, "axes on the device need 1 <= k <= 128 and 160 < d <= 1024");
   DevBuf<double> dc;
@@ -697,7 +801,7 @@ void pca_project_device(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint64
                         std::vector<float>* axes_out) {
   PM_REQUIRE(n > 0, PACMAP_ERR_EMPTY_ARRAY_MEAN, "Failed to calculate mean axis: the array is empty");
   PM_REQUIRE(k >= 1 && k <= static_cast<uint64_t>(PJ_K) && k <= d, PACMAP_ERR_UNSUPPORTED,
-             "PCA supports at most 128 components and no more than the columns");
+             "PCA supports at most 104 components and no more than the columns");
   PM_REQUIRE(d <= 1024, PACMAP_ERR_UNSUPPORTED, "PCA supports d <= 1024");
   // 1. means
   DevBuf<double> mpart(c, static_cast<uint64_t>(MEAN_BLOCKS) * d), mean(c, d);
@@ -707,12 +811,20 @@ void pca_project_device(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint64
   PM_LAUNCHED();
   // 2. covariance (unnormalised: the axes do not depend on the scale)
   const uint64_t rpc = std::max<uint64_t>(16384, (n + PCA_MAX_CHUNKS - 1) / PCA_MAX_CHUNKS);
-  const uint64_t chunks = (n + rpc - 1) / rpc, tiles = (d + PCA_T - 1) / PCA_T;
+  const uint64_t chunks = (n + rpc - 1) / rpc;
+  auto pairs = [&](uint64_t tile) { return (d + tile - 1) / tile * ((d + tile - 1) / tile + 1) / 2; };
   DevBuf<double> part(c, chunks * d * d), cov(c, d * d);
-  cov_partial_kernel<<<dim3(static_cast<unsigned>(tiles), static_cast<unsigned>(tiles), static_cast<unsigned>(chunks)),
-                       256, 0, c.stream>>>(d_x, n, d, rpc, mean.get(), part.get());
-  PM_LAUNCHED();
-  cov_reduce_kernel<<<ceil_div(d * d, 256), 256, 0, c.stream>>>(part.get(), chunks, d * d, cov.get());
+  auto partials = [&](auto kernel, uint64_t tile, int threads) {
+    kernel<<<dim3(static_cast<unsigned>(pairs(tile)), static_cast<unsigned>(chunks)), threads, 0, c.stream>>>(
+        d_x, n, d, rpc, mean.get(), part.get());
+    PM_LAUNCHED();
+  };
+  // 64-column tiles once they give every SM a block, else 16-column ones: 2.9 against 4.1 ms at 60,000 x 784 (364
+  // blocks of the wide tiles), 2.0 / 2.2 at 30,000 x 784 (182), 2.25 / 2.29 at 1,000,000 x 128 (186), 0.88 / 1.31 the
+  // other way at 60,000 x 300 (60), 0.058 / 0.164 at 2,000 x 100 (3), equal at 16,000 x 784 (91)
+  if (pairs(64) * chunks >= static_cast<uint64_t>(c.sm_count)) partials(cov_partial_kernel<4, 16>, 64, 256);
+  else partials(cov_partial_kernel<2, 8>, 16, 64);
+  cov_reduce_kernel<<<ceil_div(d * d, 256), 256, 0, c.stream>>>(part.get(), chunks, d, cov.get());
   PM_LAUNCHED();
   // 3. axes
   std::vector<double> V64;
@@ -733,8 +845,16 @@ void pca_project_device(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint64
   // 4. projection
   DevBuf<float> dV;
   upload(c, dV, V.data(), d * k);
-  project_kernel<<<ceil_div(n, PJ_ROWS), 256, 0, c.stream>>>(d_x, n, d, mean.get(), dV.get(), static_cast<int>(k),
-                                                            scale, d_out);
+  auto project = [&](auto kernel) {
+    kernel<<<ceil_div(n, PJ_ROWS), 256, 0, c.stream>>>(d_x, n, d, mean.get(), dV.get(), static_cast<int>(k), scale,
+                                                       d_out);
+  };
+  // The narrowest form that holds the k columns, since the padding is computed too; 13: the 100 axes of the wide
+  // data's reduction. 60,000 x 784: 0.28 ms for 2 columns, 1.09 for 100.
+  if (k <= 8) project(project_kernel<1>);
+  else if (k <= 32) project(project_kernel<4>);
+  else if (k <= 64) project(project_kernel<8>);
+  else project(project_kernel<13>);
   PM_LAUNCHED();
 }
 
