@@ -434,9 +434,10 @@ __global__ void __launch_bounds__(256) block_apply_kernel(const double* __restri
 // copies it over distributed shared memory, and takes its part out of the later columns it owns. For each column
 // the projections onto the earlier ones are removed in ascending order, as in the host's column-by-column loop.
 // Bound by two serial chains of d additions per column (the norm, then the dot products: those of a block's columns
-// run side by side in the lanes of one warp), 8.3 cycles an addition: 7 of the 11 us per column of 784 rows. With the
-// products formed 16 rows ahead of the additions 1.36 ms for 124 columns, with the loop only unrolled (8) 1.83. The columns lie an odd number of doubles apart, so
-// that the lanes' reads fall in different banks. At most 152 columns of 1024 rows: 19 columns per block, 164 KB.
+// run side by side in the lanes of one warp): 10 of the 11 us per column of 784 rows, 11.8 cycles an addition where its
+// latency alone is 8.3. 124 columns: 1.36 ms with the products formed 16 rows ahead of the additions, 1.83 with the
+// loop only unrolled (8). The columns lie an odd number of doubles apart, so that the lanes' reads fall in different
+// banks. At most 152 columns of 1024 rows: 19 columns per block, 164 KB.
 constexpr int MGS_BLOCKS = 8, MGS_THREADS = 512, CHAIN_AHEAD = 16;
 __host__ __device__ __forceinline__ int mgs_ld(int d) { return d | 1; }
 size_t mgs_smem(int d, int m) {
@@ -557,14 +558,16 @@ std::vector<double> top_axes_device(Ctx& c, const double* d_cov, int d, int k) {
 // the rotation, then a thread per two pairs turns their 2 x 2 block of the matrix. The rotations go to rot; the
 // wanted eigenvectors are unit vectors taken back through them, so that the full eigenvector matrix is never formed.
 // out: status (1: converged and the leading k + 1 eigenvalues lie JACOBI_GAP of the largest apart), the k leading
-// eigenvalues, the eigenvectors (d x k, row-major). Bound by each step's serial chain: two divisions, a square root
-// and a reciprocal square root in f64, then the block's products, with a barrier after either (1.2 us a step, 890
-// steps at d = 100). A 2,000 x 100 fit from the principal axes: 12.1 ms with the host's sweeps, 4.4 ms so.
+// eigenvalues, the eigenvectors (d x k, row-major). Bound by the blocks' way through shared memory (1,490 of a step's
+// 2,130 cycles at d = 100, 8 sweeps) and by the rotation's two reciprocal square roots and their chain (640; 850 with
+// the tangent from two divisions and two roots). Vectors: 240 cycles a step with a barrier for their warps only, 430
+// with the whole block's. Finding the next step's rotations beside the blocks (one barrier a step) was no faster. A
+// 2,000 x 100 fit from the principal axes: 12.1 ms with the host's sweeps, 4.1 ms so.
 constexpr int JACOBI_THREADS = 1024, JACOBI_MAX_K = 8, JACOBI_SWEEPS = 20, JACOBI_AHEAD = 8;
 constexpr int JACOBI_BLOCKS = ((JACOBI_MAX_D / 2) * (JACOBI_MAX_D / 2 - 1) / 2 + JACOBI_THREADS - 1) / JACOBI_THREADS;
-// The device from 32 columns on: 216 us against the host's 255 at 32 (copies in and out included), 162 against 123
-// at 24, 1.12 ms against 6.9 at 100, 3.0 against 63 at 160. Its residuals are the smaller (2e-15 of the largest
-// eigenvalue against 1e-14 at 100), and the f32 axes of 120 covariances of both kinds came out the same.
+// The device from 32 columns on: 173 us against the host's 259 at 32 (copies in and out included), 135 against 127
+// at 24, 0.97 ms against 7.2 at 100, 2.7 against 64 at 160. Its residuals are the smaller (7e-15 of the largest
+// eigenvalue against 1.2e-14 at 100), and the f32 axes of 120 covariances of both kinds came out the same.
 // JACOBI_GAP: axes whose eigenvalues lie closer than this (of the largest) depend on the order of the rotations in
 // digits that f32 keeps, and equal eigenvalues leave the choice of basis to it, so the host's cyclic order stays
 // for those; above it the two methods' axes differ by about 1e-12, far below f32. Eight axes: the start's dim; the
@@ -642,24 +645,26 @@ __global__ void __launch_bounds__(JACOBI_THREADS)
       if (i < j) off += a[i * ld + j] * a[i * ld + j];
     }
     off = block_sum(off);
-    done = off <= 1e-30 * total;  // false for NaN
+    done = off <= 1e-30 * total && total <= 1e300;  // false for NaN
     if (done || sweep == JACOBI_SWEEPS) break;
     for (int s = 0; s < m; ++s) {
       if (tid < h) {
         int p, q;
         jacobi_pair(tid, s, m, p, q);
         double& apq = at(p, q);
-        double c = 1.0, t = 0.0;
-        if (fabs(apq) >= 1e-300) {
-          double &app = a[p * ld + p], &aqq = a[q * ld + q];
-          const double theta = (aqq - app) / (2.0 * apq);
-          t = (theta >= 0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
-          c = rsqrt(t * t + 1.0);
-          app -= t * apq;
-          aqq += t * apq;
+        // tan 2 theta = b / delta with |theta| <= pi / 4: cos^2 = (1 + |delta| / r) / 2, sin = b / (2 r cos)
+        double2 r = make_double2(1.0, 0.0);
+        double &app = a[p * ld + p], &aqq = a[q * ld + q];
+        const double delta = aqq - app, b = 2.0 * apq, r2 = delta * delta + b * b;
+        if (fabs(apq) >= 1e-300 && r2 >= 1e-280 && r2 <= 1e280) {
+          const double ir = rsqrt(r2), c2 = 0.5 + 0.5 * fabs(delta) * ir, ic = rsqrt(c2);
+          r = make_double2(c2 * ic, (delta >= 0 ? 0.5 : -0.5) * b * ir * ic);
+          const double shift = r.y * ic * apq;
+          app -= shift;
+          aqq += shift;
           apq = 0.0;
         }
-        cs[tid] = make_double2(c, t * c);
+        cs[tid] = r;
         rot[(static_cast<size_t>(sweep) * m + s) * h + tid] = cs[tid];
       }
       __syncthreads();
@@ -708,25 +713,31 @@ __global__ void __launch_bounds__(JACOBI_THREADS)
   __syncthreads();
   for (int e = tid; e < k * n; e += JACOBI_THREADS) a[e] = e % n == order[e / n] ? 1.0 : 0.0;
   __syncthreads();
-  for (int step = sweep * m - 1; step >= 0;) {
-    const int batch = min(JACOBI_AHEAD, step + 1);
-    double2 r[JACOBI_AHEAD];
+  const int threads = (k * h + 31) / 32 * 32;  // whole warps, with a barrier of their own
+  if (tid < threads) {
+    int s = m - 1;
+    for (int step = sweep * m - 1; step >= 0;) {
+      const int batch = min(JACOBI_AHEAD, step + 1);
+      double2 r[JACOBI_AHEAD];
 #pragma unroll
-    for (int b = 0; b < JACOBI_AHEAD; ++b)
-      if (b < batch && v < k) r[b] = rot[static_cast<size_t>(step - b) * h + i];
+      for (int b = 0; b < JACOBI_AHEAD; ++b)
+        if (b < batch && v < k) r[b] = rot[static_cast<size_t>(step - b) * h + i];
 #pragma unroll
-    for (int b = 0; b < JACOBI_AHEAD; ++b) {
-      if (b < batch && v < k) {
-        int p, q;
-        jacobi_pair(i, (step - b) % m, m, p, q);
-        const double xp = a[v * n + p], xq = a[v * n + q];
-        a[v * n + p] = r[b].x * xp + r[b].y * xq;
-        a[v * n + q] = r[b].x * xq - r[b].y * xp;
+      for (int b = 0; b < JACOBI_AHEAD; ++b) {
+        if (b < batch && v < k) {
+          int p, q;
+          jacobi_pair(i, s, m, p, q);
+          const double xp = a[v * n + p], xq = a[v * n + q];
+          a[v * n + p] = r[b].x * xp + r[b].y * xq;
+          a[v * n + q] = r[b].x * xq - r[b].y * xp;
+        }
+        if (b < batch) s = s ? s - 1 : m - 1;
+        asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
       }
-      __syncthreads();
+      step -= batch;
     }
-    step -= batch;
   }
+  __syncthreads();
   for (int e = tid; e < d * k; e += JACOBI_THREADS) out[1 + k + e] = a[(e % k) * n + e / k];
 }
 
