@@ -55,9 +55,10 @@ MEASURED_PEAKS = os.path.join(ROOT, "MEASURED_PEAKS.json")
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per launch of the dominant kernels at the
 # 1,000,000 x 128 workload, from one-pass captures (ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum
 # -k regex:<kernel> -s <launches to skip> on `bench.py --minimal --steps 1 --warmup 1`): the filter's main
-# pass (the launch its roofline times; the bound pass moves 16.9 GB, mostly candidate writes), and the
-# gradient's average over the (0, 50, 150) schedule (1.182 GB per phase-2 launch, 1.143 GB per phase-3).
-TRAFFIC = {"knn_filter_kernel": 5133694464, "grad_adam_kernel": 1152481088}
+# pass (the launch its roofline times; the bound pass moves 16.6 GB, mostly candidate writes), and the
+# gradient's average over the (0, 50, 150) schedule (its two kernels together 2.437 GB per phase-2
+# iteration, 2.138 GB per phase-3: the rows' sums per tile are written and read back).
+TRAFFIC = {"knn_filter_kernel": 4941928192, "tile_gradient": 2212485696}
 
 
 def _peaks():
@@ -468,22 +469,25 @@ def run_ours(args, rank, world, local_rank):
     iters = sum(learned.SHORT_SCHEDULE)
     opt_bytes = _optimize_bytes(n, dim, learned.SHORT_SCHEDULE)
     opt_gbs = opt_bytes / (opt_ms * 1e-3) / 1e9 if opt_ms > 0 else None
-    roof_opt = {"kernel": "grad_adam_kernel (CSR gradient + Adam, one launch per iteration in a CUDA graph)",
+    roof_opt = {"kernel": ("tile_force_kernel + tile_adam_kernel (gradient from shared-memory tiles + Adam; grad_adam_kernel "
+                           "where a row has under 4 partners per tile), once per iteration in a CUDA graph"),
                 "bound": "hbm", "achieved": round(opt_gbs, 1) if opt_gbs else None, "peak": hbm, "unit": "GB/s",
-                "frac": round(opt_gbs / hbm, 4) if opt_gbs else None, "traffic": traffic.get("grad_adam_kernel"),
+                "frac": round(opt_gbs / hbm, 4) if opt_gbs else None, "traffic": traffic.get("tile_gradient"),
                 "algorithmic": ("8 B per active pair + 28*n*dim B per iteration (k, n_mn, n_fp = %d, %d, %d; mid-near "
                                 "pairs inactive in phase 3)" % _pair_counts(n)),
                 "launch_ms": round(opt_ms / iters, 4) if opt_ms else None,
                 "peak_source": f"{src} HBM copy"}
-    # what binds it: the random partner gathers, against this device's measured rate of random 8-byte loads
-    # from an L2-resident array (pacmap_gather_rate)
+    # the partner reads against this device's measured rate of random 8-byte loads from an L2-resident array
+    # (pacmap_gather_rate): a ceiling for gathers from L2, not for the near and far partners that come from
+    # shared-memory tiles
     rate = pm.gather_rate(local_rank)
     gathers = _optimize_gathers(n, learned.SHORT_SCHEDULE)
     g_rate = gathers / (opt_ms * 1e-3) if opt_ms > 0 else None
     roof_opt["gather_roofline"] = {
         "achieved": round(g_rate / 1e9, 1) if g_rate else None, "peak": round(rate / 1e9, 1), "unit": "G loads/s",
         "frac": round(g_rate / rate, 4) if g_rate and rate else None,
-        "algorithmic": "2 (k + n_fp) partner loads per point per iteration, 2 (k + n_mn + n_fp) in phases 1-2",
+        "algorithmic": ("2 (k + n_fp) partner loads per point per iteration, 2 (k + n_mn + n_fp) in phases 1-2; near and "
+                        "far ones from shared memory where the gradient is tiled"),
         "peak_source": "measured: random 8-byte loads from an L2-resident 8 MB array (pacmap_gather_rate)"}
     # the headline roofline is the kernel that takes the larger share of the learned step
     dominant_opt = opt_ms >= knn_ms

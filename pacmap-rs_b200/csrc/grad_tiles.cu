@@ -8,8 +8,9 @@
 //                      (neighbour and far pairs), a lane per row, writing the row's sum over the tile's partners;
 //   tile_adam_kernel   eight lanes per row add the row's tile sums in a fixed order, gather its mid-near partners as
 //                      grad_adam_kernel does (they are few, and none in the last phase), and take the Adam step.
-// The regrouped lists are built once per fit (build_tile_grad): rows in windows of 128, within each (tile, window) sorted
-// by their number of entries so that the 32 rows of a unit are about equally long, each row's entries in CSR order.
+// The regrouped lists are built once per fit (build_tile_grad): rows in windows of 128, within each (tile, window)
+// sorted by their number of entries so that the 32 rows of a unit are about equally long, each row's entries in CSR
+// order.
 // No atomics on floats: the sums and their order are the same on every call (another order than grad_adam_kernel's).
 #include <algorithm>
 
@@ -27,12 +28,12 @@ constexpr int MAX_TILES = 64;
 constexpr uint32_t ROW_MAX = 511;    // entries of a row: 9 bits in meta; longer rows get a warp each
 constexpr int TILE_SMEM = 232448;
 
-// The rule of build_tile_grad. From 65,536 rows on the tiled iteration wins by more than 10 us: at 60,000 rows in 2-D it
-// takes 30 us (3-D 40) against 42 (63) for grad_adam_kernel's order, which smaller fits keep to the bit; at 100,000
-// 47 (63) against 75 (112), at 200,000 86 (127) against 163 (236), at 400,000 189 (306) against 340 (510), at 1,000,000
-// 776 (1307) against 957 (1447): the fewer entries a row has in a tile, the more of a unit's time is its fixed cost. Below 4
-// (4,000,000 rows in 3-D have 1.6) it would lose. Building the lists takes 0.3 ms at 100,000 rows and 4 at 1,000,000, as
-// much as 8 to 25 iterations win back, 40 below 6 entries.
+// The rule of build_tile_grad. From 65,536 rows on the tiled iteration wins by more than 10 us: at 60,000 rows in 2-D
+// it takes 30 us (3-D 40) against 42 (63) for grad_adam_kernel's order, which smaller fits keep to the bit; at 100,000
+// 47 (63) against 75 (112), at 200,000 86 (127) against 163 (236), at 400,000 189 (306) against 340 (510), at
+// 1,000,000 776 (1307) against 957 (1447): the fewer entries a row has in a tile, the more of a unit's time is its
+// fixed cost. Below 4 (4,000,000 rows in 3-D have 1.6) it would lose. Building the lists takes 0.3 ms at 100,000 rows
+// and 4 at 1,000,000, as much as 8 to 25 iterations win back, 40 below 6 entries.
 constexpr uint64_t TILE_MIN_ROWS = 65536;
 constexpr double TILE_MIN_ENTRIES = 4.0;
 uint64_t tile_min_iters(double entries) { return entries >= 16.0 ? 12 : (entries >= 6.0 ? 32 : 64); }
@@ -178,8 +179,8 @@ template <int DIM>
 constexpr float NOWHERE = DIM == 2 ? 2.5e9f : 2.1e9f;
 
 // One entry of a row (gradient.rs:120-147): the partner's y from shared memory, its term added to acc. The per-pair
-// factor is w c2 / t^2 with t = c1 + 1 + |dy|^2; near pairs have w c2 = 20 w_nn and c1 = 10, far ones (bit 15 of e) repel:
-// -2 w_fp and 1. Multiplications and additions are fused here, which rounds less often than the separate ones.
+// factor is w c2 / t^2 with t = c1 + 1 + |dy|^2; near pairs have w c2 = 20 w_nn and c1 = 10, far ones (bit 15 of e)
+// repel: -2 w_fp and 1. Multiplications and additions are fused here, which rounds less often than the separate ones.
 template <int DIM>
 __device__ __forceinline__ void add_entry(const float* ys, uint32_t e, bool far, const float (&yi)[DIM],
                                           float near_num, float far_num, float (&acc)[DIM]) {
@@ -218,9 +219,10 @@ struct ForceArgs {
   const Sched* sched;
 };
 
-// A unit: 32 rows of one window, a lane each, over their partners in one tile. Bound by the instructions per entry (about 25,
-// a two-wide form of the arithmetic was slower: its operands cost two more shared loads and the packing) and per unit,
-// and by the latency of the list words, which are two units ahead. 200,000 rows in 2-D: 72 us for 36 million entries.
+// A unit: 32 rows of one window, a lane each, over their partners in one tile. Bound by the instructions per entry
+// (about 25; a two-wide form of the arithmetic was slower: its operands cost two more shared loads and the packing) and
+// per unit, and by the latency of the list words, which are two units ahead. 200,000 rows in 2-D: 72 us for 36 million
+// entries.
 template <int DIM>
 __global__ void __launch_bounds__(FORCE_T, 1) tile_force_kernel(const ForceArgs p, int itr) {
   extern __shared__ __align__(16) float ys[];
@@ -320,8 +322,8 @@ __global__ void __launch_bounds__(FORCE_T, 1) tile_force_kernel(const ForceArgs 
   }
 }
 
-// A row's tile sums (lane gl of eight adds tiles gl, gl + 8, ... in order), its mid-near pairs, the lanes' sums pairwise,
-// and the Adam step.
+// A row's tile sums (lane gl of eight adds tiles gl, gl + 8, ... in order), its mid-near pairs, the lanes' sums
+// pairwise, and the Adam step.
 template <int DIM>
 __global__ void __launch_bounds__(256) tile_adam_kernel(const GradArgs p, const float* __restrict__ partial,
                                                         uint32_t tiles, int itr) {
@@ -395,7 +397,8 @@ bool build_tile_grad(Ctx& c, const Csr& csr, uint64_t n, uint64_t dim, uint64_t 
   PM_CUDA(cudaMemsetAsync(words.get() + units, 0, sizeof(uint32_t), c.stream));
   out.meta.alloc(c, units * 32);
   out.unit_off.alloc(c, units + 1);
-  const size_t smem_count = static_cast<size_t>(tiles) * WIN * 2, smem_fill = smem_count + static_cast<size_t>(tiles) * WIN;
+  const size_t smem_count = static_cast<size_t>(tiles) * WIN * 2;
+  const size_t smem_fill = smem_count + static_cast<size_t>(tiles) * WIN;
   tile_count_kernel<<<out.windows, BUILD_T, smem_count, c.stream>>>(csr.row_ptr.get(), csr.col.get(), n, out.tiles,
                                                                     out.tile_pts, magic, out.windows, out.meta.get(),
                                                                     words.get());

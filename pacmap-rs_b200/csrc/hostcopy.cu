@@ -1,11 +1,11 @@
 // Copies between a caller's ordinary (pageable) host memory and the device.
 //
-// The driver moves pageable memory through its own staging buffers on the calling thread, and an output's pages are first
-// touched there, one by one: 64 MB take it 4.7 ms up and 13.6 down, where the link needs 1.2. Larger copies are cut into
-// one range per worker: each worker moves its range piece by piece through two page-locked slots of its own, copying
-// one piece on a core while the other is on the link (64 MB: 3.0 and 3.1 ms). The threads live for one copy; the slots
-// (32 MB) stay with the device until the library is unloaded. Calls on a device hold its lock, so one copy uses them at a
-// time. Memory that the caller page-locked goes to the link directly.
+// The driver moves pageable memory through its own staging buffers on the calling thread, and an output's pages are
+// first touched there, one by one: 64 MB take it 4.7 ms up and 13.6 down, where the link needs 1.2. Larger copies are
+// cut into one range per worker: each worker moves its range piece by piece through two page-locked slots of its own,
+// copying one piece on a core while the other is on the link (64 MB: 3.0 and 3.1 ms). The threads live for one copy;
+// the slots (32 MB) stay with the device until the library is unloaded. Calls on a device hold its lock, so one copy
+// uses them at a time. Memory that the caller page-locked goes to the link directly.
 #include <algorithm>
 #include <cstring>
 #include <system_error>
@@ -18,8 +18,9 @@ namespace {
 
 constexpr int COPY_WORKERS = 8;
 constexpr size_t COPY_SLOT = 2u << 20;
-// Downloads are staged from 1 MB (0.11 against 0.23 ms; 4 MB 0.45 against 0.63), uploads from 32 MB (1.6 against 1.9; at
-// 16 MB the two are equal). A worker is worth starting for 8 MB: smaller shares made 4 MB downloads 0.7 to 1.2 ms.
+// Downloads are staged from 1 MB (0.11 against 0.23 ms; 4 MB 0.45 against 0.63), uploads from 32 MB (1.6 against 1.9;
+// at 16 MB the two are equal). A worker is worth starting for 8 MB: smaller shares made 4 MB downloads 0.7 to 1.2 ms.
+// 12 and 16 workers moved 256 MB up in 9.0 and 9.3 ms, 8 in 8.4.
 constexpr size_t DOWN_MIN = 1u << 20, UP_MIN = 32u << 20, COPY_SHARE = 8u << 20;
 
 }  // namespace
@@ -88,7 +89,8 @@ void copy_host(Ctx& c, void* dst, const void* src, size_t bytes, bool to_device)
   if (!bytes) return;
   const cudaMemcpyKind kind = to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
   cudaPointerAttributes at{};
-  const bool pageable = bytes >= (to_device ? UP_MIN : DOWN_MIN) && cudaPointerGetAttributes(&at, to_device ? src : dst) == cudaSuccess &&
+  const bool pageable = bytes >= (to_device ? UP_MIN : DOWN_MIN) &&
+                        cudaPointerGetAttributes(&at, to_device ? src : dst) == cudaSuccess &&
                         at.type == cudaMemoryTypeUnregistered;
   if (!pageable) {
     PM_CUDA(cudaMemcpyAsync(dst, src, bytes, kind, c.stream));

@@ -9,9 +9,10 @@
 //   * knn_simt_kernel: every distance in the reference's exact f32 order (distance.rs:50-75) on CUDA
 //     cores, each block keeping the running k' best (distance key, index) of 32 query rows in shared
 //     memory. Used for small n, for any d, and for rows the tensor-core filter (knn_tc.cu) cannot settle,
-//     against all rows or (LIST) against the columns that its second run left for the 32 rows. When there are too few query rows to fill the GPU, the keys are split
-//     into slices (grid y); each slice writes its own k' best per row and knn_merge_kernel merges
-//     them (the keys are totally ordered, so the merged lists are the same).
+//     against all rows or (LIST) against the columns that its second run left for the 32 rows. When there
+//     are too few query rows to fill the GPU, the keys are split into slices (grid y); each slice writes
+//     its own k' best per row and knn_merge_kernel merges them (the keys are totally ordered, so the
+//     merged lists are the same).
 #include "engine.cuh"
 #include "knn_tc.cuh"
 
@@ -289,8 +290,8 @@ void knn_exact_device(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint64_t
   if (n == 0 || kp == 0) return;
   PM_REQUIRE(shard.count >= 1 && shard.index < shard.count, PACMAP_ERR_INVALID_ARGUMENT, "bad kNN shard");
   // AUTO uses the tensor cores once the O(n^2) part dominates; the TENSOR modes force them. At 5,000 rows the two
-  // paths take the same time at 16 columns and 15 neighbours (0.66 and 0.62 ms) and the tensor cores win everywhere else
-  // (100 columns: 0.85 against 1.05 ms at 15 neighbours, 1.05 against 1.43 at 72; 784 columns: 2.9 against 4.2); at
+  // paths take the same time at 16 columns and 15 neighbours (0.66 and 0.62 ms) and the tensor cores win everywhere
+  // else (100 columns: 0.85 against 1.05 ms at 15 neighbours, 1.05 against 1.43 at 72; 784 columns: 2.9 against 4.2); at
   // 4,000 the SIMT kernel wins up to 128 columns (100: 0.63 against 0.78). At 14,000 x 64 it is 1.2 against 4.2 ms.
   // The approximate search starts at 16,384 rows.
   const bool approx = mode == PACMAP_KNN_APPROX && n >= approx_threshold && n >= TC_APPROX_ROWS;

@@ -173,8 +173,8 @@ __global__ void __launch_bounds__(PV_BATCH * 32) pivot_draw_kernel(const float* 
   if (lane == 0) piv_rows[round * PV_BATCH + b] = static_cast<uint32_t>(sub_row(s, S, n));
 }
 
-// Step k of PV_FAR: dmin takes in the pivot that step k - 1 found (best[k - 1], written to piv_rows here), and best[k] the
-// largest dmin with its point: the distance's bits above, the complement of the point below (ties to the lower one).
+// Step k of PV_FAR: dmin takes in the pivot that step k - 1 found (best[k - 1], written to piv_rows here), and best[k]
+// the largest dmin with its point: the distance's bits above, the complement of the point below (ties to the lower one).
 __device__ __forceinline__ uint32_t far_point(unsigned long long key) { return ~static_cast<uint32_t>(key); }
 __global__ void __launch_bounds__(256) pivot_far_kernel(const float* __restrict__ x, uint64_t n, int d, uint32_t S, int k,
                                                         float* __restrict__ dmin,
@@ -566,7 +566,8 @@ void select_pivots(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint32_t* d
   DevBuf<unsigned long long> best(c, PV_FAR);
   PM_CUDA(cudaMemsetAsync(best.get(), 0, best.bytes(), c.stream));
   for (int k = 0; k < PV_FAR; ++k) {
-    pivot_far_kernel<<<nchunks, 256, 0, c.stream>>>(d_x, n, static_cast<int>(d), S, k, dmin.get(), best.get(), d_piv_rows);
+    pivot_far_kernel<<<nchunks, 256, 0, c.stream>>>(d_x, n, static_cast<int>(d), S, k, dmin.get(), best.get(),
+                                                    d_piv_rows);
     PM_LAUNCHED();
   }
   pivot_far_last_kernel<<<1, 1, 0, c.stream>>>(n, S, best.get(), d_piv_rows);

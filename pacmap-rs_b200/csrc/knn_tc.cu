@@ -1163,16 +1163,16 @@ __global__ void overflow_mark_kernel(const uint32_t* __restrict__ rows, const ui
     if (cand_cnt[rows[t]] < 0) cand_cnt[rows[t]] = entries;  // far rows keep their bound pass's band
 }
 
-// Far rows: after the bound pass, the few rows of a block whose bound is more than FAR_RATIO times (in squared distance) the
-// block's median bound, points apart from their cell. The tiles are chosen by a block's largest bounds, so six such
+// Far rows: after the bound pass, the few rows of a block whose bound is more than FAR_RATIO times (in squared distance)
+// the block's median bound, points apart from their cell. The tiles are chosen by a block's largest bounds, so six such
 // blocks of 400,000 rows in 256 columns visited 2,500 tiles each where the others visit 18, and the whole pass waited
 // for them: 6.0 ms, 0.3 without them. They join the overflowed rows instead: their bound no longer counts for their
 // block, their threshold lets nothing more in, and their bound pass's band gives them provisional neighbours.
 // Not when more than a quarter of a block would go (two cells of different density), or more than n / 64 in all.
 constexpr float FAR_RATIO = 4.0f;
 constexpr int FAR_BLOCK_MAX = TC_BM / 4;
-// Settling far rows apart takes about 0.6 ms; from 1,024 column tiles on a block that visits them all takes longer. (90,000
-// rows, 704 tiles: 4.4 ms without, 4.9 with.)
+// Settling far rows apart takes about 0.6 ms; from 1,024 column tiles on a block that visits them all takes longer.
+// (90,000 rows, 704 tiles: 4.4 ms without, 4.9 with.)
 constexpr uint64_t FAR_MIN_TILES = 1024;
 __global__ void __launch_bounds__(TC_BM) far_rows_kernel(uint64_t n, int rank, int blk0, const int* __restrict__ cand_cnt,
                                                          const float* __restrict__ ub, uint32_t* __restrict__ rows,

@@ -5,18 +5,21 @@
 //    segment (i, type) and partner i in the segment (j, type) -- via a counting sort, then each segment
 //    is sorted by partner. When the lists are grouped by point (the generated ones are), a mid-near or
 //    far segment is point i's own partners in pair order followed by the points that drew i, sorted:
-//    only that second part is placed by atomics and sorted (a neighbour segment is sorted whole). A pair's contribution to each endpoint is bit-identical whichever endpoint
-//    lists it (the squared distance and the weight use |y_i - y_j| only), so the sorted segments fix
-//    one deterministic summation order with no floating-point atomics. (The reference's rayon reduce,
-//    gradient.rs:53-70, has no fixed order at all.)
+//    only that second part is placed by atomics and sorted (a neighbour segment is sorted whole). A pair's
+//    contribution to each endpoint is bit-identical whichever endpoint lists it (the squared distance and
+//    the weight use |y_i - y_j| only), so the sorted segments fix one deterministic summation order with
+//    no floating-point atomics. (The reference's rayon reduce, gradient.rs:53-70, has no fixed order at
+//    all.)
 // K8 grad_adam_kernel: one group of G = 8 lanes per point sums its segments (NN c=10, MN c=10000, FP
 //    repulsive c=1, exactly the per-pair f32 arithmetic of gradient.rs:120-147), reduces across the
 //    group in a fixed butterfly, and applies the Adam step (adam.rs:45-57) to that point at once:
 //    y is ping-ponged between two buffers because other points read y_j during the iteration.
 //    Phase 3 has w_mn = 0: the MN segments are skipped (0 * finite = 0 adds nothing).
+//    Rows of more than 1,024 entries go to grad_adam_long_kernel beside it, a warp each. From 65,536 rows in 2-D
+//    and 3-D the near and far partners come from tiles of y in shared memory instead (grad_tiles.cu).
 // K9 optimize_device: up to about 18,900 rows all iterations run in one launch (grad_adam_resident_kernel); above,
-//    or with losses asked for, they are captured into one CUDA graph (one kernel node per iteration, snapshot
-//    copies as memcpy nodes). The per-iteration (w_nn, w_mn, w_fp, lr_t) schedule lives in a device table computed
+//    or with losses asked for, they are captured into one CUDA graph (one or two kernel nodes per iteration,
+//    snapshot copies as memcpy nodes). The per-iteration (w_nn, w_mn, w_fp, lr_t) schedule lives in a device table computed
 //    with the reference's f32 formulas.
 #include <chrono>
 #include <cmath>
@@ -540,7 +543,8 @@ __device__ __forceinline__ void load_y_shared(const float* y, uint32_t j, float 
 // gathers' rate).
 constexpr int RES_U = 4;
 template <int DIM, bool REPULSIVE>
-__device__ __forceinline__ void accumulate_resident(const float* y, const uint32_t* __restrict__ col, uint32_t s, uint32_t e, int gl, const float (&yi)[DIM], float c1,
+__device__ __forceinline__ void accumulate_resident(const float* y, const uint32_t* __restrict__ col, uint32_t s,
+                                                    uint32_t e, int gl, const float (&yi)[DIM], float c1,
                                                     float c2, float w, float (&acc)[DIM]) {
   constexpr uint32_t G = GRAD_G;
   for (uint32_t j = s + static_cast<uint32_t>(gl); j < e; j += RES_U * G) {
