@@ -121,8 +121,9 @@ struct TileGrad {
 };
 // Builds it when the problem's sizes favour it (else false, nothing built).
 bool build_tile_grad(Ctx& c, const Csr& csr, uint64_t n, uint64_t dim, uint64_t iters, TileGrad& out);
-// One iteration of every row but the long ones (which p.long_rows must name), on stream s: two launches.
-void launch_tile_grad(const TileGrad& tg, const GradArgs& p, uint64_t dim, int itr, cudaStream_t s);
+// One iteration of every row but the long ones (which p.long_rows must name), on stream s: two launches. mid: the
+// iteration's mid-near weight is not 0.
+void launch_tile_grad(const TileGrad& tg, const GradArgs& p, uint64_t dim, int itr, bool mid, cudaStream_t s);
 // out = num / x as the tiled gradient divides (tests).
 void debug_divide(Ctx& c, float num, const float* d_x, uint64_t n, float* d_out);
 

@@ -31,7 +31,7 @@ constexpr int TILE_SMEM = 232448;
 // The rule of build_tile_grad. From 65,536 rows on the tiled iteration wins by more than 10 us: at 60,000 rows in 2-D
 // it takes 30 us (3-D 40) against 42 (63) for grad_adam_kernel's order, which smaller fits keep to the bit; at 100,000
 // 47 (63) against 75 (112), at 200,000 86 (127) against 163 (236), at 400,000 189 (306) against 340 (510), at
-// 1,000,000 776 (1307) against 957 (1447): the fewer entries a row has in a tile, the more of a unit's time is its
+// 1,000,000 750 (1272) against 957 (1447): the fewer entries a row has in a tile, the more of a unit's time is its
 // fixed cost. Below 4 (4,000,000 rows in 3-D have 1.6) it would lose. Building the lists takes 0.3 ms at 100,000 rows
 // and 4 at 1,000,000, as much as 8 to 25 iterations win back, 40 below 6 entries.
 constexpr uint64_t TILE_MIN_ROWS = 65536;
@@ -323,8 +323,11 @@ __global__ void __launch_bounds__(FORCE_T, 1) tile_force_kernel(const ForceArgs 
 }
 
 // A row's tile sums (lane gl of eight adds tiles gl, gl + 8, ... in order), its mid-near pairs, the lanes' sums
-// pairwise, and the Adam step.
-template <int DIM>
+// pairwise, and the Adam step. Without the mid-near part (MID: their weight is not 0) a kernel of its own, 32 registers
+// a thread against 48: an iteration of the last phase at 1,000,000 rows 777 -> 750 us in 2-D, 1,320 -> 1,272 in 3-D.
+// With it the gathers' rate binds: four or eight partners in flight per lane instead of two changed nothing at
+// 1,000,000 rows.
+template <int DIM, bool MID>
 __global__ void __launch_bounds__(256) tile_adam_kernel(const GradArgs p, const float* __restrict__ partial,
                                                         uint32_t tiles, int itr) {
   const Sched sc = p.sched[itr];
@@ -355,10 +358,11 @@ __global__ void __launch_bounds__(256) tile_adam_kernel(const GradArgs p, const 
 #pragma unroll
     for (int c = 0; c < DIM; ++c) acc[c] = __fadd_rn(acc[c], v[c]);
   }
-  float unused = 0.0f;
-  if (sc.w_mn != 0.0f)
+  if constexpr (MID) {
+    float unused = 0.0f;
     accumulate_segment<DIM, false>(p.y_cur, p.col, s1, s2, gl, GRAD_G, yi, 10000.0f, 20000.0f, sc.w_mn, acc, unused,
                                    false);
+  }
 #pragma unroll
   for (int o = GRAD_G / 2; o > 0; o >>= 1)
 #pragma unroll
@@ -427,7 +431,7 @@ bool build_tile_grad(Ctx& c, const Csr& csr, uint64_t n, uint64_t dim, uint64_t 
   return true;
 }
 
-void launch_tile_grad(const TileGrad& tg, const GradArgs& p, uint64_t dim, int itr, cudaStream_t s) {
+void launch_tile_grad(const TileGrad& tg, const GradArgs& p, uint64_t dim, int itr, bool mid, cudaStream_t s) {
   ForceArgs f{};
   f.y = p.y_cur;
   f.partial = tg.partial.get();
@@ -441,13 +445,11 @@ void launch_tile_grad(const TileGrad& tg, const GradArgs& p, uint64_t dim, int i
   f.sched = p.sched;
   const size_t smem = static_cast<size_t>(tg.tile_pts + 1) * dim * sizeof(float);
   const unsigned rows = ceil_div(p.n, 256 / GRAD_G);
-  if (dim == 2) {
-    tile_force_kernel<2><<<tg.ctas, FORCE_T, smem, s>>>(f, itr);
-    tile_adam_kernel<2><<<rows, 256, 0, s>>>(p, tg.partial.get(), tg.tiles, itr);
-  } else {
-    tile_force_kernel<3><<<tg.ctas, FORCE_T, smem, s>>>(f, itr);
-    tile_adam_kernel<3><<<rows, 256, 0, s>>>(p, tg.partial.get(), tg.tiles, itr);
-  }
+  if (dim == 2) tile_force_kernel<2><<<tg.ctas, FORCE_T, smem, s>>>(f, itr);
+  else tile_force_kernel<3><<<tg.ctas, FORCE_T, smem, s>>>(f, itr);
+  const auto adam = dim == 2 ? (mid ? tile_adam_kernel<2, true> : tile_adam_kernel<2, false>)
+                             : (mid ? tile_adam_kernel<3, true> : tile_adam_kernel<3, false>);
+  adam<<<rows, 256, 0, s>>>(p, tg.partial.get(), tg.tiles, itr);
 }
 
 namespace {

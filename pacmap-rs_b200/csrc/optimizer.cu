@@ -1085,7 +1085,7 @@ void optimize_device(Ctx& c, const Csr& csr, const OptimizeArgs& a) {
       ++launches;
     }
     if (tiled) {
-      launch_tile_grad(tg, ga, dim, static_cast<int>(itr), c.stream);
+      launch_tile_grad(tg, ga, dim, static_cast<int>(itr), hs[itr].w_mn != 0.0f, c.stream);
       launches += 2;
     } else {
       fns.rows<<<grid, 256, 0, c.stream>>>(ga, static_cast<int>(itr));
