@@ -27,6 +27,7 @@
 #include <string>
 #include <type_traits>
 
+#include "arrivals.h"
 #include "engine.cuh"
 #include "grad.cuh"
 #include "ptx.cuh"
@@ -585,13 +586,13 @@ __device__ __forceinline__ bool grid_arrive_wait(uint32_t* arrived, uint32_t rou
   __syncthreads();
   if (threadIdx.x == 0) {
     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(arrived) : "memory");
-    const uint32_t want = round * gridDim.x;
+    const uint32_t want = arrivals_wanted(round, gridDim.x);
     const uint64_t t0 = globaltimer();
     uint32_t seen;
     int good = 1;
     for (uint32_t it = 1;; ++it) {
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(arrived) : "memory");
-      if (seen >= want) break;
+      if (arrivals_reached(seen, want)) break;
       if ((it & 255u) == 0 && globaltimer() - t0 > WAIT_LIMIT_NS) {
         good = 0;
         break;
@@ -960,7 +961,8 @@ bool optimize_resident(Ctx& c, const Csr& csr, const OptimizeArgs& a, ResidentFn
   if (blocks > static_cast<unsigned>(c.sm_count * per_sm)) return false;
   const uint64_t iters = a.itr_end - a.itr_begin;
   DevBuf<uint32_t> arrived(c, 1);
-  PM_CUDA(cudaMemsetAsync(arrived.get(), 0, sizeof(uint32_t), c.stream));
+  static_assert(ARRIVALS_START == 0xFFFFFFFFu, "set byte by byte");
+  PM_CUDA(cudaMemsetAsync(arrived.get(), 0xFF, sizeof(uint32_t), c.stream));
   DevBuf<int> slots;
   std::vector<int> hslots;
   if (a.d_snap && a.snapshots) {
