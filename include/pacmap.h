@@ -206,7 +206,8 @@ pacmap_status pacmap_optimize_steps(float* y, float* m, float* v, uint64_t n, ui
                                     float* out_grad);
 
 /* pacmap_grad (src/gradient.rs:35-74) with explicit weights: out_grad ((n+1) x dim) receives the
- * gradient of every point and the loss at [n, 0]. */
+ * gradient of every point and the loss at [n, 0]. Its sums run row by row; pacmap_optimize_steps may sum
+ * in another order from 65,536 rows on, so that the two agree to rounding there, not to the bit. */
 pacmap_status pacmap_gradient(const float* y, uint64_t n, uint64_t dim, const uint32_t* pnn, uint64_t n_nn,
                               const uint32_t* pmn, uint64_t n_mn, const uint32_t* pfp, uint64_t n_fp, float w_nn,
                               float w_mn, float w_fp, int32_t device, float* out_grad);

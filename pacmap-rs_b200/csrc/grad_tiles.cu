@@ -181,9 +181,12 @@ constexpr float NOWHERE = DIM == 2 ? 2.5e9f : 2.1e9f;
 // One entry of a row (gradient.rs:120-147): the partner's y from shared memory, its term added to acc. The per-pair
 // factor is w c2 / t^2 with t = c1 + 1 + |dy|^2; near pairs have w c2 = 20 w_nn and c1 = 10, far ones (bit 15 of e)
 // repel: -2 w_fp and 1. Multiplications and additions are fused here, which rounds less often than the separate ones.
-template <int DIM>
+// LOSS: its loss too, w_nn d / (10 + d) or w_fp / (1 + d) with d = 1 + |dy|^2, added to lacc; none is the unused places'
+// point, which has no loss. The arithmetic of the force is the same with and without.
+template <int DIM, bool LOSS>
 __device__ __forceinline__ void add_entry(const float* ys, uint32_t e, bool far, const float (&yi)[DIM],
-                                          float near_num, float far_num, float (&acc)[DIM]) {
+                                          float near_num, float far_num, float (&acc)[DIM], uint32_t none, float w_nn,
+                                          float w_fp, float& lacc) {
   float df[DIM];
   if constexpr (DIM == 2) {
     const float2 v = reinterpret_cast<const float2*>(ys)[e];
@@ -199,19 +202,29 @@ __device__ __forceinline__ void add_entry(const float* ys, uint32_t e, bool far,
   const float w1 = div_by(far ? far_num : near_num, t * t);
 #pragma unroll
   for (int c = 0; c < DIM; ++c) acc[c] = fmaf(w1, df[c], acc[c]);
+  if constexpr (LOSS) {
+    float dsq = 1.0f;
+#pragma unroll
+    for (int c = 0; c < DIM; ++c) dsq = fmaf(df[c], df[c], dsq);
+    const float part = far ? __fmul_rn(w_fp, __fdiv_rn(1.0f, __fadd_rn(1.0f, dsq)))
+                           : __fmul_rn(w_nn, __fdiv_rn(dsq, __fadd_rn(10.0f, dsq)));
+    if (e != none) lacc += part;
+  }
 }
 
 // The two entries of w, side by side and added in order.
-template <int DIM>
+template <int DIM, bool LOSS>
 __device__ __forceinline__ void add_two(const float* ys, uint32_t w, const float (&yi)[DIM], float near_num,
-                                        float far_num, float (&acc)[DIM]) {
-  add_entry<DIM>(ys, w & 0x7FFFu, (w & 0x8000u) != 0, yi, near_num, far_num, acc);
-  add_entry<DIM>(ys, (w >> 16) & 0x7FFFu, static_cast<int32_t>(w) < 0, yi, near_num, far_num, acc);
+                                        float far_num, float (&acc)[DIM], uint32_t none, float w_nn, float w_fp,
+                                        float& lacc) {
+  add_entry<DIM, LOSS>(ys, w & 0x7FFFu, (w & 0x8000u) != 0, yi, near_num, far_num, acc, none, w_nn, w_fp, lacc);
+  add_entry<DIM, LOSS>(ys, (w >> 16) & 0x7FFFu, static_cast<int32_t>(w) < 0, yi, near_num, far_num, acc, none, w_nn,
+                       w_fp, lacc);
 }
 
 struct ForceArgs {
   const float* y;
-  float* partial;
+  float *partial, *partial_loss;  // partial_loss: LOSS only
   const uint32_t *unit_off, *cta_units;
   const uint2* idx;
   const uint16_t* meta;
@@ -222,11 +235,12 @@ struct ForceArgs {
 // A unit: 32 rows of one window, a lane each, over their partners in one tile. Bound by the instructions per entry
 // (about 25; a two-wide form of the arithmetic was slower: its operands cost two more shared loads and the packing) and
 // per unit, and by the latency of the list words, which are two units ahead. 200,000 rows in 2-D: 72 us for 36 million
-// entries.
-template <int DIM>
+// entries. LOSS writes the row's loss over the tile's partners too, for the iterations whose loss is asked for: an instantiation
+// of its own, so that the others do not carry it, with the same sums of forces.
+template <int DIM, bool LOSS>
 __global__ void __launch_bounds__(FORCE_T, 1) tile_force_kernel(const ForceArgs p, int itr) {
   extern __shared__ __align__(16) float ys[];
-  const float near_num = 20.0f * p.sched[itr].w_nn, far_num = -2.0f * p.sched[itr].w_fp;
+  const float w_nn = p.sched[itr].w_nn, w_fp = p.sched[itr].w_fp, near_num = 20.0f * w_nn, far_num = -2.0f * w_fp;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t per_tile = p.windows * WIN_UNITS;
   uint32_t u = p.cta_units[blockIdx.x];
@@ -250,6 +264,7 @@ __global__ void __launch_bounds__(FORCE_T, 1) tile_force_kernel(const ForceArgs 
     const uint16_t* metap = p.meta + static_cast<uint64_t>(unit) * 32 + lane;
     uint32_t row0 = (unit / WIN_UNITS - t * p.windows) * WIN;
     float* outp = p.partial + (static_cast<uint64_t>(t) * p.n + row0) * DIM;
+    float* lossp = LOSS ? p.partial_loss + static_cast<uint64_t>(t) * p.n + row0 : nullptr;
     const float* yrow = p.y + static_cast<uint64_t>(row0) * DIM;
     // the first two words of a row's entries in the tile
     const uint2 none = make_uint2(p.tile_pts * 0x10001u, p.tile_pts * 0x10001u);
@@ -278,7 +293,7 @@ __global__ void __launch_bounds__(FORCE_T, 1) tile_force_kernel(const ForceArgs 
       const bool real = row0 + r < p.n;
       const uint2* words = p.idx + off + lane + 64;
       uint2 na = none, nb = none;
-      float yi_n[DIM] = {}, acc[DIM] = {};
+      float yi_n[DIM] = {}, acc[DIM] = {}, lacc = 0.0f;
       yrow += STEP / WIN_UNITS * WIN * DIM;
       row0 += STEP / WIN_UNITS * WIN;
       if (unit + STEP < ue) {
@@ -296,8 +311,8 @@ __global__ void __launch_bounds__(FORCE_T, 1) tile_force_kernel(const ForceArgs 
       for (uint32_t k = 0; k < most; k += 4) {
         const uint2 wk = k + 8 < c ? __ldcs(words) : none;
         words += 32;
-        add_two<DIM>(ys, wa.x, yi, near_num, far_num, acc);
-        if (k + 2 < most) add_two<DIM>(ys, wa.y, yi, near_num, far_num, acc);
+        add_two<DIM, LOSS>(ys, wa.x, yi, near_num, far_num, acc, p.tile_pts, w_nn, w_fp, lacc);
+        if (k + 2 < most) add_two<DIM, LOSS>(ys, wa.y, yi, near_num, far_num, acc, p.tile_pts, w_nn, w_fp, lacc);
         wa = wb;
         wb = wk;
       }
@@ -308,8 +323,10 @@ __global__ void __launch_bounds__(FORCE_T, 1) tile_force_kernel(const ForceArgs 
 #pragma unroll
           for (int d = 0; d < DIM; ++d) outp[r * DIM + d] = acc[d];
         }
+        if constexpr (LOSS) lossp[r] = lacc;
       }
       outp += STEP / WIN_UNITS * WIN * DIM;
+      if constexpr (LOSS) lossp += STEP / WIN_UNITS * WIN;
       offp += STEP;
       metap += STEP * 32;
       unit += STEP;
@@ -326,10 +343,10 @@ __global__ void __launch_bounds__(FORCE_T, 1) tile_force_kernel(const ForceArgs 
 // pairwise, and the Adam step. Without the mid-near part (MID: their weight is not 0) a kernel of its own, 32 registers
 // a thread against 48: an iteration of the last phase at 1,000,000 rows 777 -> 750 us in 2-D, 1,320 -> 1,272 in 3-D.
 // With it the gathers' rate binds: four or eight partners in flight per lane instead of two changed nothing at
-// 1,000,000 rows.
-template <int DIM, bool MID>
+// 1,000,000 rows. LOSS: the row's loss into p.row_loss, from the tiles' and the mid-near pairs', by the same lanes.
+template <int DIM, bool MID, bool LOSS>
 __global__ void __launch_bounds__(256) tile_adam_kernel(const GradArgs p, const float* __restrict__ partial,
-                                                        uint32_t tiles, int itr) {
+                                                        const float* __restrict__ partial_loss, uint32_t tiles, int itr) {
   const Sched sc = p.sched[itr];
   const int gl = threadIdx.x & (GRAD_G - 1);
   const uint64_t i = static_cast<uint64_t>(blockIdx.x) * (blockDim.x / GRAD_G) + threadIdx.x / GRAD_G;
@@ -343,6 +360,7 @@ __global__ void __launch_bounds__(256) tile_adam_kernel(const GradArgs p, const 
     yi[c] = p.y_cur[i * DIM + c];
     acc[c] = 0.0f;
   }
+  float lacc = 0.0f;
 #pragma unroll 4
   for (uint32_t t = gl; t < tiles; t += GRAD_G) {
     const float* src = partial + (static_cast<uint64_t>(t) * p.n + i) * DIM;
@@ -357,17 +375,18 @@ __global__ void __launch_bounds__(256) tile_adam_kernel(const GradArgs p, const 
     }
 #pragma unroll
     for (int c = 0; c < DIM; ++c) acc[c] = __fadd_rn(acc[c], v[c]);
+    if constexpr (LOSS) lacc += __ldcs(partial_loss + static_cast<uint64_t>(t) * p.n + i);
   }
-  if constexpr (MID) {
-    float unused = 0.0f;
-    accumulate_segment<DIM, false>(p.y_cur, p.col, s1, s2, gl, GRAD_G, yi, 10000.0f, 20000.0f, sc.w_mn, acc, unused,
-                                   false);
-  }
+  if constexpr (MID)
+    accumulate_segment<DIM, false>(p.y_cur, p.col, s1, s2, gl, GRAD_G, yi, 10000.0f, 20000.0f, sc.w_mn, acc, lacc, LOSS);
 #pragma unroll
-  for (int o = GRAD_G / 2; o > 0; o >>= 1)
+  for (int o = GRAD_G / 2; o > 0; o >>= 1) {
 #pragma unroll
     for (int c = 0; c < DIM; ++c) acc[c] = __fadd_rn(acc[c], __shfl_xor_sync(gmask, acc[c], o, GRAD_G));
+    if constexpr (LOSS) lacc += __shfl_xor_sync(gmask, lacc, o, GRAD_G);
+  }
   if (gl != 0) return;
+  if constexpr (LOSS) p.row_loss[i] = lacc;
 #pragma unroll
   for (int c = 0; c < DIM; ++c) {
     p.y_next[i * DIM + c] = adam_coord(acc[c], yi[c], p.m + i * DIM + c, p.v + i * DIM + c, p.a1, p.a2, sc.lr_t);
@@ -375,9 +394,22 @@ __global__ void __launch_bounds__(256) tile_adam_kernel(const GradArgs p, const 
   }
 }
 
+using ForceFn = void (*)(const ForceArgs, int);
+ForceFn force_kernel(uint64_t dim, bool loss) {
+  if (dim == 2) return loss ? tile_force_kernel<2, true> : tile_force_kernel<2, false>;
+  return loss ? tile_force_kernel<3, true> : tile_force_kernel<3, false>;
+}
+
+using AdamFn = void (*)(const GradArgs, const float*, const float*, uint32_t, int);
+template <bool LOSS>
+AdamFn adam_kernel(uint64_t dim, bool mid) {
+  if (dim == 2) return mid ? tile_adam_kernel<2, true, LOSS> : tile_adam_kernel<2, false, LOSS>;
+  return mid ? tile_adam_kernel<3, true, LOSS> : tile_adam_kernel<3, false, LOSS>;
+}
+
 }  // namespace
 
-bool build_tile_grad(Ctx& c, const Csr& csr, uint64_t n, uint64_t dim, uint64_t iters, TileGrad& out) {
+bool build_tile_grad(Ctx& c, const Csr& csr, uint64_t n, uint64_t dim, uint64_t iters, bool losses, TileGrad& out) {
   if ((dim != 2 && dim != 3) || n < TILE_MIN_ROWS || n >= (1ull << 24)) return false;
   const uint64_t fit = (TILE_SMEM / (4 * dim) - 1) / 4 * 4;  // a tile's points and NOWHERE
   const uint64_t tiles = (n + fit - 1) / fit;
@@ -426,8 +458,9 @@ bool build_tile_grad(Ctx& c, const Csr& csr, uint64_t n, uint64_t dim, uint64_t 
                                                                        out.cta_units.get());
   PM_LAUNCHED();
   out.partial.alloc(c, tiles * n * dim);
-  PM_CUDA(cudaFuncSetAttribute(tile_force_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, TILE_SMEM));
-  PM_CUDA(cudaFuncSetAttribute(tile_force_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, TILE_SMEM));
+  if (losses) out.partial_loss.alloc(c, tiles * n);
+  for (const bool loss : {false, true})
+    PM_CUDA(cudaFuncSetAttribute(force_kernel(dim, loss), cudaFuncAttributeMaxDynamicSharedMemorySize, TILE_SMEM));
   return true;
 }
 
@@ -435,6 +468,7 @@ void launch_tile_grad(const TileGrad& tg, const GradArgs& p, uint64_t dim, int i
   ForceArgs f{};
   f.y = p.y_cur;
   f.partial = tg.partial.get();
+  f.partial_loss = tg.partial_loss.get();
   f.unit_off = tg.unit_off.get();
   f.idx = reinterpret_cast<const uint2*>(tg.idx.get());
   f.cta_units = tg.cta_units.get();
@@ -445,11 +479,10 @@ void launch_tile_grad(const TileGrad& tg, const GradArgs& p, uint64_t dim, int i
   f.sched = p.sched;
   const size_t smem = static_cast<size_t>(tg.tile_pts + 1) * dim * sizeof(float);
   const unsigned rows = ceil_div(p.n, 256 / GRAD_G);
-  if (dim == 2) tile_force_kernel<2><<<tg.ctas, FORCE_T, smem, s>>>(f, itr);
-  else tile_force_kernel<3><<<tg.ctas, FORCE_T, smem, s>>>(f, itr);
-  const auto adam = dim == 2 ? (mid ? tile_adam_kernel<2, true> : tile_adam_kernel<2, false>)
-                             : (mid ? tile_adam_kernel<3, true> : tile_adam_kernel<3, false>);
-  adam<<<rows, 256, 0, s>>>(p, tg.partial.get(), tg.tiles, itr);
+  const bool loss = p.row_loss != nullptr;
+  force_kernel(dim, loss)<<<tg.ctas, FORCE_T, smem, s>>>(f, itr);
+  const AdamFn adam = loss ? adam_kernel<true>(dim, mid) : adam_kernel<false>(dim, mid);
+  adam<<<rows, 256, 0, s>>>(p, tg.partial.get(), tg.partial_loss.get(), tg.tiles, itr);
 }
 
 namespace {

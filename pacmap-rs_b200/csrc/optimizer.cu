@@ -950,15 +950,22 @@ struct Branch {
   Branch& operator=(const Branch&) = delete;
 };
 
-// optimize_device for rows that fit the GPU at once, eight lanes each; false when they do not, or when the call wants
-// what only the other path gives (losses, the last gradient, long rows beside the others).
-bool optimize_resident(Ctx& c, const Csr& csr, const OptimizeArgs& a, ResidentFn fn, const Sched* sched, float* yb,
-                       float a1, float a2) {
-  if (a.h_loss || a.d_grad_last || csr.n_long > 0 || a.n >= (1ull << 24)) return false;
+// The blocks of the resident form when all rows fit the GPU at once, eight lanes each, and none is a long one, else 0.
+unsigned resident_blocks(Ctx& c, const Csr& csr, uint64_t n, ResidentFn fn) {
+  if (csr.n_long > 0 || n >= (1ull << 24)) return 0;
   int per_sm = 0;
   PM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 256, 0));
-  const unsigned blocks = ceil_div(a.n, 256 / GRAD_G);
-  if (blocks > static_cast<unsigned>(c.sm_count * per_sm)) return false;
+  const unsigned blocks = ceil_div(n, 256 / GRAD_G);
+  return blocks <= static_cast<unsigned>(c.sm_count * per_sm) ? blocks : 0;
+}
+
+// optimize_device in the resident form; false when the rows do not fit, or when the call wants what only the other path
+// gives (losses, the last gradient).
+bool optimize_resident(Ctx& c, const Csr& csr, const OptimizeArgs& a, ResidentFn fn, const Sched* sched,
+                       float* const (&bufs)[2], float a1, float a2) {
+  if (a.h_loss || a.d_grad_last) return false;
+  const unsigned blocks = resident_blocks(c, csr, a.n, fn);
+  if (blocks == 0) return false;
   const uint64_t iters = a.itr_end - a.itr_begin;
   DevBuf<uint32_t> arrived(c, 1);
   static_assert(ARRIVALS_START == 0xFFFFFFFFu, "set byte by byte");
@@ -976,8 +983,8 @@ bool optimize_resident(Ctx& c, const Csr& csr, const OptimizeArgs& a, ResidentFn
     upload(c, slots, hslots.data(), iters);
   }
   ResidentArgs ra{};
-  ra.y[0] = a.d_y;
-  ra.y[1] = yb;
+  ra.y[0] = bufs[0];
+  ra.y[1] = bufs[1];
   ra.m = a.d_m;
   ra.v = a.d_v;
   ra.rp = csr.row_ptr.get();
@@ -995,8 +1002,8 @@ bool optimize_resident(Ctx& c, const Csr& csr, const OptimizeArgs& a, ResidentFn
   void* params[] = {&ra};
   PM_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(fn), dim3(blocks), dim3(256), params, 0, c.stream));
   count_launch();
-  if (iters & 1)
-    PM_CUDA(cudaMemcpyAsync(a.d_y, yb, a.n * a.dim * sizeof(float), cudaMemcpyDeviceToDevice, c.stream));
+  if (bufs[iters & 1] != a.d_y)
+    PM_CUDA(cudaMemcpyAsync(a.d_y, bufs[iters & 1], a.n * a.dim * sizeof(float), cudaMemcpyDeviceToDevice, c.stream));
   PM_CUDA(cudaStreamSynchronize(c.stream));
   last_graph_setup_ms() = 0.0;
   return true;
@@ -1012,8 +1019,9 @@ void optimize_device(Ctx& c, const Csr& csr, const OptimizeArgs& a) {
   const uint64_t n = a.n, dim = a.dim;
   if (a.itr_end <= a.itr_begin || n == 0 || dim == 0) return;
   PM_REQUIRE(dim <= 8, PACMAP_ERR_UNSUPPORTED, "the optimiser supports embedding dimensions 1..8");
-  if (a.h_loss && a.last_loss_only && a.itr_end - a.itr_begin > 1) {
-    // the iterations before the last without losses, which every form of the optimiser takes
+  const GradFns fns = pick_grad_kernel(dim);
+  if (a.h_loss && a.last_loss_only && a.itr_end - a.itr_begin > 1 && resident_blocks(c, csr, n, fns.resident) > 0) {
+    // the iterations before the last without losses, in the resident form
     OptimizeArgs b = a;
     b.itr_end = a.itr_end - 1;
     b.h_loss = nullptr;
@@ -1024,7 +1032,6 @@ void optimize_device(Ctx& c, const Csr& csr, const OptimizeArgs& a) {
     optimize_device(c, csr, b);
     return;
   }
-  const GradFns fns = pick_grad_kernel(dim);
   const uint64_t total_iters = a.p1 + a.p2 + a.p3;
   const uint64_t sched_len = std::max<uint64_t>(total_iters, a.itr_end);
   std::vector<Sched> hs(sched_len);
@@ -1036,16 +1043,26 @@ void optimize_device(Ctx& c, const Csr& csr, const OptimizeArgs& a) {
   DevBuf<float> yb(c, n * dim);
   DevBuf<float> row_loss, loss_dev;
   const uint64_t iters = a.itr_end - a.itr_begin;
+  const uint64_t losses = a.last_loss_only ? 1 : iters;
   if (a.h_loss) {
     row_loss.alloc(c, n);
-    loss_dev.alloc(c, iters);
+    loss_dev.alloc(c, losses);
   }
-  if (optimize_resident(c, csr, a, fns.resident, sched.get(), yb.get(), a1, a2)) return;
+  // The tiles of y are copied 16 bytes at a time and the points of two coordinates loaded by 8. A caller's buffer that
+  // starts off the 16-byte grid is worked on in a copy, so that its address does not choose the form of an iteration
+  // (whose sums differ in their last digits).
+  const bool on_grid = (reinterpret_cast<uintptr_t>(a.d_y) & 15u) == 0;
+  DevBuf<float> ya;
+  if (!on_grid) {
+    ya.alloc(c, n * dim);
+    PM_CUDA(cudaMemcpyAsync(ya.get(), a.d_y, n * dim * sizeof(float), cudaMemcpyDeviceToDevice, c.stream));
+  }
+  float* bufs[2] = {on_grid ? a.d_y : ya.get(), yb.get()};
+  if (optimize_resident(c, csr, a, fns.resident, sched.get(), bufs, a1, a2)) return;
   int per_sm = 0;
   PM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fns.rows, 256, 0));
   const unsigned grid = static_cast<unsigned>(std::max<uint64_t>(
       1, std::min<uint64_t>(ceil_div(n, 256 / GRAD_G), static_cast<uint64_t>(c.sm_count) * std::max(per_sm, 1))));
-  float* bufs[2] = {a.d_y, yb.get()};
   GradArgs ga{};
   ga.m = a.d_m;
   ga.v = a.d_v;
@@ -1057,12 +1074,9 @@ void optimize_device(Ctx& c, const Csr& csr, const OptimizeArgs& a) {
   ga.sched = sched.get();
   ga.a1 = a1;
   ga.a2 = a2;
-  ga.row_loss = a.h_loss ? row_loss.get() : nullptr;
-  // Many rows: the partners through shared memory, tile by tile (not with losses, which need every pair's term by row).
+  // Many rows: the partners through shared memory, tile by tile.
   TileGrad tg;
-  // The tiles are copied 16 bytes at a time: y is the caller's buffer.
-  const bool tiled = !a.h_loss && (reinterpret_cast<uintptr_t>(a.d_y) & 15u) == 0 &&
-                     build_tile_grad(c, csr, n, dim, iters, tg);
+  const bool tiled = build_tile_grad(c, csr, n, dim, iters, a.h_loss != nullptr, tg);
   if (tiled) {
     ga.long_rows = tg.long_rows.get();
     ga.n_long = tg.n_long;
@@ -1080,7 +1094,9 @@ void optimize_device(Ctx& c, const Csr& csr, const OptimizeArgs& a) {
     const int src = static_cast<int>((itr - a.itr_begin) & 1), dst = src ^ 1;
     ga.y_cur = bufs[src];
     ga.y_next = bufs[dst];
-    ga.grad_out = (itr + 1 == a.itr_end) ? a.d_grad_last : nullptr;
+    const bool last = itr + 1 == a.itr_end, want_loss = a.h_loss && (last || !a.last_loss_only);
+    ga.grad_out = last ? a.d_grad_last : nullptr;
+    ga.row_loss = want_loss ? row_loss.get() : nullptr;
     if (ga.n_long > 0) {
       capture_ok = branch.fork(c.stream) && capture_ok;
       fns.long_rows<<<ceil_div(ga.n_long, 8), 256, 0, branch.stream>>>(ga, static_cast<int>(itr));
@@ -1094,8 +1110,9 @@ void optimize_device(Ctx& c, const Csr& csr, const OptimizeArgs& a) {
       ++launches;
     }
     if (ga.n_long > 0) capture_ok = branch.join(c.stream) && capture_ok;
-    if (a.h_loss) {
-      loss_reduce_kernel<<<1, 1024, 0, c.stream>>>(row_loss.get(), n, loss_dev.get() + (itr - a.itr_begin));
+    if (want_loss) {
+      loss_reduce_kernel<<<1, 1024, 0, c.stream>>>(row_loss.get(), n,
+                                                   loss_dev.get() + (a.last_loss_only ? 0 : itr - a.itr_begin));
       ++launches;
     }
     if (a.d_snap && a.snapshots) {
@@ -1128,10 +1145,10 @@ void optimize_device(Ctx& c, const Csr& csr, const OptimizeArgs& a) {
   cudaGraphExecDestroy(exec);
   cudaGraphDestroy(graph);
   PM_CUDA(lerr);
-  if ((iters & 1) == 1)
-    PM_CUDA(cudaMemcpyAsync(a.d_y, yb.get(), n * dim * sizeof(float), cudaMemcpyDeviceToDevice, c.stream));
+  if (bufs[iters & 1] != a.d_y)
+    PM_CUDA(cudaMemcpyAsync(a.d_y, bufs[iters & 1], n * dim * sizeof(float), cudaMemcpyDeviceToDevice, c.stream));
   if (a.h_loss) {
-    PM_CUDA(cudaMemcpyAsync(a.h_loss, loss_dev.get(), iters * sizeof(float), cudaMemcpyDeviceToHost, c.stream));
+    PM_CUDA(cudaMemcpyAsync(a.h_loss, loss_dev.get(), losses * sizeof(float), cudaMemcpyDeviceToHost, c.stream));
   }
   PM_CUDA(cudaStreamSynchronize(c.stream));
 }

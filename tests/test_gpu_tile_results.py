@@ -1,0 +1,71 @@
+"""What a call returns from 65,536 rows on (the tiled gradient, 2-D and 3-D) depends on its data and schedule alone: the
+same bits whatever else is asked for, and the losses and the last gradient of the iterations that were run."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _lists(n, seed, ks=(12, 6, 24), hubs=()):
+    rng = np.random.default_rng(seed)
+    out = []
+    for q, k in enumerate(ks):
+        p = (np.arange(n)[:, None] + rng.integers(1, 300, size=(n, k))) % n if q == 0 else rng.integers(0, n, size=(n, k))
+        for h, size in hubs:
+            p[rng.choice(n, size=size * k // sum(ks), replace=False), 0] = h
+        out.append(np.stack([np.repeat(np.arange(n), k), p.reshape(-1)], 1).astype(np.uint32))
+    return out
+
+
+HUBS = [(0, 600), (129, 450), (65000, 1500), (777, 6000)]
+
+
+@pytest.mark.parametrize("n,dim", [(65537, 2), (66001, 3)])
+def test_asking_for_losses_changes_nothing(lib, n, dim):
+    x = np.random.default_rng(3).normal(size=(n, 8)).astype(np.float32)
+    cfg = lib.Configuration(initialization=lib.Initialization.Random(3), seed=5, num_iters=(14, 13, 13), snapshots=[5, 20, 40],
+                            embedding_dimensions=dim,
+                            pair_configuration=lib.PairConfiguration.AllProvided(*_lists(n, 11, hubs=HUBS)))
+    a, sa = lib.fit_transform(x, cfg)
+    b, sb, loss = lib.fit_transform(x, cfg, loss_trace=True)
+    assert np.array_equal(a, b) and np.array_equal(sa, sb)
+    assert loss.shape == (40,) and (loss > 0).all()
+
+
+# weights 3, 3, 1 and 1, 0, 1 in the last iteration; exactly the first size and a ragged one
+@pytest.mark.parametrize("n,dim,end", [(65536, 2, 164), (66001, 3, 219)])
+def test_last_gradient_and_loss(lib, orc, n, dim, end):
+    """out_grad leaves the state's bits alone, is the gradient that Adam took (its step on it gives y, m, v bit for bit),
+    and lies within the bounds of the other gradient tests: 1e-5 of a row's sum of |contributions|, the loss (a sum of
+    positive terms, at most 512 additions after one another and 8 roundings a term: 3e-5) 3e-5 of itself."""
+    pairs = _lists(n, n, hubs=HUBS)
+    y0 = np.random.default_rng(dim).normal(0, 4, size=(n, dim)).astype(np.float32)
+    state = [(y0.copy(), np.zeros_like(y0), np.zeros_like(y0)) for _ in range(2)]
+    g = lib.stages.optimize_steps(*state[0], *pairs, 1.0, 100, 100, end - 14, end)
+    lib.stages.optimize_steps(*state[1], *pairs, 1.0, 100, 100, end - 14, end, want_grad=False)
+    assert all(np.array_equal(p, q) for p, q in zip(*state))
+    y, m, v = y0.copy(), np.zeros_like(y0), np.zeros_like(y0)
+    lib.stages.optimize_steps(y, m, v, *pairs, 1.0, 100, 100, end - 14, end - 1, want_grad=False)
+    _, g64, absum = orc.grad(y, *pairs, *((3.0, 3.0, 1.0) if end < 200 else (1.0, 0.0, 1.0)), with64=True)
+    assert (np.abs(g[:-1] - g64[:-1]) <= 1e-5 * absum + 1e-30).all()
+    assert abs(g[-1, 0] - g64[-1, 0]) <= 3e-5 * abs(g64[-1, 0])
+    orc.adam(y, g, m, v, 1.0, end - 1)
+    assert all(np.array_equal(p, q) for p, q in zip((y, m, v), state[0]))
+
+
+@pytest.mark.parametrize("n,dim", [(66000, 2), (65537, 3), (3000, 2), (20000, 3)])
+def test_output_buffer_address_changes_nothing(lib, n, dim):
+    """fit_transform_device into a buffer 8 bytes off the 16-byte grid, after an odd and an even number of iterations."""
+    import torch
+
+    x = np.random.default_rng(3).normal(size=(n, 8)).astype(np.float32)
+    pairs = lib.PairConfiguration.AllProvided(*_lists(n, 12))
+    dx = torch.from_numpy(x).cuda()
+    for iters in ((6, 6, 6), (6, 6, 7)):
+        cfg = lib.Configuration(initialization=lib.Initialization.Random(3), seed=5, num_iters=iters, embedding_dimensions=dim,
+                                pair_configuration=pairs)
+        out = torch.zeros(dim * n + 2, device="cuda")
+        torch.cuda.synchronize()
+        lib.fit_transform_device(dx.data_ptr(), n, 8, out.data_ptr() + 8, cfg)
+        a, _ = lib.fit_transform(x, cfg)
+        assert np.array_equal(out[2:].cpu().numpy().reshape(n, dim), a)
