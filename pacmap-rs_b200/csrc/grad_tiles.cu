@@ -387,11 +387,7 @@ __global__ void __launch_bounds__(256) tile_adam_kernel(const GradArgs p, const 
   }
   if (gl != 0) return;
   if constexpr (LOSS) p.row_loss[i] = lacc;
-#pragma unroll
-  for (int c = 0; c < DIM; ++c) {
-    p.y_next[i * DIM + c] = adam_coord(acc[c], yi[c], p.m + i * DIM + c, p.v + i * DIM + c, p.a1, p.a2, sc.lr_t);
-    if (p.grad_out) p.grad_out[i * DIM + c] = acc[c];
-  }
+  finish_row<DIM>(p, i, acc, yi, sc.lr_t);
 }
 
 using ForceFn = void (*)(const ForceArgs, int);

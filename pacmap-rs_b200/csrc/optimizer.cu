@@ -483,12 +483,7 @@ __device__ __forceinline__ void grad_adam_row(const GradArgs& p, const Sched& sc
     if (want_loss) lacc += __shfl_xor_sync(gmask, lacc, o, G);
   }
   if (gl == 0) {
-#pragma unroll
-    for (int c = 0; c < DIM; ++c) {
-      if (!p.grad_only)
-        p.y_next[i * DIM + c] = adam_coord(acc[c], yi[c], p.m + i * DIM + c, p.v + i * DIM + c, p.a1, p.a2, sc.lr_t);
-      if (p.grad_out) p.grad_out[i * DIM + c] = acc[c];
-    }
+    finish_row<DIM>(p, i, acc, yi, sc.lr_t);
     if (want_loss) p.row_loss[i] = lacc;
   }
 }
