@@ -33,10 +33,10 @@ constexpr int TILE_SMEM = 232448;
 // 47 (63) against 75 (112), at 200,000 86 (127) against 163 (236), at 400,000 189 (306) against 340 (510), at
 // 1,000,000 750 (1272) against 957 (1447): the fewer entries a row has in a tile, the more of a unit's time is its
 // fixed cost. Below 4 (4,000,000 rows in 3-D have 1.6) it would lose. Building the lists takes 0.3 ms at 100,000 rows
-// and 4 at 1,000,000, as much as 8 to 25 iterations win back, 40 below 6 entries.
+// and 4 at 1,000,000, as much as 8 to 25 iterations win back. The number of iterations is no part of the rule all the
+// same: the sums' order, and with it their last digits, would depend on how a caller cuts a schedule into calls.
 constexpr uint64_t TILE_MIN_ROWS = 65536;
 constexpr double TILE_MIN_ENTRIES = 4.0;
-uint64_t tile_min_iters(double entries) { return entries >= 16.0 ? 12 : (entries >= 6.0 ? 32 : 64); }
 
 __device__ __forceinline__ uint32_t div_magic(uint32_t col, uint64_t magic) {
   return static_cast<uint32_t>((col * magic) >> 40);  // col / tile_pts for col < 2^24, tile_pts < 2^15
@@ -405,14 +405,13 @@ AdamFn adam_kernel(uint64_t dim, bool mid) {
 
 }  // namespace
 
-bool build_tile_grad(Ctx& c, const Csr& csr, uint64_t n, uint64_t dim, uint64_t iters, bool losses, TileGrad& out) {
+bool build_tile_grad(Ctx& c, const Csr& csr, uint64_t n, uint64_t dim, bool losses, TileGrad& out) {
   if ((dim != 2 && dim != 3) || n < TILE_MIN_ROWS || n >= (1ull << 24)) return false;
   const uint64_t fit = (TILE_SMEM / (4 * dim) - 1) / 4 * 4;  // a tile's points and NOWHERE
   const uint64_t tiles = (n + fit - 1) / fit;
   const double per_row = static_cast<double>(csr.entries) / static_cast<double>(n);
   const double entries = per_row / static_cast<double>(tiles);  // of a row in a tile
-  if (tiles > MAX_TILES || per_row > 0.8 * ROW_MAX || entries < TILE_MIN_ENTRIES || iters < tile_min_iters(entries))
-    return false;
+  if (tiles > MAX_TILES || per_row > 0.8 * ROW_MAX || entries < TILE_MIN_ENTRIES) return false;
   out.tiles = static_cast<uint32_t>(tiles);
   out.tile_pts = static_cast<uint32_t>(((n + tiles - 1) / tiles + 3) / 4 * 4);
   out.windows = ceil_div(n, WIN);

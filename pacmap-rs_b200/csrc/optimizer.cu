@@ -1071,7 +1071,7 @@ void optimize_device(Ctx& c, const Csr& csr, const OptimizeArgs& a) {
   ga.a2 = a2;
   // Many rows: the partners through shared memory, tile by tile.
   TileGrad tg;
-  const bool tiled = build_tile_grad(c, csr, n, dim, iters, a.h_loss != nullptr, tg);
+  const bool tiled = build_tile_grad(c, csr, n, dim, a.h_loss != nullptr, tg);
   if (tiled) {
     ga.long_rows = tg.long_rows.get();
     ga.n_long = tg.n_long;

@@ -69,3 +69,19 @@ def test_output_buffer_address_changes_nothing(lib, n, dim):
         lib.fit_transform_device(dx.data_ptr(), n, 8, out.data_ptr() + 8, cfg)
         a, _ = lib.fit_transform(x, cfg)
         assert np.array_equal(out[2:].cpu().numpy().reshape(n, dim), a)
+
+
+@pytest.mark.parametrize("n,dim", [(65536, 2), (90001, 3)])
+def test_a_schedule_cut_into_calls_changes_nothing(lib, n, dim):
+    """Twenty iterations across the last change of phase in one call, in two, and one by one; with the gradient asked for in
+    some."""
+    pairs = _lists(n, n, hubs=HUBS)
+    y0 = np.random.default_rng(dim).normal(0, 4, size=(n, dim)).astype(np.float32)
+    states = []
+    for cuts in ((190, 210), (190, 200, 210), (190, *range(191, 211))):
+        y, m, v = y0.copy(), np.zeros_like(y0), np.zeros_like(y0)
+        for a, b in zip(cuts, cuts[1:]):
+            lib.stages.optimize_steps(y, m, v, *pairs, 1.0, 100, 100, a, b, want_grad=b % 3 == 0)
+        states.append((y, m, v))
+    for s in states[1:]:
+        assert all(np.array_equal(p, q) for p, q in zip(states[0], s))
