@@ -117,7 +117,7 @@ struct Csr {
   DevBuf<uint32_t> col;      // partner of each entry, ascending within a segment
   DevBuf<uint32_t> long_rows;  // the rows with the most entries, which the gradient gives a warp each
   uint32_t n_long = 0;
-  uint64_t entries = 0;
+  uint64_t entries = 0, entries_mn = 0;  // all, and at most how many of mid-near pairs
 };
 // grouped_known: the lists are known to hold each point's pairs together (generated lists), so the
 // device check of that (a kernel and a host round trip) is skipped.

@@ -28,15 +28,18 @@ constexpr int MAX_TILES = 64;
 constexpr uint32_t ROW_MAX = 511;    // entries of a row: 9 bits in meta; longer rows get a warp each
 constexpr int TILE_SMEM = 232448;
 
-// The rule of build_tile_grad. From 65,536 rows on the tiled iteration wins by more than 10 us: at 60,000 rows in 2-D
-// it takes 30 us (3-D 40) against 42 (63) for grad_adam_kernel's order, which smaller fits keep to the bit; at 100,000
-// 47 (63) against 75 (112), at 200,000 86 (127) against 163 (236), at 400,000 189 (306) against 340 (510), at
-// 1,000,000 750 (1272) against 957 (1447): the fewer entries a row has in a tile, the more of a unit's time is its
-// fixed cost. Below 4 (4,000,000 rows in 3-D have 1.6) it would lose. Building the lists takes 0.3 ms at 100,000 rows
-// and 4 at 1,000,000, as much as 8 to 25 iterations win back. The number of iterations is no part of the rule all the
-// same: the sums' order, and with it their last digits, would depend on how a caller cuts a schedule into calls.
+// The rule of build_tile_grad, from 65,536 rows on (smaller fits keep grad_adam_kernel's order of sums to the bit). An
+// iteration of the last phase, tiled against grad_adam_kernel, in us, lists in random order of rows, 2-D (3-D):
+//   65,536 rows with 144 near and far entries each 29 (39) against 44 (66); 100,000 with 144 41 (51) / 67 (97);
+//   200,000 with 192 80 (108) / 167 (243); 400,000 with 192 170 (252) / 320 (482); 1,000,000 with 240 734 (1177) / 961 (1463).
+// Two fixed costs bound it from below: of a row in each tile (a unit's time whatever its entries), paid from 3 to 4.5
+// entries per row and tile on (1,000,000 rows, 2-D: 4.1 entries 592 / 599, 2.7 507 / 433), and of the second kernel and the
+// tiles' loads, paid from 24 to 50 entries per row on (65,536 rows, 2-D: 36 entries 18.4 / 18.8, with neighbours close by in
+// memory 19.2 / 17.1). Building the lists takes 0.1 ms at 100,000 rows and 3 at 1,000,000. The number of iterations is no
+// part of the rule: the sums' order, and with it their last digits, would depend on how a caller cuts a schedule into calls.
 constexpr uint64_t TILE_MIN_ROWS = 65536;
-constexpr double TILE_MIN_ENTRIES = 4.0;
+constexpr double TILE_MIN_ROW_ENTRIES = 48.0;
+double tile_min_entries(uint64_t dim) { return dim == 2 ? 4.5 : 4.0; }
 
 __device__ __forceinline__ uint32_t div_magic(uint32_t col, uint64_t magic) {
   return static_cast<uint32_t>((col * magic) >> 40);  // col / tile_pts for col < 2^24, tile_pts < 2^15
@@ -410,8 +413,10 @@ bool build_tile_grad(Ctx& c, const Csr& csr, uint64_t n, uint64_t dim, bool loss
   const uint64_t fit = (TILE_SMEM / (4 * dim) - 1) / 4 * 4;  // a tile's points and NOWHERE
   const uint64_t tiles = (n + fit - 1) / fit;
   const double per_row = static_cast<double>(csr.entries) / static_cast<double>(n);
-  const double entries = per_row / static_cast<double>(tiles);  // of a row in a tile
-  if (tiles > MAX_TILES || per_row > 0.8 * ROW_MAX || entries < TILE_MIN_ENTRIES) return false;
+  const double near_far = static_cast<double>(csr.entries - csr.entries_mn) / static_cast<double>(n);
+  if (tiles > MAX_TILES || per_row > 0.8 * ROW_MAX || near_far < TILE_MIN_ROW_ENTRIES ||
+      near_far < tile_min_entries(dim) * static_cast<double>(tiles))
+    return false;
   out.tiles = static_cast<uint32_t>(tiles);
   out.tile_pts = static_cast<uint32_t>(((n + tiles - 1) / tiles + 3) / 4 * 4);
   out.windows = ceil_div(n, WIN);

@@ -813,6 +813,7 @@ void build_csr(Ctx& c, uint64_t n, const uint32_t* d_pnn, uint64_t n_nn, const u
   PM_CUDA(cudaMemcpyAsync(&total, out.row_ptr.get() + nseg, sizeof(uint32_t), cudaMemcpyDeviceToHost, c.stream));
   PM_CUDA(cudaStreamSynchronize(c.stream));
   out.entries = total;
+  out.entries_mn = std::min<uint64_t>(total, 2 * n_mn);
   out.col.alloc(c, std::max<uint64_t>(total, 1));
   if (grouped) {
     // forward entries in pair order; reverse entries after them by atomics (cursor = row_ptr + forward)
