@@ -165,10 +165,10 @@ __global__ void tile_shares_kernel(const uint32_t* __restrict__ unit_off, uint64
 // num / x for x >= 1, without a branch: an approximate reciprocal, one Newton step, and a correction of the quotient by
 // its exact remainder (P. W. Markstein, Computation of elementary functions on the IBM RISC System/6000 processor, IBM
 // J. Res. Dev. 34, 1990): correctly rounded up to x = 2^126 (tested against the / operator for every mantissa of x),
-// 0 beyond, where the quotient is below 1e-36. The compiler's division checks its operands and branches, which kept
+// 0 beyond, where the quotient is below 1e-36; NaN for NaN, as a division. The compiler's division checks its operands and branches, which kept
 // two entries' divisions from overlapping.
 __device__ __forceinline__ float div_by(float num, float x) {
-  x = fminf(x, 3.402823466e+38f);
+  asm("min.NaN.f32 %0, %0, %1;" : "+f"(x) : "f"(3.402823466e+38f));  // infinity would make the remainder NaN
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   y = fmaf(fmaf(-x, y, 1.0f), y, y);

@@ -85,3 +85,21 @@ def test_a_schedule_cut_into_calls_changes_nothing(lib, n, dim):
         states.append((y, m, v))
     for s in states[1:]:
         assert all(np.array_equal(p, q) for p, q in zip(states[0], s))
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+def test_non_finite_coordinates_spread_as_in_the_reference(lib, orc, dim):
+    """A NaN in one coordinate of a point makes its pairs' factors NaN, and so all coordinates of its partners' gradients; an
+    infinite one makes the factors 0, and only its own coordinate NaN (0 times infinity). The mid-near pairs are left out
+    in the last phase, where their weight is 0 (the engine skips them there, in every form)."""
+    n = 65600
+    pairs = _lists(n, 5, hubs=HUBS)
+    y = np.random.default_rng(dim).normal(0, 4, size=(n, dim)).astype(np.float32)
+    y[300, 0], y[40000, dim - 1], y[65599] = np.nan, np.nan, np.nan
+    y[7, 1], y[50001, 0], y[12345] = np.inf, -np.inf, np.inf
+    for itr, w in ((150, (3.0, 3.0, 1.0)), (220, (1.0, 0.0, 1.0))):
+        g = lib.stages.optimize_steps(y.copy(), np.zeros_like(y), np.zeros_like(y), *pairs, 1.0, 100, 100, itr, itr + 1)
+        with np.errstate(all="ignore"):
+            e = orc.grad(y, pairs[0], pairs[1] if w[1] else pairs[1][:0], pairs[2], *w)
+        assert np.array_equal(np.isnan(g[:-1]), np.isnan(e[:-1]))
+        assert 300 < np.isnan(e[:-1]).any(1).sum() < n // 10
