@@ -176,10 +176,10 @@ __device__ __forceinline__ float div_by(float num, float x) {
   return fmaf(fmaf(-x, q, num), y, q);
 }
 
-// The place after a tile's points that unused places of a unit name: a point so far away that t^2 is between 2^126 and
-// the largest number, whose factor is 0.
-template <int DIM>
-constexpr float NOWHERE = DIM == 2 ? 2.5e9f : 2.1e9f;
+// The coordinates of the place after a tile's points, which unused places of a unit name. Whatever finite yi is, that place
+// adds nothing: numbers of this size lie 2^76 apart, so a coordinate's difference is 0 or so large that t^2 is infinite
+// and the factor 0 (or all differences are 0); and no difference overflows, which would make 0 times it NaN.
+constexpr float NOWHERE = 1e30f;
 
 // One entry of a row (gradient.rs:120-147): the partner's y from shared memory, its term added to acc. The per-pair
 // factor is w c2 / t^2 with t = c1 + 1 + |dy|^2; near pairs have w c2 = 20 w_nn and c1 = 10, far ones (bit 15 of e)
@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(FORCE_T, 1) tile_force_kernel(const ForceArgs 
     __syncthreads();
     for (uint32_t e = threadIdx.x; e < floats / 4; e += FORCE_T) cp_async16(ys + 4 * e, src + 4 * e);
     for (uint32_t e = (floats & ~3u) + threadIdx.x; e < floats; e += FORCE_T) ys[e] = src[e];
-    if (threadIdx.x < DIM) ys[p.tile_pts * DIM + threadIdx.x] = NOWHERE<DIM>;
+    if (threadIdx.x < DIM) ys[p.tile_pts * DIM + threadIdx.x] = NOWHERE;
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     // While a unit is summed, the next one's first entries and its rows' y are on their way, and the place and rows of
@@ -364,8 +364,10 @@ __global__ void __launch_bounds__(256) tile_adam_kernel(const GradArgs p, const 
     acc[c] = 0.0f;
   }
   float lacc = 0.0f;
+  // A row without near and far pairs has only unused places, whose sums are NaN when its y is not finite.
+  const uint32_t used = s0 == s1 && s2 == s3 ? 0u : tiles;
 #pragma unroll 4
-  for (uint32_t t = gl; t < tiles; t += GRAD_G) {
+  for (uint32_t t = gl; t < used; t += GRAD_G) {
     const float* src = partial + (static_cast<uint64_t>(t) * p.n + i) * DIM;
     float v[DIM];
     if constexpr (DIM == 2) {

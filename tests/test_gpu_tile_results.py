@@ -103,3 +103,41 @@ def test_non_finite_coordinates_spread_as_in_the_reference(lib, orc, dim):
             e = orc.grad(y, pairs[0], pairs[1] if w[1] else pairs[1][:0], pairs[2], *w)
         assert np.array_equal(np.isnan(g[:-1]), np.isnan(e[:-1]))
         assert 300 < np.isnan(e[:-1]).any(1).sum() < n // 10
+
+
+def _moment_gradient(lib, y, pairs):
+    """The gradient in the last phase, from Adam's first moment after 14 iterations with a learning rate of 0."""
+    m = np.zeros_like(y)
+    lib.stages.optimize_steps(y.copy(), m, np.zeros_like(y), *pairs, 0.0, 100, 100, 220, 234, want_grad=False)
+    return m / (1 - 0.9 ** 14)
+
+
+# around 2.1e9, 2.5e9 and 1e30, and at the largest numbers of both signs, in all coordinates and in one
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("at", [2.1e9, 2.5e9, 1e30, -1e30, 3.4e38, -3.4e38])
+def test_points_anywhere_have_only_their_own_pairs(lib, orc, dim, at):
+    """Far points, whose true factors are 0 or tiny; the places that fill a tile's lists up must not act on them either."""
+    n = 65537
+    pairs = _lists(n, 8)
+    rng = np.random.default_rng(dim)
+    y = rng.normal(0, 4, size=(n, dim)).astype(np.float32)
+    y[::3000] = np.float32(at)
+    y[5::3000] = np.nextafter(np.float32(at), np.float32(0))
+    y[9::3000, 0] = np.float32(at)
+    g = _moment_gradient(lib, y, pairs)
+    with np.errstate(all="ignore"):
+        _, e64, absum = orc.grad(y, *pairs, 1.0, 0.0, 1.0, with64=True)
+    assert np.isfinite(g).all() and np.isfinite(absum).all()
+    assert (np.abs(g - e64[:-1]) <= 1e-5 * absum + 1e-26).all()
+
+
+def test_points_without_near_and_far_pairs(lib):
+    """Points with no pairs at all, or mid-near ones only, among others of their window: no gradient, wherever they lie."""
+    n = 65537
+    alone = np.array([0, 5, 130, 65536])
+    pnn, pmn, pfp = (p[~np.isin(p, alone).any(1)] for p in _lists(n, 8))
+    pmn = np.concatenate([pmn, np.array([[5, 9]], np.uint32)])
+    y = np.random.default_rng(1).normal(0, 4, size=(n, 2)).astype(np.float32)
+    y[alone] = [[np.inf, 1], [3, 4], [np.nan, np.nan], [-1e30, 1e30]]
+    g = _moment_gradient(lib, y, (pnn, pmn, pfp))
+    assert (g[alone] == 0).all() and np.isfinite(g).all()
