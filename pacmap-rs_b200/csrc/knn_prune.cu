@@ -18,7 +18,8 @@
 // Pivots: k-means++ seeding (Arthur & Vassilvitskii, SODA 2007) in batches of 16 draws on a subsample of
 // at most 16,384 rows, then 16 times the point farthest from every pivot (Gonzalez, Theor. Comput. Sci. 38, 1985), so
 // that every well-separated group of points receives a pivot and the cells stay compact; the draws come from
-// a Philox4x32-10 stream with a fixed key (the same pivots on every call).
+// a Philox4x32-10 stream with a fixed key (the same pivots on every call). The approximate search, whose rows depend on
+// the cells, draws all of its pivots, on up to 65,536 rows.
 #include <algorithm>
 #include <cmath>
 
@@ -34,9 +35,9 @@ constexpr int PV_BATCH = 16;             // pivots drawn per round
 // points then spread over other cells and spoiled their bounds (400,000 x 256 from 200 Gaussians: 788,000 of 4,886,000
 // tile pairs kept with 256 draws, 28,000 with 240 and 16 farthest).
 constexpr int PV_FAR = 16;
-// 64 points per pivot; four times as many took 0.8 ms longer on that data and pruned no better.
-constexpr uint32_t PV_SUB_MAX = 16384;   // subsample size limit
-constexpr int PV_CHUNK = 64;             // subsample points per block (and per prefix-sum entry)
+// The subsample: up to 256 chunks of CHUNK points, one per block (and per prefix-sum entry). 64 points per pivot for the
+// exact search; four times as many took 0.8 ms longer on that data and pruned no better.
+constexpr int PV_CHUNKS = 256, CHUNK_EXACT = 64, CHUNK_PROBE = 256;
 constexpr uint32_t TAG_PIVOT = 0x50495654u;  // 'PIVT'
 constexpr int SEGS = 4;                  // cell segments kept per tile (further cells merge into the last)
 constexpr float PRUNE_MARGIN = 1e-4f;    // relative margin of the skip test
@@ -48,6 +49,7 @@ __host__ __device__ __forceinline__ uint64_t sub_row(uint32_t s, uint32_t S, uin
 // dmin[s] = min(dmin[s], |x_row(s) - q|^2 over the 16 pivots q of the batch starting at p0) for the
 // subsample points of this block's chunk, and the chunk's sum of dmin (f64, a fixed order). p0 == 0
 // starts dmin from +inf. One warp per point, lanes over the columns; the batch is staged in shared memory.
+template <int CHUNK>
 __global__ void __launch_bounds__(256) pivot_dmin_kernel(const float* __restrict__ x, uint64_t n, int d, uint32_t S,
                                                          const uint32_t* __restrict__ piv_rows, int p0,
                                                          float* __restrict__ dmin, double* __restrict__ chunk_sum) {
@@ -59,13 +61,13 @@ __global__ void __launch_bounds__(256) pivot_dmin_kernel(const float* __restrict
   }
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  constexpr int PER_WARP = PV_CHUNK / 8;
+  constexpr int PER_WARP = CHUNK / 8;
   double ws = 0.0;
   // four subsample rows at a time (their loads in flight together); each row's sums and the order of
   // the block's double sum are those of one row at a time
   static_assert(PER_WARP % 4 == 0 && (PIV - PV_FAR) % PV_BATCH == 0, "rows are taken four at a time");
   for (int t0 = 0; t0 < PER_WARP; t0 += 4) {
-    const uint32_t s0 = blockIdx.x * PV_CHUNK + warp * PER_WARP + t0;
+    const uint32_t s0 = blockIdx.x * CHUNK + warp * PER_WARP + t0;
     if (s0 >= S) break;  // warp-uniform
     const float* xr[4];
 #pragma unroll
@@ -117,12 +119,13 @@ __global__ void __launch_bounds__(256) pivot_dmin_kernel(const float* __restrict
 // Round 0: 16 evenly spaced subsample points. Round r > 0: 16 draws, each point with probability
 // proportional to dmin (its squared distance to the nearest pivot so far); a degenerate subsample (all
 // dmin zero) falls back to evenly spaced points.
+template <int CHUNK>
 __global__ void __launch_bounds__(PV_BATCH * 32) pivot_draw_kernel(const float* __restrict__ dmin, uint32_t S,
                                                                    uint64_t n, const double* __restrict__ chunk_sum,
                                                                    int nchunks, int round,
                                                                    uint32_t* __restrict__ piv_rows) {
-  __shared__ double cs[PV_SUB_MAX / PV_CHUNK];
-  __shared__ double pre[PV_SUB_MAX / PV_CHUNK + 1];
+  __shared__ double cs[PV_CHUNKS];
+  __shared__ double pre[PV_CHUNKS + 1];
   for (int ch = threadIdx.x; round > 0 && ch < nchunks; ch += blockDim.x) cs[ch] = chunk_sum[ch];
   __syncthreads();
   if (threadIdx.x == 0) {  // the prefix in chunk order, from shared memory
@@ -153,7 +156,7 @@ __global__ void __launch_bounds__(PV_BATCH * 32) pivot_draw_kernel(const float* 
       else hi = mid - 1;
     }
     double acc = pre[lo];
-    const uint32_t a = static_cast<uint32_t>(lo) * PV_CHUNK, e = min(S, a + PV_CHUNK);
+    const uint32_t a = static_cast<uint32_t>(lo) * CHUNK, e = min(S, a + CHUNK);
     uint32_t pick = 0xFFFFFFFFu;
     bool done = false;
     for (uint32_t base = a; base < e && !done; base += 32) {
@@ -188,8 +191,8 @@ __global__ void __launch_bounds__(256) pivot_far_kernel(const float* __restrict_
     if (blockIdx.x == 0 && threadIdx.x == 0) piv_rows[PIV - PV_FAR + k - 1] = static_cast<uint32_t>(q);
   }
   unsigned long long mine = 0;
-  for (int t = 0; t < PV_CHUNK / 8; ++t) {
-    const uint32_t s = blockIdx.x * PV_CHUNK + warp * (PV_CHUNK / 8) + t;
+  for (int t = 0; t < CHUNK_EXACT / 8; ++t) {
+    const uint32_t s = blockIdx.x * CHUNK_EXACT + warp * (CHUNK_EXACT / 8) + t;
     if (s >= S) break;  // warp-uniform
     float v = dmin[s];
     if (k > 0) {
@@ -540,34 +543,48 @@ uint64_t build_probe_tile_lists(Ctx& c, const float* d_x, uint64_t d, const uint
   return total;
 }
 
-void select_pivots(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint32_t* d_piv_rows, bool seeded) {
-  if (!seeded) {
+namespace {
+// The first `rounds` batches of pivots by draws; dmin ends up with the distances to all of them.
+template <int CHUNK>
+void draw_pivots(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint32_t S, int rounds, bool last_dmin, float* dmin,
+                 uint32_t* d_piv_rows) {
+  const int nchunks = static_cast<int>(ceil_div(S, CHUNK));
+  DevBuf<double> csum(c, nchunks);
+  const size_t smem = static_cast<size_t>(PV_BATCH) * d * sizeof(float);
+  PM_CUDA(cudaFuncSetAttribute(pivot_dmin_kernel<CHUNK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               static_cast<int>(smem)));
+  for (int r = 0; r <= rounds; ++r) {
+    if (r > 0 && (r < rounds || last_dmin)) {
+      pivot_dmin_kernel<CHUNK><<<nchunks, 256, smem, c.stream>>>(d_x, n, static_cast<int>(d), S, d_piv_rows,
+                                                                 (r - 1) * PV_BATCH, dmin, csum.get());
+      PM_LAUNCHED();
+    }
+    if (r == rounds) break;
+    pivot_draw_kernel<CHUNK><<<1, PV_BATCH * 32, 0, c.stream>>>(dmin, S, n, csum.get(), nchunks, r, d_piv_rows);
+    PM_LAUNCHED();
+  }
+}
+}  // namespace
+
+void select_pivots(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint32_t* d_piv_rows, PivotUse use) {
+  if (use == PivotUse::ORDER) {
     even_pivots_kernel<<<1, PIV, 0, c.stream>>>(n, d_piv_rows);
     PM_LAUNCHED();
     return;
   }
-  const uint32_t S = static_cast<uint32_t>(std::min<uint64_t>(n, PV_SUB_MAX));
-  const int nchunks = static_cast<int>(ceil_div(S, PV_CHUNK));
+  const uint64_t chunk = use == PivotUse::PROBE ? CHUNK_PROBE : CHUNK_EXACT;
+  const uint32_t S = static_cast<uint32_t>(std::min<uint64_t>(n, PV_CHUNKS * chunk));
   DevBuf<float> dmin(c, S);
-  DevBuf<double> csum(c, nchunks);
-  const size_t smem = static_cast<size_t>(PV_BATCH) * d * sizeof(float);
-  PM_CUDA(cudaFuncSetAttribute(pivot_dmin_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-  pivot_draw_kernel<<<1, PV_BATCH * 32, 0, c.stream>>>(dmin.get(), S, n, csum.get(), nchunks, 0, d_piv_rows);
-  PM_LAUNCHED();
-  constexpr int ROUNDS = (PIV - PV_FAR) / PV_BATCH;
-  for (int r = 1; r <= ROUNDS; ++r) {
-    pivot_dmin_kernel<<<nchunks, 256, smem, c.stream>>>(d_x, n, static_cast<int>(d), S, d_piv_rows, (r - 1) * PV_BATCH,
-                                                        dmin.get(), csum.get());
-    PM_LAUNCHED();
-    if (r == ROUNDS) break;
-    pivot_draw_kernel<<<1, PV_BATCH * 32, 0, c.stream>>>(dmin.get(), S, n, csum.get(), nchunks, r, d_piv_rows);
-    PM_LAUNCHED();
+  if (use == PivotUse::PROBE) {
+    draw_pivots<CHUNK_PROBE>(c, d_x, n, d, S, PIV / PV_BATCH, false, dmin.get(), d_piv_rows);
+    return;
   }
+  draw_pivots<CHUNK_EXACT>(c, d_x, n, d, S, (PIV - PV_FAR) / PV_BATCH, true, dmin.get(), d_piv_rows);
   DevBuf<unsigned long long> best(c, PV_FAR);
   PM_CUDA(cudaMemsetAsync(best.get(), 0, best.bytes(), c.stream));
   for (int k = 0; k < PV_FAR; ++k) {
-    pivot_far_kernel<<<nchunks, 256, 0, c.stream>>>(d_x, n, static_cast<int>(d), S, k, dmin.get(), best.get(),
-                                                    d_piv_rows);
+    pivot_far_kernel<<<ceil_div(S, CHUNK_EXACT), 256, 0, c.stream>>>(d_x, n, static_cast<int>(d), S, k, dmin.get(),
+                                                                    best.get(), d_piv_rows);
     PM_LAUNCHED();
   }
   pivot_far_last_kernel<<<1, 1, 0, c.stream>>>(n, S, best.get(), d_piv_rows);

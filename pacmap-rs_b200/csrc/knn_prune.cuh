@@ -4,8 +4,11 @@
 
 namespace pacmap {
 
-// PIV pivot rows of d_x (n x d), deterministic: by k-means++ seeding in batches on a fixed subsample, or evenly spaced.
-void select_pivots(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint32_t* d_piv_rows, bool seeded);
+// PIV pivot rows of d_x (n x d), deterministic, for what a search needs the cells for: near rows near each other (ORDER:
+// evenly spaced), tight bounds (PRUNE: k-means++ seeding in batches on a fixed subsample, then farthest points), or the
+// cells that an approximate search looks into, on which its rows depend (PROBE: seeding alone, a larger subsample).
+enum class PivotUse { ORDER, PRUNE, PROBE };
+void select_pivots(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint32_t* d_piv_rows, PivotUse use);
 
 // Inputs of the tile test, all on the device and in the locality order unless noted:
 //   perm        position r -> original row

@@ -1333,7 +1333,8 @@ bool knn_tc_device(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint64_t kp
   // wants near rows near each other, for which evenly spaced points do.
   const uint32_t chunks = ceil_div(n, PL_CHUNK);
   DevBuf<uint32_t> piv_rows(c, PIV), cell(c, n), cell_counts(c, static_cast<uint64_t>(chunks) * PIV), perm(c, n);
-  select_pivots(c, d_x, n, d, piv_rows.get(), /*seeded=*/n >= PRUNE_MIN_ROWS || nprobe > 0);
+  select_pivots(c, d_x, n, d, piv_rows.get(),
+                nprobe > 0 ? PivotUse::PROBE : (n >= PRUNE_MIN_ROWS ? PivotUse::PRUNE : PivotUse::ORDER));
   DevBuf<float> score, pnorm;
   if (prune) {
     score.alloc(c, n * PIV);
