@@ -334,6 +334,10 @@ uint64_t pacmap_take_launch_count(void);
  * of hanging; on = 0 restores normal operation. The caller's current device is kept. */
 pacmap_status pacmap_debug_stall_knn_loads(int32_t device, int32_t on);
 
+/* Test hook (no reference analogue; tests only): with on != 0, calls of this thread get no memory beyond what they
+ * cannot do without, as when the device or the host has none left; they return the same results, later. */
+void pacmap_debug_scarce_memory(int32_t on);
+
 /* Test hook (no reference analogue): out[i] = num / x[i] on the device with the division that the optimiser's tiled
  * gradient uses for its pair factors. x, out: n values of host memory. */
 pacmap_status pacmap_debug_divide(float num, const float* x, uint64_t n, int32_t device, float* out);

@@ -2,6 +2,7 @@
 #pragma once
 
 #include <memory>
+#include <new>
 #include <vector>
 
 #include "common.cuh"
@@ -55,6 +56,24 @@ struct DevBuf {
   T* get() const { return p; }
   size_t bytes() const { return count * sizeof(T); }
 };
+
+// Throws PACMAP_ERR_OOM while the calling thread's test hook asks for it (pacmap_debug_scarce_memory).
+void scarce_memory_hook();
+
+// Runs f, which takes memory that only makes a call faster; false when that cannot be had, with no CUDA error left behind.
+template <typename F>
+bool try_scratch(F&& f) {
+  try {
+    scarce_memory_hook();
+    f();
+    return true;
+  } catch (const Fail& e) {
+    if (e.code != PACMAP_ERR_OOM) throw;
+  } catch (const std::bad_alloc&) {
+  }
+  cudaGetLastError();
+  return false;
+}
 
 // ---- hostcopy.cu ----
 // Copies on the call's stream between the device and a caller's host memory, which the call may let go of (to_device) or

@@ -5,7 +5,8 @@
 // cut into one range per worker: each worker moves its range piece by piece through two page-locked slots of its own,
 // copying one piece on a core while the other is on the link (64 MB: 3.0 and 3.1 ms). The threads live for one copy;
 // the slots (32 MB) stay with the device until the library is unloaded. Calls on a device hold its lock, so one copy
-// uses them at a time. Memory that the caller page-locked goes to the link directly.
+// uses them at a time. Memory that the caller page-locked goes to the link directly, and everything goes the driver's way
+// when the slots cannot be page-locked.
 #include <algorithm>
 #include <cstring>
 #include <system_error>
@@ -29,12 +30,13 @@ struct HostStaging {
   char* buf = nullptr;
   cudaEvent_t ev[COPY_WORKERS][2] = {};
   HostStaging() {
-    PM_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&buf), 2 * COPY_WORKERS * COPY_SLOT, cudaHostAllocDefault));
+    if (cudaHostAlloc(reinterpret_cast<void**>(&buf), 2 * COPY_WORKERS * COPY_SLOT, cudaHostAllocDefault) != cudaSuccess)
+      throw Fail{PACMAP_ERR_OOM, "cudaHostAlloc (staging)"};  // whatever the reason: the copy has another way
     for (auto& w : ev)
       for (auto& e : w)
         if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
           release();
-          throw Fail{PACMAP_ERR_CUDA, "cudaEventCreateWithFlags (staging)"};
+          throw Fail{PACMAP_ERR_OOM, "cudaEventCreateWithFlags (staging)"};
         }
   }
   void release() {
@@ -92,11 +94,12 @@ void copy_host(Ctx& c, void* dst, const void* src, size_t bytes, bool to_device)
   const bool pageable = bytes >= (to_device ? UP_MIN : DOWN_MIN) &&
                         cudaPointerGetAttributes(&at, to_device ? src : dst) == cudaSuccess &&
                         at.type == cudaMemoryTypeUnregistered;
-  if (!pageable) {
+  if (!pageable || !try_scratch([&] {
+        if (!g_staging[c.device]) g_staging[c.device] = std::make_unique<HostStaging>();
+      })) {
     PM_CUDA(cudaMemcpyAsync(dst, src, bytes, kind, c.stream));
     return;
   }
-  if (!g_staging[c.device]) g_staging[c.device] = std::make_unique<HostStaging>();
   HostStaging& st = *g_staging[c.device];
   const int cores = static_cast<int>(std::max(1u, std::thread::hardware_concurrency()));
   const int workers = static_cast<int>(
