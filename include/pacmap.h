@@ -335,7 +335,8 @@ uint64_t pacmap_take_launch_count(void);
 pacmap_status pacmap_debug_stall_knn_loads(int32_t device, int32_t on);
 
 /* Test hook (no reference analogue; tests only): with on != 0, calls of this thread get no memory beyond what they
- * cannot do without, as when the device or the host has none left; they return the same results, later. */
+ * cannot do without, as when the device or the host has none left; they return the same results, later (from 65,536 rows on an
+ * embedding's last digits may differ: its sums run in another order). */
 void pacmap_debug_scarce_memory(int32_t on);
 
 /* Test hook (no reference analogue): out[i] = num / x[i] on the device with the division that the optimiser's tiled

@@ -160,7 +160,8 @@ struct TileGrad {
   DevBuf<uint32_t> long_rows;   // rows left to grad_adam_long_kernel
   uint32_t n_long = 0;
 };
-// Builds it when the problem's sizes favour it (else false, nothing built); the same lists always get the same answer. losses: some iteration wants its loss.
+// Builds it when the problem's sizes favour it and the device has the memory (else false, nothing built); the same lists
+// get the same answer unless memory runs out. losses: some iteration wants its loss.
 bool build_tile_grad(Ctx& c, const Csr& csr, uint64_t n, uint64_t dim, bool losses, TileGrad& out);
 // One iteration of every row but the long ones (which p.long_rows must name), on stream s: two launches. mid: the
 // iteration's mid-near weight is not 0. With p.row_loss the rows' losses too; y, m and v are the same bits either way.

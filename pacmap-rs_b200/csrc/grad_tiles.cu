@@ -408,17 +408,8 @@ AdamFn adam_kernel(uint64_t dim, bool mid) {
   return mid ? tile_adam_kernel<3, true, LOSS> : tile_adam_kernel<3, false, LOSS>;
 }
 
-}  // namespace
-
-bool build_tile_grad(Ctx& c, const Csr& csr, uint64_t n, uint64_t dim, bool losses, TileGrad& out) {
-  if ((dim != 2 && dim != 3) || n < TILE_MIN_ROWS || n >= (1ull << 24)) return false;
-  const uint64_t fit = (TILE_SMEM / (4 * dim) - 1) / 4 * 4;  // a tile's points and NOWHERE
-  const uint64_t tiles = (n + fit - 1) / fit;
-  const double per_row = static_cast<double>(csr.entries) / static_cast<double>(n);
-  const double near_far = static_cast<double>(csr.entries - csr.entries_mn) / static_cast<double>(n);
-  if (tiles > MAX_TILES || per_row > 0.8 * ROW_MAX || near_far < TILE_MIN_ROW_ENTRIES ||
-      near_far < tile_min_entries(dim) * static_cast<double>(tiles))
-    return false;
+// The lists for `tiles` tiles; false when too many rows are long ones.
+bool build_lists(Ctx& c, const Csr& csr, uint64_t n, uint64_t dim, uint64_t tiles, bool losses, TileGrad& out) {
   out.tiles = static_cast<uint32_t>(tiles);
   out.tile_pts = static_cast<uint32_t>(((n + tiles - 1) / tiles + 3) / 4 * 4);
   out.windows = ceil_div(n, WIN);
@@ -464,6 +455,23 @@ bool build_tile_grad(Ctx& c, const Csr& csr, uint64_t n, uint64_t dim, bool loss
   for (const bool loss : {false, true})
     PM_CUDA(cudaFuncSetAttribute(force_kernel(dim, loss), cudaFuncAttributeMaxDynamicSharedMemorySize, TILE_SMEM));
   return true;
+}
+
+}  // namespace
+
+bool build_tile_grad(Ctx& c, const Csr& csr, uint64_t n, uint64_t dim, bool losses, TileGrad& out) {
+  if ((dim != 2 && dim != 3) || n < TILE_MIN_ROWS || n >= (1ull << 24)) return false;
+  const uint64_t fit = (TILE_SMEM / (4 * dim) - 1) / 4 * 4;  // a tile's points and NOWHERE
+  const uint64_t tiles = (n + fit - 1) / fit;
+  const double per_row = static_cast<double>(csr.entries) / static_cast<double>(n);
+  const double near_far = static_cast<double>(csr.entries - csr.entries_mn) / static_cast<double>(n);
+  if (tiles > MAX_TILES || per_row > 0.8 * ROW_MAX || near_far < TILE_MIN_ROW_ENTRIES ||
+      near_far < tile_min_entries(dim) * static_cast<double>(tiles))
+    return false;
+  // The lists and the tiles' sums take 1 GB at 1,000,000 rows, which grad_adam_kernel does without.
+  bool built = false;
+  if (!try_scratch([&] { built = build_lists(c, csr, n, dim, tiles, losses, out); }) || !built) out = TileGrad();
+  return built;
 }
 
 void launch_tile_grad(const TileGrad& tg, const GradArgs& p, uint64_t dim, int itr, bool mid, cudaStream_t s) {

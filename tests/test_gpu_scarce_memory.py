@@ -25,3 +25,19 @@ def test_copies_without_page_locked_slots(lib, orc):
         got = lib.stages.preprocess(x)[0]
     assert np.array_equal(got, orc.preprocess(x)[0])
     assert np.array_equal(lib.stages.preprocess(x)[0], got)
+
+
+def test_gradient_without_tile_lists(lib):
+    """66,001 points in 3-D: the row-by-row gradient's bits, and a fit that goes through."""
+    n = 66001
+    rng = np.random.default_rng(0)
+    pairs = [np.stack([np.repeat(np.arange(n), k), rng.integers(0, n, n * k)], 1).astype(np.uint32) for k in (12, 6, 24)]
+    y = rng.normal(0, 4, size=(n, 3)).astype(np.float32)
+    cfg = lib.Configuration(initialization=lib.Initialization.Random(3), seed=5, num_iters=(4, 4, 4), embedding_dimensions=3,
+                            pair_configuration=lib.PairConfiguration.AllProvided(*pairs))
+    with _scarce(lib):
+        g = lib.stages.optimize_steps(y.copy(), np.zeros_like(y), np.zeros_like(y), *pairs, 1.0, 100, 100, 150, 151)
+        e, _ = lib.fit_transform(y, cfg)
+    assert np.array_equal(g, lib.stages.gradient(y, *pairs, 3.0, 3.0, 1.0))
+    a, _ = lib.fit_transform(y, cfg)
+    assert np.linalg.norm(a - e) <= 1e-4 * np.linalg.norm(a) and not np.array_equal(a, e)
