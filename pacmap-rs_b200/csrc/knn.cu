@@ -300,9 +300,16 @@ void knn_exact_device(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint64_t
                        ((mode == PACMAP_KNN_AUTO || mode == PACMAP_KNN_APPROX) && n >= TC_AUTO_ROWS);
   const bool forced = mode != PACMAP_KNN_AUTO && mode != PACMAP_KNN_APPROX;
   if (want_tc && knn_tc_supported(n, d, kp)) {
-    if (knn_tc_device(c, d_x, n, d, kp, mode == PACMAP_KNN_TENSOR_BF16, d_idx, d_dist, shard, approx ? 16 : 0,
-                      /*prune=*/mode != PACMAP_KNN_TENSOR_F16_FULL, /*any_scale=*/forced || n >= TC_APPROX_ROWS))
-      return;
+    bool done = false;
+    auto tensor = [&] {
+      done = knn_tc_device(c, d_x, n, d, kp, mode == PACMAP_KNN_TENSOR_BF16, d_idx, d_dist, shard, approx ? 16 : 0,
+                           /*prune=*/mode != PACMAP_KNN_TENSOR_F16_FULL, /*any_scale=*/forced || n >= TC_APPROX_ROWS);
+    };
+    // Where it was chosen for its speed alone, the SIMT kernel stands in when its buffers (4 KB a row and more) cannot be
+    // had; not for a shard, whose rows are the others' complement in the tensor path's order.
+    if (forced || n >= TC_APPROX_ROWS || shard.count > 1) tensor();
+    else try_scratch(tensor);
+    if (done) return;
   }
   PM_REQUIRE(mode == PACMAP_KNN_AUTO || mode == PACMAP_KNN_SIMT_EXACT || mode == PACMAP_KNN_APPROX,
              PACMAP_ERR_UNSUPPORTED,

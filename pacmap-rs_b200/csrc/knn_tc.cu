@@ -1626,11 +1626,16 @@ bool knn_tc_device(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint64_t kp
 
   // The overflowed rows: sorted, through the filter with fixed thresholds into column lists, exact distances over
   // those. A launch takes at most one block per SM; fewer row blocks split the column tiles.
-  if (counts[0] > 0) {
-    const uint32_t total = counts[0];
+  const uint32_t total = counts[0];
+  DevBuf<uint32_t> ids(c, total);
+  auto original_ids = [&] {
+    original_ids_kernel<<<ceil_div(total, 256), 256, 0, c.stream>>>(ovf.get(), total, perm.get(), ids.get());
+    PM_LAUNCHED();
+  };
+  auto settle_over_lists = [&] {
     const uint32_t fblocks = ceil_div(n, OL_ROWS);
     DevBuf<uint8_t> flags(c, n);
-    DevBuf<uint32_t> fcounts(c, fblocks), ids(c, total);
+    DevBuf<uint32_t> fcounts(c, fblocks);
     PM_CUDA(cudaMemsetAsync(flags.get(), 0, n, c.stream));
     overflow_flag_kernel<<<ceil_div(total, 256), 256, 0, c.stream>>>(ovf.get(), total, flags.get());
     PM_LAUNCHED();
@@ -1638,8 +1643,7 @@ bool knn_tc_device(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint64_t kp
     PM_LAUNCHED();
     overflow_place_kernel<<<fblocks, OL_ROWS, 0, c.stream>>>(flags.get(), n, fcounts.get(), ovf.get());
     PM_LAUNCHED();
-    original_ids_kernel<<<ceil_div(total, 256), 256, 0, c.stream>>>(ovf.get(), total, perm.get(), ids.get());
-    PM_LAUNCHED();
+    original_ids();
     const uint64_t blocks_fit = std::max<uint64_t>(1, WIDE_COLS_MAX / (n_pad * (TC_BM / 32)));
     const uint32_t blocks_max = static_cast<uint32_t>(
         std::min<uint64_t>({ceil_div(total, TC_BM), static_cast<uint64_t>(c.sm_count), blocks_fit}));
@@ -1679,9 +1683,13 @@ bool knn_tc_device(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint64_t kp
       knn_rows_simt(c, d_x, n, d, kp, ids.get() + q0, m, d_idx, d_dist, /*scatter=*/true, &kl);
     }
     c.check_errors("tensor-core kNN wide rows");
+  };
+  if (total > 0 && !try_scratch(settle_over_lists)) {  // no memory for the lists (up to 1 GB): over all columns
+    original_ids();
+    knn_rows_simt(c, d_x, n, d, kp, ids.get(), total, d_idx, d_dist, /*scatter=*/true);
   }
   // Rows with fewer certified candidates than neighbours: exact SIMT recomputation, scattered into place.
-  st.wide_rows = counts[0];
+  st.wide_rows = total;
   st.fallback_rows = counts[1];
   if (counts[1]) knn_rows_simt(c, d_x, n, d, kp, fbk.get(), counts[1], d_idx, d_dist, /*scatter=*/true);
   return true;

@@ -41,3 +41,26 @@ def test_gradient_without_tile_lists(lib):
     assert np.array_equal(g, lib.stages.gradient(y, *pairs, 3.0, 3.0, 1.0))
     a, _ = lib.fit_transform(y, cfg)
     assert np.linalg.norm(a - e) <= 1e-4 * np.linalg.norm(a) and not np.array_equal(a, e)
+
+
+def test_knn_below_16384_rows_without_filter_buffers(lib):
+    x = np.random.default_rng(1).normal(size=(6001, 20)).astype(np.float32)
+    with _scarce(lib):
+        gi, gd = lib.knn.find_k_nearest_neighbors(x, 15)
+    ei, ed = lib.knn.find_k_nearest_neighbors(x, 15)
+    assert np.array_equal(gi, ei) and np.array_equal(gd, ed)
+
+
+def test_knn_of_overflowed_rows_without_column_lists(lib, orc):
+    """2,000 exact ties and a dense clump far from the origin, more than the filter's buffers hold."""
+    rng = np.random.default_rng(2)
+    x = rng.normal(size=(17001, 24)).astype(np.float32)
+    x[3000:5000] = x[3000]
+    x[9000:12000] = 300 + 0.001 * rng.normal(size=(3000, 24)).astype(np.float32)
+    with _scarce(lib):
+        gi, gd = lib.knn.find_k_nearest_neighbors(x, 20)
+    ei, ed = lib.knn.find_k_nearest_neighbors(x, 20)
+    assert np.array_equal(gi, ei) and np.array_equal(gd, ed)
+    rows = np.arange(0, 17001, 29, dtype=np.uint32)
+    oi, od = orc.knn_rows(x, rows, 20)
+    assert np.array_equal(gi[rows], oi) and np.array_equal(gd[rows], od)
