@@ -1172,8 +1172,10 @@ void gradient_device(Ctx& c, const Csr& csr, const float* d_y, uint64_t n, uint6
   ga.grad_only = 1;
   fns.rows<<<grid, 256, 0, c.stream>>>(ga, 0);
   PM_LAUNCHED();
-  if (csr.n_long > 0) fns.long_rows<<<ceil_div(csr.n_long, 8), 256, 0, c.stream>>>(ga, 0);
-  PM_LAUNCHED();
+  if (csr.n_long > 0) {
+    fns.long_rows<<<ceil_div(csr.n_long, 8), 256, 0, c.stream>>>(ga, 0);
+    PM_LAUNCHED();
+  }
   loss_reduce_kernel<<<1, 1024, 0, c.stream>>>(row_loss.get(), n, loss_dev.get());
   PM_LAUNCHED();
   PM_CUDA(cudaMemcpyAsync(h_loss, loss_dev.get(), sizeof(float), cudaMemcpyDeviceToHost, c.stream));
