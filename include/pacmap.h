@@ -334,6 +334,11 @@ uint64_t pacmap_take_launch_count(void);
  * of hanging; on = 0 restores normal operation. The caller's current device is kept. */
 pacmap_status pacmap_debug_stall_knn_loads(int32_t device, int32_t on);
 
+/* Failure-detection test hook (no reference analogue; tests only): with on != 0, the optimiser's blocks in this thread's
+ * calls of up to about 18,900 rows meet after each iteration with one block more than there are, so that their bounded
+ * wait runs out (2 s) and the call fails with PACMAP_ERR_DEVICE_INVARIANT instead of hanging. */
+void pacmap_debug_stall_optimizer(int32_t on);
+
 /* Test hook (no reference analogue; tests only): with on != 0, calls of this thread get no memory beyond what they
  * cannot do without, as when the device or the host has none left; they return the same results, later (from 65,536 rows on an
  * embedding's last digits may differ: its sums run in another order). */

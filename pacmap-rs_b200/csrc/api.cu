@@ -18,7 +18,7 @@ namespace pacmap {
 namespace {
 thread_local std::string g_last_error;
 thread_local uint64_t g_launches = 0;
-thread_local bool g_stage_timing = false, g_scarce_memory = false;
+thread_local bool g_stage_timing = false, g_scarce_memory = false, g_stall_optimizer = false;
 thread_local std::vector<double> g_stage_ms;
 std::mutex g_device_mutex[64];
 
@@ -33,6 +33,7 @@ DeviceState g_devices[64];
 
 void set_last_error(const std::string& msg) { g_last_error = msg; }
 void count_launch(uint64_t k) { g_launches += k; }
+bool stall_optimizer_hook() { return g_stall_optimizer; }
 void scarce_memory_hook() {
   if (g_scarce_memory) throw Fail{PACMAP_ERR_OOM, "no scratch memory (test hook)"};
 }
@@ -904,6 +905,7 @@ pacmap_status pacmap_init_random(uint64_t n, uint64_t dim, uint64_t seed, int32_
 }
 
 void pacmap_debug_scarce_memory(int32_t on) { g_scarce_memory = on != 0; }
+void pacmap_debug_stall_optimizer(int32_t on) { g_stall_optimizer = on != 0; }
 
 pacmap_status pacmap_debug_divide(float num, const float* x, uint64_t n, int32_t device, float* out) {
   return guarded([&] {

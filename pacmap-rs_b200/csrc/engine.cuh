@@ -57,6 +57,9 @@ struct DevBuf {
   size_t bytes() const { return count * sizeof(T); }
 };
 
+// Whether the calling thread's test hook asks the resident optimiser to wait in vain (pacmap_debug_stall_optimizer).
+bool stall_optimizer_hook();
+
 // Throws PACMAP_ERR_OOM while the calling thread's test hook asks for it (pacmap_debug_scarce_memory).
 void scarce_memory_hook();
 

@@ -86,6 +86,7 @@ _SIGS = {
                                                 _vp]),
     "pacmap_debug_small_axes": (C.c_int, [_vp, _u64, _u64, _i32, _vp, _vp]),
     "pacmap_debug_scarce_memory": (None, [_i32]),
+    "pacmap_debug_stall_optimizer": (None, [_i32]),
     "pacmap_debug_divide": (C.c_int, [_f32, _vp, _u64, _i32, _vp]),
     "pacmap_debug_stall_knn_loads": (C.c_int, [_i32, _i32]),
     "pacmap_set_stage_timing": (None, [_i32]),
