@@ -167,8 +167,12 @@ __global__ void tile_shares_kernel(const uint32_t* __restrict__ unit_off, uint64
 // J. Res. Dev. 34, 1990): correctly rounded up to x = 2^126 (tested against the / operator for every mantissa of x),
 // 0 beyond, where the quotient is below 1e-36; NaN for NaN, as a division. The compiler's division checks its operands and branches, which kept
 // two entries' divisions from overlapping.
+__device__ __forceinline__ float min_or_nan(float x, float most) {
+  asm("min.NaN.f32 %0, %0, %1;" : "+f"(x) : "f"(most));
+  return x;
+}
 __device__ __forceinline__ float div_by(float num, float x) {
-  asm("min.NaN.f32 %0, %0, %1;" : "+f"(x) : "f"(3.402823466e+38f));  // infinity would make the remainder NaN
+  x = min_or_nan(x, 3.402823466e+38f);  // infinity would make the remainder NaN
   float y;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   y = fmaf(fmaf(-x, y, 1.0f), y, y);
@@ -209,9 +213,9 @@ __device__ __forceinline__ void add_entry(const float* ys, uint32_t e, bool far,
     float dsq = 1.0f;
 #pragma unroll
     for (int c = 0; c < DIM; ++c) dsq = fmaf(df[c], df[c], dsq);
-    const float part = far ? __fmul_rn(w_fp, __fdiv_rn(1.0f, __fadd_rn(1.0f, dsq)))
-                           : __fmul_rn(w_nn, __fdiv_rn(dsq, __fadd_rn(10.0f, dsq)));
-    if (e != none) lacc += part;
+    dsq = min_or_nan(dsq, 1.2676506e30f);  // 2^100: both losses are at their limits there, and div_by is exact enough
+    const float part = div_by(far ? 1.0f : dsq, (far ? 1.0f : 10.0f) + dsq);
+    if (e != none) lacc = fmaf(far ? w_fp : w_nn, part, lacc);
   }
 }
 

@@ -17,8 +17,8 @@
 //    Phase 3 has w_mn = 0: the MN segments are skipped (0 * finite = 0 adds nothing).
 //    Rows of more than 1,024 entries go to grad_adam_long_kernel beside it, a warp each. From 65,536 rows in 2-D
 //    and 3-D the near and far partners come from tiles of y in shared memory instead (grad_tiles.cu).
-// K9 optimize_device: up to about 18,900 rows all iterations run in one launch (grad_adam_resident_kernel); above,
-//    or with losses asked for, they are captured into one CUDA graph (one or two kernel nodes per iteration,
+// K9 optimize_device: while all rows fit the GPU at once (18,944 in 1-D and 2-D, 14,208 in 3-D, 9,472 in 4-D and 5-D, 4,736
+//    above, on 148 SMs) all iterations run in one launch (grad_adam_resident_kernel); above, or with losses asked for, they are captured into one CUDA graph (one or two kernel nodes per iteration,
 //    snapshot copies as memcpy nodes). The per-iteration (w_nn, w_mn, w_fp, lr_t) schedule lives in a device table computed
 //    with the reference's f32 formulas.
 #include <chrono>
@@ -669,12 +669,22 @@ __global__ void long_rows_kernel(const uint32_t* __restrict__ rp, uint64_t n, ui
   if (i < n && rp[3 * i + 3] - rp[3 * i] > GRAD_LONG) rows[atomicAdd(count, 1u)] = static_cast<uint32_t>(i);
 }
 
-// Sum of the per-row losses in a fixed order; each pair was counted at both endpoints.
+// Sum of the per-row losses in a fixed order (one block of 1,024 threads); each pair was counted at both endpoints.
 __global__ void __launch_bounds__(1024) loss_reduce_kernel(const float* __restrict__ row_loss, uint64_t n,
                                                            float* __restrict__ out) {
   __shared__ double red[1024];
   double s = 0.0;
-  for (uint64_t i = threadIdx.x; i < n; i += blockDim.x) s += row_loss[i];
+  // A thread's additions are one chain in this order; LOSS_AHEAD loads are in flight ahead of them.
+  constexpr int LOSS_AHEAD = 16;
+  uint64_t i = threadIdx.x;
+  for (; i + (LOSS_AHEAD - 1) * 1024ull < n; i += LOSS_AHEAD * 1024ull) {
+    float v[LOSS_AHEAD];
+#pragma unroll
+    for (int q = 0; q < LOSS_AHEAD; ++q) v[q] = row_loss[i + q * 1024ull];
+#pragma unroll
+    for (int q = 0; q < LOSS_AHEAD; ++q) s += v[q];
+  }
+  for (; i < n; i += 1024) s += row_loss[i];
   red[threadIdx.x] = s;
   __syncthreads();
   for (int o = 512; o > 0; o >>= 1) {
