@@ -265,13 +265,6 @@ def _optimize_bytes(n, dim, iters):
     return (iters[0] + iters[1]) * per(p12) + iters[2] * per(p3)
 
 
-def _optimize_gathers(n, iters):
-    """Partner gathers of the gradient iterations: every active pair is an entry in both endpoints'
-    segments, and each entry loads its partner's coordinates once (mid-near pairs inactive in phase 3)."""
-    k, n_mn, n_fp = _pair_counts(n)
-    return (iters[0] + iters[1]) * 2 * n * (k + n_mn + n_fp) + iters[2] * 2 * n * (k + n_fp)
-
-
 def run_ours(args, rank, world, local_rank):
     import ctypes as C
 
@@ -470,25 +463,13 @@ def run_ours(args, rank, world, local_rank):
     opt_bytes = _optimize_bytes(n, dim, learned.SHORT_SCHEDULE)
     opt_gbs = opt_bytes / (opt_ms * 1e-3) / 1e9 if opt_ms > 0 else None
     roof_opt = {"kernel": ("tile_force_kernel + tile_adam_kernel (gradient from shared-memory tiles + Adam; grad_adam_kernel "
-                           "where a row has under 4 partners per tile), once per iteration in a CUDA graph"),
+                           "where a row has few partners per tile), once per iteration in a CUDA graph"),
                 "bound": "hbm", "achieved": round(opt_gbs, 1) if opt_gbs else None, "peak": hbm, "unit": "GB/s",
                 "frac": round(opt_gbs / hbm, 4) if opt_gbs else None, "traffic": traffic.get("tile_gradient"),
                 "algorithmic": ("8 B per active pair + 28*n*dim B per iteration (k, n_mn, n_fp = %d, %d, %d; mid-near "
                                 "pairs inactive in phase 3)" % _pair_counts(n)),
                 "launch_ms": round(opt_ms / iters, 4) if opt_ms else None,
                 "peak_source": f"{src} HBM copy"}
-    # the partner reads against this device's measured rate of random 8-byte loads from an L2-resident array
-    # (pacmap_gather_rate): a ceiling for gathers from L2, not for the near and far partners that come from
-    # shared-memory tiles
-    rate = pm.gather_rate(local_rank)
-    gathers = _optimize_gathers(n, learned.SHORT_SCHEDULE)
-    g_rate = gathers / (opt_ms * 1e-3) if opt_ms > 0 else None
-    roof_opt["gather_roofline"] = {
-        "achieved": round(g_rate / 1e9, 1) if g_rate else None, "peak": round(rate / 1e9, 1), "unit": "G loads/s",
-        "frac": round(g_rate / rate, 4) if g_rate and rate else None,
-        "algorithmic": ("2 (k + n_fp) partner loads per point per iteration, 2 (k + n_mn + n_fp) in phases 1-2; near and "
-                        "far ones from shared memory where the gradient is tiled"),
-        "peak_source": "measured: random 8-byte loads from an L2-resident 8 MB array (pacmap_gather_rate)"}
     # the headline roofline is the kernel that takes the larger share of the learned step
     dominant_opt = opt_ms >= knn_ms
     rnd = lambda q: {"knn10_preservation": round(q[0], 5), "triplet_accuracy": round(q[1], 4)}  # noqa: E731

@@ -335,7 +335,7 @@ uint64_t pacmap_take_launch_count(void);
 pacmap_status pacmap_debug_stall_knn_loads(int32_t device, int32_t on);
 
 /* Failure-detection test hook (no reference analogue; tests only): with on != 0, the optimiser's blocks in this thread's
- * calls of up to about 18,900 rows meet after each iteration with one block more than there are, so that their bounded
+ * calls of few rows (2-D: up to 18,944) meet after each iteration with one block more than there are, so that their bounded
  * wait runs out (2 s) and the call fails with PACMAP_ERR_DEVICE_INVARIANT instead of hanging. */
 void pacmap_debug_stall_optimizer(int32_t on);
 

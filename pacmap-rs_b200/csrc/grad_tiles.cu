@@ -1,16 +1,17 @@
 // The gradient of many points with the partners' coordinates in shared memory.
 //
 // grad_adam_kernel (optimizer.cu) gathers every partner's y from L2, one 32-byte sector request per 8-byte partner, and
-// runs at the rate of those requests (0.97 ms an iteration for 1,000,000 points in 2-D, 240 to 280 million gathers).
-// Here the points are cut into tiles of up to 29,056 (2-D; what 227 KB of shared memory hold). An iteration is two
-// kernels:
+// runs at the rate of those requests (0.96 ms an iteration for 1,000,000 points in 2-D, 240 to 280 million gathers).
+// Here the points are cut into tiles of up to 29,052 (2-D; 19,364 in 3-D: what 227 KB of shared memory hold beside the
+// unused places' point). An iteration is two kernels:
 //   tile_force_kernel  each block keeps one tile's y in shared memory and goes over the rows that have partners there
 //                      (neighbour and far pairs), a lane per row, writing the row's sum over the tile's partners;
 //   tile_adam_kernel   eight lanes per row add the row's tile sums in a fixed order, gather its mid-near partners as
 //                      grad_adam_kernel does (they are few, and none in the last phase), and take the Adam step.
 // The regrouped lists are built once per fit (build_tile_grad): rows in windows of 128, within each (tile, window)
-// sorted by their number of entries so that the 32 rows of a unit are about equally long, each row's entries in CSR
-// order.
+// sorted by their number of entries and cut into units of 32, each row's entries in CSR order. A unit runs to its longest
+// row: for entries spread at random it goes over 1.1 places per entry at 48 entries per row and tile, 1.2 at 20, 1.36 at 7
+// (1,000,000 rows), and stores 1.1, 1.25 and 1.5.
 // No atomics on floats: the sums and their order are the same on every call (another order than grad_adam_kernel's).
 #include <algorithm>
 
@@ -162,15 +163,17 @@ __global__ void tile_shares_kernel(const uint32_t* __restrict__ unit_off, uint64
   cta_units[b] = b == ctas ? static_cast<uint32_t>(units) : static_cast<uint32_t>(lo);
 }
 
-// num / x for x >= 1, without a branch: an approximate reciprocal, one Newton step, and a correction of the quotient by
-// its exact remainder (P. W. Markstein, Computation of elementary functions on the IBM RISC System/6000 processor, IBM
-// J. Res. Dev. 34, 1990): correctly rounded up to x = 2^126 (tested against the / operator for every mantissa of x),
-// 0 beyond, where the quotient is below 1e-36; NaN for NaN, as a division. The compiler's division checks its operands and branches, which kept
-// two entries' divisions from overlapping.
+// x, at most `most`; NaN stays NaN (fminf would give `most`).
 __device__ __forceinline__ float min_or_nan(float x, float most) {
   asm("min.NaN.f32 %0, %0, %1;" : "+f"(x) : "f"(most));
   return x;
 }
+
+// num / x for x >= 1, without a branch: an approximate reciprocal, one Newton step, and a correction of the quotient by
+// its exact remainder (P. W. Markstein, Computation of elementary functions on the IBM RISC System/6000 processor, IBM
+// J. Res. Dev. 34, 1990): correctly rounded up to x = 2^126 (tested against the / operator for every mantissa of x),
+// 0 beyond, where the quotient is below 1e-36; NaN for NaN, as a division. The compiler's division checks its operands
+// and branches, which kept two entries' divisions from overlapping.
 __device__ __forceinline__ float div_by(float num, float x) {
   x = min_or_nan(x, 3.402823466e+38f);  // infinity would make the remainder NaN
   float y;
@@ -348,7 +351,7 @@ __global__ void __launch_bounds__(FORCE_T, 1) tile_force_kernel(const ForceArgs 
 
 // A row's tile sums (lane gl of eight adds tiles gl, gl + 8, ... in order), its mid-near pairs, the lanes' sums
 // pairwise, and the Adam step. Without the mid-near part (MID: their weight is not 0) a kernel of its own, 32 registers
-// a thread against 48: an iteration of the last phase at 1,000,000 rows 777 -> 750 us in 2-D, 1,320 -> 1,272 in 3-D.
+// a thread against 39: an iteration of the last phase at 1,000,000 rows 777 -> 750 us in 2-D, 1,320 -> 1,272 in 3-D.
 // With it the gathers' rate binds: four or eight partners in flight per lane instead of two changed nothing at
 // 1,000,000 rows. LOSS: the row's loss into p.row_loss, from the tiles' and the mid-near pairs', by the same lanes.
 template <int DIM, bool MID, bool LOSS>

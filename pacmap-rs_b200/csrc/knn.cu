@@ -289,11 +289,12 @@ void knn_exact_device(Ctx& c, const float* d_x, uint64_t n, uint64_t d, uint64_t
                       float* d_dist, const KnnShard& shard, uint64_t approx_threshold) {
   if (n == 0 || kp == 0) return;
   PM_REQUIRE(shard.count >= 1 && shard.index < shard.count, PACMAP_ERR_INVALID_ARGUMENT, "bad kNN shard");
-  // AUTO uses the tensor cores once the O(n^2) part dominates; the TENSOR modes force them. At 5,000 rows the two
-  // paths take the same time at 16 columns and 15 neighbours (0.66 and 0.62 ms) and the tensor cores win everywhere
-  // else (100 columns: 0.85 against 1.05 ms at 15 neighbours, 1.05 against 1.43 at 72; 784 columns: 2.9 against 4.2); at
-  // 4,000 the SIMT kernel wins up to 128 columns (100: 0.63 against 0.78). At 14,000 x 64 it is 1.2 against 4.2 ms.
-  // The approximate search starts at 16,384 rows.
+  // AUTO uses the tensor cores once the O(n^2) part dominates; the TENSOR modes force them. Tensor cores against the SIMT
+  // kernel at 5,000 rows, in ms: up to 32 columns and 15 neighbours the SIMT kernel is still ahead (2 columns 0.63 / 0.57, 32
+  // columns 0.77 / 0.67); at 72 neighbours 0.79 / 0.99 and 0.86 / 1.13, at 192 0.97 / 3.3 and 1.08 / 3.4, at 446 (1,024
+  // candidates a row) 1.4 / 10.2 and 1.5 / 10.3; 100 columns 0.75 / 1.05 at 15 neighbours, 784 columns 1.5 / 3.8. At 7,000
+  // rows it is ahead with 5 neighbours of 2 columns only (0.71 / 0.66), at 10,000 nowhere (0.89 / 1.37 there); at 4,000 up
+  // to 128 columns (100: 0.78 / 0.63). The approximate search starts at 16,384 rows.
   const bool approx = mode == PACMAP_KNN_APPROX && n >= approx_threshold && n >= TC_APPROX_ROWS;
   const bool want_tc = (mode == PACMAP_KNN_TENSOR_F16 || mode == PACMAP_KNN_TENSOR_BF16 ||
                         mode == PACMAP_KNN_TENSOR_F16_FULL) ||

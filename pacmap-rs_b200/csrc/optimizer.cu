@@ -18,9 +18,10 @@
 //    Rows of more than 1,024 entries go to grad_adam_long_kernel beside it, a warp each. From 65,536 rows in 2-D
 //    and 3-D the near and far partners come from tiles of y in shared memory instead (grad_tiles.cu).
 // K9 optimize_device: while all rows fit the GPU at once (18,944 in 1-D and 2-D, 14,208 in 3-D, 9,472 in 4-D and 5-D, 4,736
-//    above, on 148 SMs) all iterations run in one launch (grad_adam_resident_kernel); above, or with losses asked for, they are captured into one CUDA graph (one or two kernel nodes per iteration,
-//    snapshot copies as memcpy nodes). The per-iteration (w_nn, w_mn, w_fp, lr_t) schedule lives in a device table computed
-//    with the reference's f32 formulas.
+//    above, on 148 SMs) all iterations run in one launch (grad_adam_resident_kernel); above, with losses asked for, or with
+//    a row of more than 1,024 entries, they are captured into one CUDA graph (one to three kernel nodes per iteration,
+//    snapshot copies as memcpy nodes). The per-iteration (w_nn, w_mn, w_fp, lr_t) schedule lives in a device table
+//    computed with the reference's f32 formulas.
 #include <chrono>
 #include <cmath>
 #include <cstring>
