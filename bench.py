@@ -56,9 +56,9 @@ MEASURED_PEAKS = os.path.join(ROOT, "MEASURED_PEAKS.json")
 # 1,000,000 x 128 workload, from one-pass captures (ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum
 # -k regex:<kernel> -s <launches to skip> on `bench.py --minimal --steps 1 --warmup 1`): the filter's main
 # pass (the launch its roofline times; the bound pass moves 16.6 GB, mostly candidate writes), and the
-# gradient's average over the (0, 50, 150) schedule (its two kernels together 2.437 GB per phase-2
-# iteration, 2.138 GB per phase-3: the rows' sums per tile are written and read back).
-TRAFFIC = {"knn_filter_kernel": 4941928192, "tile_gradient": 2212485696}
+# gradient's average over the (0, 50, 150) schedule (its two kernels together 2.436 GB per phase-2
+# iteration, 2.137 GB per phase-3: the rows' sums per tile are written and read back).
+TRAFFIC = {"knn_filter_kernel": 4882010368, "tile_gradient": 2211543872}
 
 
 def _peaks():
