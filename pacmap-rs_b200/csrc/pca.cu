@@ -567,10 +567,12 @@ constexpr int JACOBI_THREADS = 1024, JACOBI_MAX_K = 8, JACOBI_SWEEPS = 20, JACOB
 constexpr int JACOBI_BLOCKS = ((JACOBI_MAX_D / 2) * (JACOBI_MAX_D / 2 - 1) / 2 + JACOBI_THREADS - 1) / JACOBI_THREADS;
 // The device from 32 columns on: 173 us against the host's 259 at 32 (copies in and out included), 135 against 127
 // at 24, 0.97 ms against 7.2 at 100, 2.7 against 64 at 160. Its residuals are the smaller (7e-15 of the largest
-// eigenvalue against 1.2e-14 at 100), and the f32 axes of 120 covariances of both kinds came out the same.
+// eigenvalue against 1.2e-14 at 100), and of 1,590 covariances of five kinds one had an f32 axis entry that came out
+// another way than the host's (uniform data, whose eigenvalues lie close together).
 // JACOBI_GAP: axes whose eigenvalues lie closer than this (of the largest) depend on the order of the rotations in
 // digits that f32 keeps, and equal eigenvalues leave the choice of basis to it, so the host's cyclic order stays
-// for those; above it the two methods' axes differ by about 1e-12, far below f32. Eight axes: the start's dim; the
+// for those; above it the two methods' axes differ by at most 10 * 2.2e-16 divided by the gap (6e-13 seen), which
+// shows in f32 only where an entry lies that close to the middle between two numbers. Eight axes: the start's dim; the
 // 100 axes of the wide data's reduction have closer pairs among them as a rule.
 constexpr int JACOBI_MIN_D = 32;
 constexpr double JACOBI_GAP = 1e-3;
